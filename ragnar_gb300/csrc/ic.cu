@@ -6,35 +6,50 @@
 //   Gamma = 4 g e_s,  q = (e / g) / (Gamma (1 - e / g)),
 //   KN(Gamma, q) = 2 q ln q + (1 - q) (1 + 2 q + (Gamma q)^2 / (2 (1 + Gamma q))).
 //
-// Rewritten so that the per-(g, s, e) work is one multiply and one logarithm:
-//   t = Gamma q = e / (g - e) depends on (e, g) only; g - e is exact in FP32 where it
-//     matters (e in [g/2, g]), so t avoids the reference's 1 - e/g cancellation;
-//   q = t / Gamma = (t / g) (1 / (4 e_s));  e <= g Gamma / (1 + Gamma)  <=>  q <= 1 (e < g);
-//   KN = q (2 ln 2) log2 q + ((1 + h) + (1 - h) q - 2 q^2),  h = t^2 / (2 (1 + t)).
-// With L = 2 ln 2 and p = L q (so 2 q ln q = p log2 q = p (log2 p - log2 L)) this is
-//   KN = p log2 p + ((1 + h) + ((1 - h) / L - log2 L) p - (2 / L^2) p^2),
-// whose quadratic's coefficients depend on (e, g) only and are set once per item.
-// Per eval: FMUL (p = (L t / g) (1 / (4 e_s))), MUFU.LG2, two FFMA (quadratic), FFMA (log
-// term), max(KN, 0), FFMA into the FP32 accumulator.  max(KN, 0) is KN [q <= 1]: at fixed
-// h, KN(1) = 0, KN'(1) = -1 - h < 0 and KN'' = 2/q - 4 < 0 for q > 1/2, so KN < 0 for every
-// q > 1, while KN >= 0 on (0, 1] (the Klein-Nishina kernel).  Evals with p = inf (masked
-// soft photons; (e, g) pairs that no soft photon reaches, e >= g or an invalid e, which get
-// pg = inf) evaluate to NaN, which max(., 0) also maps to 0.  q >= 1e-30 is guaranteed by a
-// floor on t/g set per (e, g) from the smallest 1 / (4 e_s), so the log's argument is a
-// normal float or inf.  (A form without the per-eval logarithm, log2 p split into
-// log2 (t/g) + log2 (1/(4 e_s)) per item and per photon, takes five FP32 instructions per
-// eval but leaves absolute errors of a few ulp of those logarithms' magnitudes in KN: 2.4e-5
-// to 8.6e-5 from FP64 on the reference's delta-function soft-photon cases, where a single
-// (g, s) pair at 1 - q = 3.5e-3 feeds an IC bin.)
+// Rewritten so that what depends on (e, g) and what depends on the soft photon separate:
+//   t = Gamma q = e / (g - e),  z = t / g,  q = z i_s with i_s = 1 / (4 e_s),
+//   e <= g Gamma / (1 + Gamma)  <=>  q <= 1 (e < g),  h = t^2 / (2 (1 + t)),
+//   KN = (1 + h) + (1 - h) q - 2 q^2 + 2 q ln q.
 //
-// Layout: lanes own IC bins (K rows of 32 per lane, 512-bin slices in blockIdx.y); warps take
-// (gamma bin, 64-soft-photon chunk) items; per item the FP32 sums are scaled by
-// e^2 f_g / g^k and folded into a double-float; per-warp FP64 partials are reduced in a
-// fixed order: the block's warps in FP64 at its end, then the blocks by a second kernel
-// (deterministic).  Non-positive or non-finite IC bins give
-// 0 (the reference produces NaN there).
-#include "rg_common.cuh"
-#include "rg_internal.hpp"
+// Regular soft photons (up to 16384 in any order or any number in ascending order, valid
+// energies in [1e-30, 1e30] and |w_s| <= 1e30, w_s = f_s / e_s: every tabulated distribution).
+// In descending order of i_s the photons with q <= 1 are a suffix s >= j of the table, and
+// with q_j = z i_j, the largest q of the suffix,
+//   sum_{s >= j} w_s KN = W0 + q V1 - 2 q^2 V2 + 2 q (V1 ln q + V3) + h (W0 - q V1),  q = q_j,
+//   W0 = sum w,  V1 = sum w r,  V2 = sum w r^2,  V3 = sum w r ln r,  r = i_s / i_j in (0, 1],
+// so one (gamma bin, IC bin) pair costs a binary search for j and a fixed number of
+// operations instead of a logarithm per soft photon: the work is ng x ne log2(ns), not
+// ng x ne x ns.  The suffix sums are formed in FP64 and stored as double-floats, and the
+// pair's terms are summed in double-float arithmetic: near q = 1 they cancel to
+// KN ~ (1 + h)(1 - q), which FP32 sums would leave with an error of 1e-7 / (1 - q).  FP32
+// pipes do it at about seven times the FP64 pipe's rate here (1.6 FP64 operations per clock
+// and SM against ~110 FP32).
+//
+// Any other soft photons (infinities and NaN among them) take the direct kernel, with L = 2 ln 2 and p = L q
+// (2 q ln q = p (log2 p - log2 L)):
+//   KN = p log2 p + ((1 + h) + ((1 - h) / L - log2 L) p - (2 / L^2) p^2),
+// per eval FMUL (p), MUFU.LG2, two FFMA (quadratic), FFMA (log term), max(KN, 0), FFMA into the
+// FP32 accumulator.  max(KN, 0) is KN [q <= 1]: at fixed h, KN(1) = 0, KN'(1) = -1 - h < 0 and
+// KN'' = 2/q - 4 < 0 for q > 1/2, so KN < 0 for every q > 1, while KN >= 0 on (0, 1] (the
+// Klein-Nishina kernel).  Evals with p = inf (masked soft photons; (e, g) pairs that no soft
+// photon reaches, e >= g or an invalid e, which get pg = inf) evaluate to NaN, which max(., 0)
+// also maps to 0.  q >= 1e-30 is guaranteed by a floor on t/g set per (e, g) from the smallest
+// 1 / (4 e_s), so the log's argument is a normal float or inf.  Lanes own IC bins (K rows of 32
+// per lane, 512-bin slices in blockIdx.y); warps take (gamma bin, 64-soft-photon chunk) items;
+// per item the FP32 sums are scaled by e^2 f_g / g^k and folded into a double-float.
+//
+// Which of the two runs is decided on the device (ic_sums_kernel), so a call needs no
+// host synchronisation; the other kernel's blocks return at once.  Both sum their warps in
+// FP64 at a block's end into one partial row, and the rows are summed in a fixed order
+// (deterministic).  Non-positive or non-finite IC bins give 0 (the reference produces NaN
+// there).
+//
+// Measured at 1024 gamma x 1024 soft-photon x 1024 IC bins, back to back on one stream: 54 us a
+// call (67 us with the photons shuffled) against 356 us with every triple evaluated, the largest
+// error against FP64 1e-7 against 2.2e-5 (a line of photons at the Klein-Nishina edge).  The
+// kernels: terms 9 us, sums 10 us (latency of one tile), pairs 21 us (issue: ~250 instructions
+// a pair, 40 of them the search), the direct kernel's early return 2.5 us, reduction 4.5 us.
+#include "moments_common.cuh"
 
 #include <algorithm>
 #include <cmath>
@@ -49,37 +64,236 @@ namespace rg {
     constexpr int kIcSChunk  = 64; // soft photons per work item
     constexpr int kIcMaxRows = 16; // rows of 32 IC bins per lane (the slice width is rows x 32)
 
+    // Suffix sums of a regular soft-photon table, as double-floats (hi, lo) per photon.
+    struct IcSums {
+      float2* i4; // 1 / (4 e_s)
+      float2* w0; // W0
+      float2* v1; // V1, V2, V3 relative to the photon's own 1 / (4 e_s)
+      float2* v2;
+      float2* v3;
+    };
+
     struct IcParams {
       const float* gb;      // ng gamma (gamma beta) bins
       const float* fp;      // ng particle distribution
       int          ng;
       int          log_spaced;
-      const float* inv4es;  // ns: 1 / (4 e_s)
-      const float* inv4es_min; // min over s of 1 / (4 e_s) (positive values), one float
-      const float* ws;      // ns: f_s / e_s
-      const float4* setup;  // ng x ne_pad per (gamma bin, IC bin): (pg, 1 + h, B1, 0), or null
-      int          ne_pad;  // nslices x slice_w
+      const float* es;      // ns soft-photon energies and distribution, as given
+      const float* fs;
+      float*       inv4es;  // ns, in the order of the sums: 1 / (4 e_s), inf for masked photons
+      float*       inv4es_min; // min over s of 1 / (4 e_s) (positive values), one float
+      float*       ws;      // ns: f_s / e_s
+      double*      terms;   // [6][ns]: w, w i, w i^2, w i ln i, ln i, 1 / i with i = 1 / (4 e_s)
+      int*         block_ok; // per block of ic_terms_kernel: its photons are in order and in range
+      int*         regular; // 1: the pair kernel runs, 0: the direct kernel
+      IcSums       sums;
       int          ns;
       const float* eic;     // ne IC photon energies
       int          ne;
-      int          nslices;
-      int          slice_w;  // IC bins per slice: K x 32
-      double*      partials; // [grid][nslices][slice_w]: one row per block
+      int          nslices; // direct kernel: slices of slice_w IC bins (K x 32)
+      int          slice_w;
+      double*      partials;  // direct kernel: [grid][nslices][slice_w], one row per block
+      double*      pairs;     // pair kernel: [splits][ne], one row per range of gamma bins
     };
 
-    // inv4es, ws and the smallest positive inv4es (positive floats order like their bit
-    // patterns, so an unsigned atomicMin finds it; the slot starts at +inf)
-    __global__ void ic_prep_kernel(const float* __restrict__ es, const float* __restrict__ fs, int ns,
-                                   float* __restrict__ inv4es, float* __restrict__ ws, unsigned* min_bits) {
-      const int s = blockIdx.x * blockDim.x + threadIdx.x;
-      if (s < ns) {
-        const float e  = es[s];
-        const bool  ok = e > 0.0f && isfinite(e); // non-positive soft-photon bins contribute nothing
-        const float i4 = ok ? __frcp_rn(__fmul_rn(4.0f, e)) : __int_as_float(0x7f800000); // q = inf: masked
-        inv4es[s]      = i4;
-        ws[s]          = ok ? __fdiv_rn(fs[s], e) : 0.0f;
-        if (ok && i4 > 0.0f) {
-          atomicMin(min_bits, __float_as_uint(i4));
+    // ---- soft-photon tables ---------------------------------------------------------------
+
+    constexpr int kPrepThreads = 256;
+    constexpr int kPrepItems   = 4; // photons per thread and tile
+    constexpr int kRankMax     = 16384; // photons that are ranked when they are out of order
+    constexpr int kRankTile    = 1024;
+    // energies and |weights| of a regular table: far enough from the ends of the float range for
+    // every double-float product of the pair kernel
+    constexpr float kRegularLo = 1e-30f, kRegularHi = 1e30f;
+
+    __device__ __forceinline__ ff ff_div(ff a, ff b) {
+      const float r  = __frcp_rn(b.hi);
+      const float q0 = __fmul_rn(a.hi, r);
+      const float e  = __fadd_rn(__fmaf_rn(-q0, b.hi, a.hi), __fmaf_rn(-q0, b.lo, a.lo));
+      return fast_two_sum(q0, __fmul_rn(e, r));
+    }
+
+    __device__ __forceinline__ double ff_to_double(ff a) {
+      return static_cast<double>(a.hi) + static_cast<double>(a.lo);
+    }
+
+    __device__ __forceinline__ float2 double_to_ff(double d) {
+      const float h = __double2float_rn(d);
+      return make_float2(h, isfinite(h) ? __double2float_rn(d - static_cast<double>(h)) : 0.0f);
+    }
+
+    // 1 / (4 e) of a valid photon energy, inf for one that contributes nothing (e <= 0, not
+    // finite, or 1 / (4 e) above the float range): masked photons come first in the order.
+    __device__ __forceinline__ float ic_inv4(float e) {
+      return (e > 0.0f && isfinite(e)) ? __frcp_rn(__fmul_rn(4.0f, e)) : __int_as_float(0x7f800000);
+    }
+
+    // Per photon (a thread each): its place in descending order of 1 / (4 e_s), and its terms of the
+    // four sums.  A table already in order keeps its places; one of up to kRankMax photons in any
+    // other order is ranked by comparing all pairs (ns^2 comparisons against ng x ne x ns evals of
+    // the direct kernel); a longer one is left to the direct kernel.  Quotients and logarithms are
+    // taken in double-floats, as FP64 issues at 1.6 operations per clock and SM.
+    __global__ void __launch_bounds__(kPrepThreads) ic_terms_kernel(const __grid_constant__ IcParams p) {
+      __shared__ float keys[kRankTile];
+      const int  s    = blockIdx.x * kPrepThreads + threadIdx.x;
+      const bool mine = s < p.ns;
+      const bool rank = p.ns <= kRankMax;
+      // in order over the whole table (each block decides for itself) or, above kRankMax, over
+      // this block's photons
+      bool out_of_order = false;
+      for (int k = rank ? static_cast<int>(threadIdx.x) : s; k + 1 < p.ns; k += kPrepThreads) {
+        out_of_order = out_of_order || ic_inv4(p.es[k]) < ic_inv4(p.es[k + 1]);
+        if (!rank) {
+          break;
+        }
+      }
+      const bool  unsorted = __syncthreads_or(out_of_order) != 0;
+      const float e = mine ? p.es[s] : 0.0f, f = mine ? p.fs[s] : 0.0f;
+      const float i4  = ic_inv4(e);
+      const bool  use = i4 <= 3.402823466e38f; // false for inf: a photon that contributes nothing
+      int         at  = s;
+      if (unsorted && rank) {
+        at = 0;
+        for (int t0 = 0; t0 < p.ns; t0 += kRankTile) {
+          const int m = min(kRankTile, p.ns - t0);
+          __syncthreads();
+          for (int k = threadIdx.x; k < m; k += kPrepThreads) {
+            keys[k] = ic_inv4(p.es[t0 + k]);
+          }
+          __syncthreads();
+          for (int k = 0; k < m; ++k) {
+            at += (keys[k] > i4 || (keys[k] == i4 && t0 + k < s)) ? 1 : 0;
+          }
+        }
+      }
+      bool ok = rank || !unsorted;
+      if (mine) {
+        const float wf = use ? __fdiv_rn(f, e) : 0.0f;
+        p.inv4es[at]   = i4;
+        p.ws[at]       = wf;
+        ok = ok && (!use || (e >= kRegularLo && e <= kRegularHi && fabsf(wf) <= kRegularHi));
+        double w = 0.0, i = 0.0, lni = 0.0, ri = 0.0;
+        ff     iv { i4, 0.0f };
+        if (use) {
+          iv              = ff_div(ff { 0.25f, 0.0f }, ff { e, 0.0f });
+          w               = ff_to_double(ff_div(ff { f, 0.0f }, ff { e, 0.0f }));
+          i               = ff_to_double(iv);
+          ri              = 4.0 * static_cast<double>(e);
+          const LnParts l = ln_parts(ff { e, 0.0f }); // ln i = -ln(4 e)
+          lni             = -((static_cast<double>(l.e) + 2.0) * M_LN2 + ff_to_double(ff { l.h, l.l }));
+        }
+        const double wi = w * i;
+        p.sums.i4[at]   = make_float2(iv.hi, iv.lo);
+        p.terms[at]             = w;
+        p.terms[p.ns + at]      = wi;
+        p.terms[2 * static_cast<int64_t>(p.ns) + at] = wi * i;
+        p.terms[3 * static_cast<int64_t>(p.ns) + at] = wi * lni;
+        p.terms[4 * static_cast<int64_t>(p.ns) + at] = lni;
+        p.terms[5 * static_cast<int64_t>(p.ns) + at] = ri;
+      }
+      const int all = __syncthreads_and(ok);
+      if (threadIdx.x == 0) {
+        p.block_ok[blockIdx.x] = all;
+      }
+    }
+
+    // One block per sum (blockIdx.x = 0: W0, 1: V1, 2: V2, 3: V3): the photons are walked from the
+    // end in tiles of 1024, a thread summing four consecutive ones, in FP64 (the sums' range
+    // exceeds FP32's); four SMs share the FP64 additions.  Block 0 also decides which kernel runs.
+    __global__ void __launch_bounds__(kPrepThreads) ic_sums_kernel(const __grid_constant__ IcParams p) {
+      __shared__ double wtot[2][kPrepThreads / 32];
+      __shared__ float  wmin[kPrepThreads / 32];
+      const int     which = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+      const int     tile = kPrepThreads * kPrepItems;
+      const int64_t ns   = p.ns;
+      double        carry = 0.0, carry1 = 0.0; // sums over the tiles done (carry1: V3's sum of w i)
+      for (int64_t r0 = 0; r0 < ns; r0 += tile) {
+        double a[kPrepItems], a1[kPrepItems];
+        double t = 0.0, t1 = 0.0;
+#pragma unroll
+        for (int k = 0; k < kPrepItems; ++k) {
+          const int64_t s = ns - 1 - (r0 + tid * kPrepItems + k);
+          a[k]  = s >= 0 ? p.terms[which * ns + s] : 0.0;
+          a1[k] = (s >= 0 && which == 3) ? p.terms[ns + s] : 0.0;
+          t += a[k];
+          t1 += a1[k];
+        }
+        // inclusive sums over the warp's threads
+        double x = t, x1 = t1;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const double y  = __shfl_up_sync(0xffffffffu, x, o);
+          const double y1 = which == 3 ? __shfl_up_sync(0xffffffffu, x1, o) : 0.0;
+          if (lane >= o) {
+            x += y;
+            x1 += y1;
+          }
+        }
+        if (lane == 31) {
+          wtot[0][warp] = x;
+          wtot[1][warp] = x1;
+        }
+        __syncthreads();
+        double before = carry, before1 = carry1;
+#pragma unroll
+        for (int w = 0; w < kPrepThreads / 32; ++w) {
+          if (w == warp) {
+            before  = carry;
+            before1 = carry1;
+          }
+          carry += wtot[0][w];
+          carry1 += wtot[1][w];
+        }
+        // the lane below holds this lane's exclusive sum within the warp
+        const double up = __shfl_up_sync(0xffffffffu, x, 1), up1 = __shfl_up_sync(0xffffffffu, x1, 1);
+        double       run = lane > 0 ? before + up : before, run1 = lane > 0 ? before1 + up1 : before1;
+        __syncthreads(); // wtot is reused by the next tile
+#pragma unroll
+        for (int k = 0; k < kPrepItems; ++k) {
+          const int64_t s = ns - 1 - (r0 + tid * kPrepItems + k);
+          run += a[k];
+          run1 += a1[k];
+          if (s >= 0) {
+            if (which == 0) {
+              p.sums.w0[s] = double_to_ff(run);
+            } else {
+              const double ri = p.terms[5 * ns + s];
+              if (which == 1) {
+                p.sums.v1[s] = double_to_ff(run * ri);
+              } else if (which == 2) {
+                p.sums.v2[s] = double_to_ff(run * ri * ri);
+              } else {
+                p.sums.v3[s] = double_to_ff((run - p.terms[4 * ns + s] * run1) * ri);
+              }
+            }
+          }
+        }
+      }
+      if (which == 0) {
+        bool  ok   = true;
+        float imin = __int_as_float(0x7f7f7f7f); // above any 1 / (4 e_s) of a positive float
+        for (int64_t s = tid; s < ns; s += kPrepThreads) {
+          const float i4 = p.inv4es[s];
+          imin           = i4 > 0.0f ? fminf(imin, i4) : imin;
+        }
+        for (int k = tid; k < (p.ns + kPrepThreads - 1) / kPrepThreads; k += kPrepThreads) {
+          ok = ok && p.block_ok[k] != 0;
+        }
+        const int all = __syncthreads_and(ok);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+          imin = fminf(imin, __shfl_xor_sync(0xffffffffu, imin, o));
+        }
+        if (lane == 0) {
+          wmin[warp] = imin;
+        }
+        __syncthreads();
+        if (tid == 0) {
+          for (int w = 1; w < kPrepThreads / 32; ++w) {
+            imin = fminf(imin, wmin[w]);
+          }
+          *p.inv4es_min = imin;
+          *p.regular    = all;
         }
       }
     }
@@ -114,22 +328,94 @@ namespace rg {
       return __fdiv_rn(1e-30f, *p.inv4es_min);
     }
 
-    // The pair setups of every (gamma bin, padded IC bin), once per call: the main kernel's
-    // items (gamma bin, 64 soft photons) would otherwise repeat them for every chunk.
-    __global__ void ic_setup_kernel(const __grid_constant__ IcParams p, float4* __restrict__ setup) {
-      const int64_t t = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-      if (t >= static_cast<int64_t>(p.ng) * p.ne_pad) {
+    // ---- regular soft photons: one (gamma bin, IC bin) pair per thread and step ---------------
+
+    // Lanes own IC bins, warps take gamma bins (every kIcWarps x gridDim.y-th one).
+    __global__ void __launch_bounds__(kIcThreads) ic_pair_kernel(const __grid_constant__ IcParams p) {
+      __shared__ double red[kIcWarps][32];
+      const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+      if (!*p.regular) {
         return;
       }
-      const int   g   = static_cast<int>(t / p.ne_pad), bin = static_cast<int>(t % p.ne_pad);
-      const float gv  = __ldg(p.gb + g);
-      // invalid gamma bins are skipped by the main kernel before it reads their row
-      setup[t] = (gv > 0.0f && isfinite(gv)) ? ic_pair_setup(ic_bin_energy(p, bin), gv, __frcp_rn(gv), ic_tg_floor(p))
-                                             : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+      const int   bin = blockIdx.x * 32 + lane;
+      const float e   = ic_bin_energy(p, bin);
+      const float ee  = __fmul_rn(e, e);
+      float       hi = 0.0f, lo = 0.0f;
+      for (int g = blockIdx.y * kIcWarps + warp; g < p.ng; g += kIcWarps * gridDim.y) {
+        const float gv = __ldg(p.gb + g), fv = __ldg(p.fp + g);
+        if (!(gv > 0.0f) || !isfinite(gv)) {
+          continue; // non-positive or non-finite gamma bins contribute nothing (warp-uniform)
+        }
+        ff S { 0.0f, 0.0f };
+        if (e > 0.0f && gv > e) {
+          const ff    t  = ff_div(ff { e, 0.0f }, two_sum(gv, -e));
+          const ff    z  = ff_div(t, ff { gv, 0.0f });
+          const float h  = __fdiv_rn(__fmul_rn(0.5f * t.hi, t.hi), __fadd_rn(1.0f, t.hi));
+          // the first photon with q <= 1 (1 / (4 e_s) descends)
+          int j = 0, n = p.ns;
+          while (j < n) {
+            const int mid = (j + n) >> 1;
+            if (__fmul_rn(z.hi, __ldg(p.inv4es + mid)) <= 1.0f) {
+              n = mid;
+            } else {
+              j = mid + 1;
+            }
+          }
+          ff q { 0.0f, 0.0f };
+          for (; j < p.ns; ++j) { // q in double-float: the float product may have rounded down to 1
+            const float2 iv = __ldg(p.sums.i4 + j);
+            q               = ff_mul(z, ff { iv.x, iv.y });
+            if (q.hi < 1.0f || (q.hi == 1.0f && q.lo <= 0.0f)) {
+              break;
+            }
+          }
+          if (j < p.ns) {
+            const float2 w0 = __ldg(p.sums.w0 + j), v1 = __ldg(p.sums.v1 + j);
+            const float2 v2 = __ldg(p.sums.v2 + j), v3 = __ldg(p.sums.v3 + j);
+            const ff     W0 { w0.x, w0.y }, V1 { v1.x, v1.y }, V2 { v2.x, v2.y }, V3 { v3.x, v3.y };
+            S               = W0;
+            if (q.hi >= 1e-30f) { // below, KN = 1 + h to rounding
+              const LnParts l  = ln_parts_rcp(q);
+              const float   fe = static_cast<float>(l.e);
+              // e ln2 with ln2 = 0.693145751953125 (16 bits: exact product) + 1.42860677e-6
+              ff ln  = two_sum(__fmul_rn(fe, 0.693145751953125f), l.h);
+              ln     = fast_two_sum(ln.hi, __fadd_rn(ln.lo, __fmaf_rn(fe, 1.4286068203094173e-6f, l.l)));
+              ff c   = ff_add(ff_mul(ln, V1), V3);
+              c      = ff_add(c, ff_neg(ff_mul(q, V2)));     // V1 ln q + V3 - q V2
+              c      = ff { 2.0f * c.hi, 2.0f * c.lo };
+              S      = ff_add(W0, ff_mul(q, ff_add(V1, c)));  // W0 + q V1 + 2 q (...)
+            }
+            const ff d = ff_add(W0, ff_neg(ff_mul(q, V1)));
+            S          = ff_add(S, ff_mul(ff { h, 0.0f }, d));
+          }
+        }
+        // times f_g / g^k and e^2, into the double-float sum
+        const float inv_g = __frcp_rn(gv);
+        const float fg    = p.log_spaced ? __fmul_rn(fv, inv_g) : __fmul_rn(__fmul_rn(fv, inv_g), inv_g);
+        const ff    term  = ff_mul(ff_mul(S, ff { fg, 0.0f }), ff { ee, 0.0f });
+        const ff    sm    = two_sum(hi, term.hi);
+        hi                = sm.hi;
+        lo                = __fadd_rn(lo, __fadd_rn(sm.lo, term.lo));
+      }
+      red[warp][lane] = static_cast<double>(hi) + static_cast<double>(lo);
+      __syncthreads();
+      if (warp == 0 && bin < p.ne) {
+        double t = 0.0;
+#pragma unroll
+        for (int w = 0; w < kIcWarps; ++w) {
+          t += red[w][lane];
+        }
+        p.pairs[static_cast<int64_t>(blockIdx.y) * p.ne + bin] = t;
+      }
     }
+
+    // ---- any soft photons: every (gamma bin, soft photon, IC bin) evaluated --------------------
 
     template <int K>
     __global__ void __launch_bounds__(kIcThreads, 2) ic_kernel(const __grid_constant__ IcParams p) {
+      if (*p.regular) {
+        return;
+      }
       const int     lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
       const int     slice = blockIdx.y;
       const int     nsc   = (p.ns + kIcSChunk - 1) / kIcSChunk;
@@ -159,13 +445,12 @@ namespace rg {
           continue; // non-positive or non-finite gamma bins contribute nothing (warp-uniform)
         }
         const float inv_g = __frcp_rn(gv);
-        // per (e, g): pg, 1 + h and the linear coefficient (ic_pair_setup), from the call's
-        // setup table when there is one; q = (t / g) / (4 e_s) > 1 marks no contribution
+        // per (e, g): pg, 1 + h and the linear coefficient (ic_pair_setup);
+        // q = (t / g) / (4 e_s) > 1 marks no contribution
         float pg[K], A0[K], B1[K], acc[K];
-        const float4* su = p.setup ? p.setup + static_cast<int64_t>(g) * p.ne_pad + slice * (K * 32) + lane : nullptr;
 #pragma unroll
         for (int k = 0; k < K; ++k) {
-          const float4 v = su ? __ldg(su + k * 32) : ic_pair_setup(energy(k), gv, inv_g, tg_floor);
+          const float4 v = ic_pair_setup(energy(k), gv, inv_g, tg_floor);
           pg[k]  = v.x;
           A0[k]  = v.y;
           B1[k]  = v.z;
@@ -214,24 +499,28 @@ namespace rg {
       }
     }
 
-    // out[e] = sum over blocks (fixed order) of the partial rows; 32 bins x 32 row groups.
+    // out[e] = sum (fixed order) over the partial rows of the kernel that ran: `splits` rows of
+    // ne bins (pair kernel) or `grid` rows of slices (direct kernel); 32 bins x 32 row groups.
     __global__ void __launch_bounds__(1024)
-      ic_reduce_kernel(const double* __restrict__ partials, int grid, int nslices, int slice_w, int ne,
-                       float* __restrict__ out) {
+      ic_reduce_kernel(const __grid_constant__ IcParams p, int splits, int grid, float* __restrict__ out) {
       __shared__ double part[32][33];
       const int bin = blockIdx.x * 32 + threadIdx.x, ty = threadIdx.y;
       double    sum = 0.0;
-      if (bin < ne) {
-        const int slice = bin / slice_w, j = bin % slice_w;
+      if (bin < p.ne) {
+        const bool    pairs = *p.regular != 0;
+        const int     rows  = pairs ? splits : grid;
+        const double* src   = pairs ? p.pairs + bin
+                                    : p.partials + static_cast<int64_t>(bin / p.slice_w) * p.slice_w + bin % p.slice_w;
+        const int64_t step  = pairs ? p.ne : static_cast<int64_t>(p.nslices) * p.slice_w;
         // unrolled so that several rows' loads are in flight (the adds stay in row order)
 #pragma unroll 8
-        for (int r = ty; r < grid; r += 32) {
-          sum += partials[(static_cast<int64_t>(r) * nslices + slice) * slice_w + j];
+        for (int r = ty; r < rows; r += 32) {
+          sum += src[r * step];
         }
       }
       part[ty][threadIdx.x] = sum;
       __syncthreads();
-      if (ty == 0 && bin < ne) {
+      if (ty == 0 && bin < p.ne) {
         double t = 0.0;
         for (int y = 0; y < 32; ++y) {
           t += part[y][threadIdx.x];
@@ -289,53 +578,57 @@ int rg_ic_spectrum(const float* gbins, const float* f, int32_t ng, int32_t log_s
   const int64_t items   = static_cast<int64_t>(ng) * ((ns + rg::kIcSChunk - 1) / rg::kIcSChunk);
   const int     grid    = static_cast<int>(std::max<int64_t>(
     1, std::min<int64_t>(2 * ctx->sms, (items + rg::kIcWarps - 1) / rg::kIcWarps)));
-  // one stream-ordered scratch allocation: inv4es, ws, partials
-  const size_t off_ws   = 256 * ((sizeof(float) * ns + 255) / 256);
-  const size_t off_min  = off_ws + 256 * ((sizeof(float) * ns + 255) / 256);
-  const size_t off_part = off_min + 256;
-  // the (gamma bin, IC bin) setup table when it is small (it is 16 bytes per pair)
-  const int64_t ne_pad    = static_cast<int64_t>(nslices) * slice_w;
-  const size_t  set_bytes = sizeof(float4) * static_cast<size_t>(ng) * static_cast<size_t>(ne_pad);
-  const bool    use_setup = set_bytes <= (size_t(64) << 20);
-  const size_t  off_set   = 256 * ((off_part + sizeof(double) * static_cast<size_t>(grid) * nslices * slice_w + 255) / 256);
-  const size_t  bytes     = off_set + (use_setup ? set_bytes : 0);
-  unsigned char* buf    = nullptr;
+  // ranges of gamma bins of the pair kernel: about four blocks per SM, each warp at least one bin
+  const int col_blocks = (ne + 31) / 32;
+  const int splits     = std::max(1, std::min((ng + rg::kIcWarps - 1) / rg::kIcWarps,
+                                              (4 * ctx->sms + col_blocks - 1) / col_blocks));
+  // one stream-ordered scratch allocation: photon arrays, sums, partial rows
+  const auto     up       = [](size_t v) { return 256 * ((v + 255) / 256); };
+  const size_t   n4 = up(sizeof(float) * ns), n8 = up(sizeof(float2) * ns), n48 = up(sizeof(double) * 6 * ns);
+  const int      term_blocks = (ns + rg::kPrepThreads - 1) / rg::kPrepThreads;
+  const size_t   off_sums = 2 * n4, off_terms = off_sums + 5 * n8, off_min = off_terms + n48;
+  const size_t   off_ok = off_min + 256, off_pairs = off_ok + up(sizeof(int) * term_blocks);
+  const size_t   off_part = off_pairs + up(sizeof(double) * static_cast<size_t>(splits) * ne);
+  const size_t   bytes    = off_part + sizeof(double) * static_cast<size_t>(grid) * nslices * slice_w;
+  unsigned char* buf      = nullptr;
   RG_CUDA_TRY(cudaMallocAsync(reinterpret_cast<void**>(&buf), bytes, s));
   rg::IcParams p {};
   p.gb         = gbins;
   p.fp         = f;
   p.ng         = ng;
   p.log_spaced = log_spaced ? 1 : 0;
+  p.es         = es;
+  p.fs         = fs;
   p.inv4es     = reinterpret_cast<float*>(buf);
-  p.ws         = reinterpret_cast<float*>(buf + off_ws);
+  p.ws         = reinterpret_cast<float*>(buf + n4);
+  float2** sums[5] = { &p.sums.i4, &p.sums.w0, &p.sums.v1, &p.sums.v2, &p.sums.v3 };
+  for (int k = 0; k < 5; ++k) {
+    *sums[k] = reinterpret_cast<float2*>(buf + off_sums + k * n8);
+  }
+  p.terms      = reinterpret_cast<double*>(buf + off_terms);
+  p.block_ok   = reinterpret_cast<int*>(buf + off_ok);
+  p.inv4es_min = reinterpret_cast<float*>(buf + off_min);
+  p.regular    = reinterpret_cast<int*>(buf + off_min + 128);
   p.ns         = ns;
   p.eic        = eic;
   p.ne         = ne;
   p.nslices    = nslices;
   p.slice_w    = slice_w;
+  p.pairs      = reinterpret_cast<double*>(buf + off_pairs);
   p.partials   = reinterpret_cast<double*>(buf + off_part);
-  p.ne_pad     = static_cast<int>(ne_pad);
-  p.setup      = nullptr;
-  p.inv4es_min = reinterpret_cast<float*>(buf + off_min);
-  // the minimum slot starts at 0x7f7f7f7f (3.4e38, above any 1 / (4 e_s) of a positive float)
-  cudaError_t e = cudaMemsetAsync(buf + off_min, 0x7f, sizeof(unsigned), s);
+  rg::ic_terms_kernel<<<term_blocks, rg::kPrepThreads, 0, s>>>(p);
+  cudaError_t e = cudaGetLastError();
   if (e == cudaSuccess) {
-    rg::ic_prep_kernel<<<(ns + 255) / 256, 256, 0, s>>>(es, fs, ns, reinterpret_cast<float*>(buf),
-                                                         reinterpret_cast<float*>(buf + off_ws),
-                                                         reinterpret_cast<unsigned*>(buf + off_min));
+    rg::ic_sums_kernel<<<4, rg::kPrepThreads, 0, s>>>(p);
     e = cudaGetLastError();
   }
-  if (e == cudaSuccess && use_setup) {
-    auto* setup  = reinterpret_cast<float4*>(buf + off_set);
-    const int64_t pairs = static_cast<int64_t>(ng) * ne_pad;
-    rg::ic_setup_kernel<<<static_cast<unsigned>((pairs + 255) / 256), 256, 0, s>>>(p, setup);
-    e       = cudaGetLastError();
-    p.setup = setup;
+  if (e == cudaSuccess) {
+    rg::ic_pair_kernel<<<dim3(col_blocks, splits), rg::kIcThreads, 0, s>>>(p);
+    e = cudaGetLastError();
   }
   if (e == cudaSuccess) e = rg::launch_ic(K, p, dim3(grid, nslices), s);
   if (e == cudaSuccess) {
-    rg::ic_reduce_kernel<<<dim3((ne + 31) / 32), dim3(32, 32), 0, s>>>(p.partials, grid, nslices, slice_w, ne,
-                                                                        out);
+    rg::ic_reduce_kernel<<<col_blocks, dim3(32, 32), 0, s>>>(p, splits, grid, out);
     e = cudaGetLastError();
   }
   const cudaError_t ef = cudaFreeAsync(buf, s);

@@ -130,3 +130,54 @@ def test_dropin_module(gpu, oracle_lib):
                                                            rg.DeltaGenerator(1e-8, 1e-9)), bins)
     with pytest.raises(RuntimeError, match="E_ic must be in units of mec\\^2"):
         rg.ICSpectrum(dist_prtls, dist_soft, rg.Bins(rg.Logspace(1e3, 1e7, 200)))
+
+
+@pytest.mark.parametrize("ns,width", [(1, 1.0), (2, 1e-3), (33, 1e-2), (1023, 6.0), (1025, 6.0), (4100, 12.0)])
+def test_photon_orders(gpu, oracle_lib, ns, width):
+    """Soft photons in ascending and in any order (suffix sums, one (gamma bin, IC bin) pair at
+    a time) within the spectrum tolerance of FP64, around the 1024-photon tiles of the sums,
+    from a single photon (one Klein-Nishina edge per IC bin) to 12 decades."""
+    rng = np.random.default_rng(ns)
+    gb = oracle_lib.logspace(10.0, 1e6, 301)
+    fp = (gb.astype(np.float64) ** -2.0).astype(np.float32)
+    es = oracle_lib.logspace(1e-8, 1e-8 * 10.0**width, ns)
+    fs = (rng.uniform(0.5, 1.5, ns) * es.astype(np.float64) ** -0.5).astype(np.float32)
+    fs[rng.random(ns) < 0.2] = 0.0
+    fs[-1] = 1.0
+    eic = oracle_lib.logspace(1e-3, 1e6, 333)
+    want = oracle_lib.ic_spectrum_f64(gb, fp, True, es, fs, eic)
+    assert max_rel(gpu_ic(gb, fp, True, es, fs, eic, gpu), want) <= SPECTRUM_RTOL
+    order = rng.permutation(ns)
+    assert max_rel(gpu_ic(gb, fp, True, es[order], fs[order], eic, gpu), want) <= SPECTRUM_RTOL
+    # photons below zero before the first valid one are masked, on the same route
+    got = gpu_ic(gb, fp, True, np.concatenate([[-1.0, 0.0], es]), np.concatenate([[1.0, 1.0], fs]), eic, gpu)
+    assert max_rel(got, want) <= SPECTRUM_RTOL
+
+
+def test_out_of_order_photons_above_the_ranked_count(gpu, oracle_lib):
+    """16385 photons out of order: the direct kernel; in order: the sums."""
+    ns = 16385
+    rng = np.random.default_rng(ns)
+    gb = oracle_lib.logspace(1e2, 1e5, 40)
+    fp = (gb.astype(np.float64) ** -2.0).astype(np.float32)
+    es = oracle_lib.logspace(1e-8, 1e-3, ns)
+    fs = (rng.uniform(0.5, 1.5, ns) * es.astype(np.float64) ** -0.5).astype(np.float32)
+    eic = oracle_lib.logspace(1e-2, 1e5, 70)
+    want = oracle_lib.ic_spectrum_f64(gb, fp, True, es, fs, eic)
+    order = rng.permutation(ns)
+    assert max_rel(gpu_ic(gb, fp, True, es, fs, eic, gpu), want) <= SPECTRUM_RTOL
+    assert max_rel(gpu_ic(gb, fp, True, es[order], fs[order], eic, gpu), want) <= SPECTRUM_RTOL
+
+
+def test_non_finite_photon_weights_spread_as_before(gpu, oracle_lib):
+    """A NaN or infinite photon weight makes the table irregular: the direct kernel's products
+    (0 x inf and NaN terms) then reach every IC bin a gamma bin reaches."""
+    gb = oracle_lib.logspace(1e3, 1e5, 64)
+    fp = np.ones(64, np.float32)
+    es = oracle_lib.logspace(1e-9, 1e-7, 40)
+    eic = oracle_lib.logspace(1e2, 9e4, 50)
+    for bad in (np.nan, np.inf):
+        fs = np.ones(40, np.float32)
+        fs[7] = bad
+        got = gpu_ic(gb, fp, True, es, fs, eic, gpu)
+        assert not np.any(np.isfinite(got))
