@@ -79,33 +79,6 @@ namespace rg {
     return __longlong_as_double(static_cast<long long>(d));
   }
 
-  // a r as a double for a float a of normal magnitude (either sign) and an integer
-  // 0 <= r < 2^30: the 24-bit mantissa times r is an exact integer below 2^54,
-  // rounded to 53 bits.
-  __device__ __forceinline__ double product_to_double_bits(float a, uint32_t r) {
-    if (r == 0) {
-      return 0.0;
-    }
-    const uint32_t b   = __float_as_uint(a);
-    const uint64_t P   = static_cast<uint64_t>((b & 0x7fffffu) | 0x800000u) * r;
-    int            top = 63 - __clzll(static_cast<long long>(P)); // leading bit position, <= 53
-    uint64_t       mant;
-    if (top <= 52) {
-      mant = P << (52 - top);
-    } else { // 54 significant bits: round to nearest (ties up)
-      mant = (P + 1) >> 1;
-      if (mant >> 53) {
-        mant >>= 1;
-        ++top;
-      }
-    }
-    // |value| = P 2^(E - 150) with E the float's biased exponent
-    const int64_t  e = static_cast<int64_t>(top) + static_cast<int64_t>((b >> 23) & 0xffu) - 150 + 1023;
-    const uint64_t d = (static_cast<uint64_t>(b >> 31) << 63) | (static_cast<uint64_t>(e) << 52) |
-                       (mant & ((uint64_t(1) << 52) - 1));
-    return __longlong_as_double(static_cast<long long>(d));
-  }
-
   // FP64 atomic add of a float: values of normal magnitude take the integer-built
   // operand, subnormals the FP64 pipe, zeros nothing.
   __device__ __forceinline__ void red_add_float(double* dst, float v) {

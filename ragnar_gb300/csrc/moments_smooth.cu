@@ -150,17 +150,19 @@ namespace rg {
     }
 
     // Sums each cell's sub-cells into the compact cell table cells[seg][cell][4] (thread per
-    // (segment, cell, moment)).
-    __global__ void smooth_fold_kernel(const double* __restrict__ hist, int64_t cells_total, double* __restrict__ cells) {
+    // (segment, cell, moment))
+    // and clears them for the next run.
+    __global__ void smooth_fold_kernel(double* __restrict__ hist, int64_t cells_total, double* __restrict__ cells) {
       const int64_t t = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
       if (t >= cells_total * 4) {
         return;
       }
-      const double* h = hist + (t >> 2) * kSub * 4 + (t & 3);
-      double        s = 0.0;
+      double* h = hist + (t >> 2) * kSub * 4 + (t & 3);
+      double  s = 0.0;
 #pragma unroll
       for (int k = 0; k < kSub; ++k) {
         s += h[k * 4];
+        h[k * 4] = 0.0;
       }
       cells[t] = s;
     }
@@ -553,7 +555,7 @@ namespace rg {
     const int64_t cells_total = static_cast<int64_t>(nseg) * pl->sm_cells;
     RG_TRY(smooth_reserve_cells(pl, static_cast<size_t>(cells_total)));
     smooth_fold_kernel<<<static_cast<int>((cells_total * 4 + 255) / 256), 256, 0, s>>>(
-      reinterpret_cast<const double*>(pl->d_hist), cells_total, pl->d_cells);
+      reinterpret_cast<double*>(pl->d_hist), cells_total, pl->d_cells);
     RG_CUDA_TRY(cudaGetLastError());
     SmoothReduceParams r {};
     r.cells    = pl->d_cells;
@@ -567,6 +569,7 @@ namespace rg {
     r.out      = out;
     smooth_reduce_kernel<<<dim3(pl->nbins, nseg), kSmRedThreads, 0, s>>>(r);
     RG_CUDA_TRY(cudaGetLastError());
+    pl->hist_dirty = false;
     return RG_OK;
   }
 

@@ -735,12 +735,10 @@ namespace rg {
     // the interval moments of max_seg segments, so that runs allocate nothing (and can be
     // captured in a CUDA graph)
     if (moments_selected(pl, max_seg)) {
-      const size_t need = static_cast<size_t>(max_seg) * static_cast<size_t>(pl->hist_per_seg);
-      if (need > pl->hist_cap) {
-        cudaFree(pl->d_hist);
-        pl->d_hist = nullptr;
-        RG_CUDA_TRY(cudaMalloc(&pl->d_hist, sizeof(double2) * need));
-        pl->hist_cap = need;
+      const size_t cap = pl->hist_cap, sums = pl->msum_cap;
+      RG_TRY(moments_reserve(pl, max_seg, nullptr));
+      if (pl->hist_cap != cap || pl->msum_cap != sums) {
+        RG_CUDA_TRY(cudaStreamSynchronize(nullptr)); // zeroed before any stream's run
       }
       // the smooth moment path's per-cell scratch (folded moments, adjoint cubics)
       if (pl->aligned) {

@@ -47,12 +47,21 @@ struct rg_spectrum_plan {
   int64_t*              d_mrange    = nullptr; // per slice: (Pmin, Pmax) in the finer coordinate
   int64_t               mom_L       = 0;       // table segments in the finer coordinate
   int32_t*              d_thr       = nullptr; // per slice: sorted low parts of Pmax - P_b (kSliceBins)
-  uint16_t*             d_bucket    = nullptr; // per slice: first threshold of each bucket (kMomBuckets + 1)
-  int4*                 d_binfo     = nullptr; // per bin: (sorted position, cell offset, low part, valid)
-  double2*              d_mcoef     = nullptr; // per table segment: FP64 (c0, c1 per fraction bit)
+  uint32_t*             d_bucket    = nullptr; // per slice: rank table of the low parts (kMomBuckets)
+  int4*                 d_binfo     = nullptr; // per bin: (sorted position, cell offset, low part, bin) by cell offset;
+                                               // smooth: (cell offset, residual, 0, valid)
+  float4*               d_mcoef     = nullptr; // -1 .. segments: (c0, c1) as double-floats
   int64_t               hist_per_seg = 0;      // double2 entries of one segment's histograms
-  double2*              d_hist      = nullptr;
+  double2*              d_hist      = nullptr; // zero between runs (the finish kernels clear what they read)
   size_t                hist_cap    = 0;       // double2 entries
+  double*               d_msum      = nullptr; // per (segment, slice): bin sums, then block counts; zero between runs
+  size_t                msum_cap    = 0;       // (segment, slice) pairs
+  bool                  hist_dirty  = false;   // a run has deposited and not finished
+  // fixed-point logarithm of the pair stage (pair_stage.cuh)
+  int64_t*              d_logt      = nullptr;
+  int                   log_fx      = 0;
+  float                 log_Sh = 0, log_Sl = 0;
+  int64_t               log_Cfx     = 0;
   // smooth table aligned to log-uniform bins (moments_smooth.cu)
   rg::SmoothTable       own_smooth;            // the plan's own table when `aligned`
   bool                  aligned     = false;
@@ -86,6 +95,8 @@ namespace rg {
   int  moments_prepare(rg_spectrum_plan* pl, const std::vector<uint8_t>& valid, double ln_xmin, double dln,
                        double ln_k0);
   bool moments_selected(const rg_spectrum_plan* pl, int nseg);
+  int  moments_reserve(rg_spectrum_plan* pl, int nseg, cudaStream_t s);
+  int  fixed_log_prepare(rg_spectrum_plan* pl, int F, double dln);
   int  moments_begin(rg_spectrum_plan* pl, int nseg, cudaStream_t s);
   int  moments_deposit(rg_spectrum_plan* pl, const float* const comp[10], const int64_t* d_off, int64_t n,
                        int nseg, cudaStream_t s);

@@ -155,3 +155,28 @@ def test_negative_amplitudes(gpu, oracle_lib, table, B0, eps, negw):
     for algo, got in res.items():
         # signed sums can cancel: compare against the largest magnitude
         assert np.max(np.abs(got - truth)) <= SPECTRUM_RTOL * scale, algo
+
+
+@pytest.mark.parametrize("n,nbins", [(1, 1), (255, 31), (257, 32), (512, 63), (513, 200), (1023, 512), (1025, 513),
+                                     (3001, 700)])
+@pytest.mark.parametrize("wscale", [1.0, 1e-33, 1e31])
+def test_moments_edges_of_steps_and_rows(gpu, oracle_lib, table, n, nbins, wscale):
+    """Particle counts around the deposit's 512-particle steps, bin counts around the finish's
+    32-entry lanes and 512-bin slices, streams that start off a 16-byte boundary, and weights
+    near both ends of the float range, against FP64."""
+    P = particles(n + 1, seed=n + nbins, bfield="iso", weights=True, umax=1e3)
+    P = {k: v[1:] for k, v in P.items()}
+    P["w"] = (P["w"] * np.float32(wscale)).astype(np.float32)
+    bins = oracle_lib.logspace(1e-2, 1e6, nbins) if nbins > 1 else np.array([3.0], np.float32)
+    full = {k: torch.zeros(n + 1, device=gpu) for k in P}
+    for k, v in P.items():
+        full[k][1:] = torch.from_numpy(np.ascontiguousarray(v)).to(gpu)
+    T = {k: v[1:] for k, v in full.items()}
+    prt = capi.particles([T["ux"], T["uy"], T["uz"]], b=[T["bx"], T["by"], T["bz"]], w=T["w"], n=n)
+    plan = capi.SpectrumPlan(bins, 1.0, 1.0, 1.0)
+    out = torch.full((nbins,), -1.0, device=gpu)
+    for _ in range(2):  # the tables are clear again after a run
+        plan.run(prt, out)
+    plan.check()
+    truth = oracle_lib.sync_spectrum_f64(P, bins, 1.0, 1.0, 1.0, table)
+    assert max_rel(out.cpu().numpy(), truth) <= SPECTRUM_RTOL
