@@ -52,25 +52,17 @@ namespace rg {
     constexpr int kMomExtra      = 8;                // bits below them before rounding (LogParams::fx)
     constexpr int kMomBuckets    = 4096;             // buckets over the low kMomFrac bits
     constexpr int kMomBucketBits = kMomFrac - 12;
-    constexpr int kMomSharedSeg  = 1024;             // segment offsets staged in shared memory
-    constexpr int kMomThreads    = 256;
-    constexpr int kMomChunk      = 2 * kMomThreads;  // particles per block and step
+    constexpr int kMomSharedSeg  = kPairSharedSeg;   // largest run in segments
     constexpr int kMomBlocksPerSM = 2;
-    constexpr int64_t kMomWindow = int64_t(1) << 31; // particles per launch
     constexpr int kMomMaxTable   = 256;              // largest reference table (segments) this path takes
     constexpr size_t kMomMaxBytes = size_t(8) << 30; // histogram memory above which the fused kernel runs
-    constexpr uint32_t kNoEntry  = 0xffffffffu;
 
     struct MomentParams {
-      FusedParams     fp;      // streams, kinematics constants, status
-      LogParams       log;     // base is formed per slice from range
+      FusedParams     fp;      // kinematics constants, status
+      LogParams       log;
       const int64_t*  range;   // per slice: (Pmin, Pmax) in kMomFrac units
       int64_t         L;       // table segments << kMomFrac
-      const int64_t*  seg_off; // nseg + 1 particle offsets (device), or null: particles [0, n)
-      int             nseg;
-      int64_t         n;       // stream length
-      int64_t         window;  // this launch takes particles [window, window + kMomWindow); fp.comp points at the first
-      uint32_t        stride[kComps]; // bytes between particles: 4, or 0 for a stream that is not given
+      PairStreams     in;
       const int4*     mslice;  // per slice: (valid bins, cells, histogram offset, 0)
       const int32_t*  thr;     // per slice: kSliceBins sorted low parts
       const uint32_t* bucket;  // per slice: kMomBuckets entries (bucket_entry)
@@ -101,12 +93,6 @@ namespace rg {
         }
       }
       return lo;
-    }
-
-    __device__ __forceinline__ void red_add_if(bool on, double* p, double v) {
-      asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %2, 0;\n\t@q red.global.add.f64 [%0], %1;\n\t}" ::"l"(p), "d"(v),
-                   "r"(static_cast<uint32_t>(on))
-                   : "memory");
     }
 
     // Adds (M0, M1) = (A, A Rl) of every lane's particle (idx: its entry, kNoEntry for none) to the
@@ -142,35 +128,18 @@ namespace rg {
     // and the loads behind them set its pace.  Also measured: three blocks per SM 0.95 ms, loads
     // staged through shared memory by cp.async 0.93 ms, entries scattered over the table no gain.
     template <bool kE, bool kSeg>
-    __global__ void __launch_bounds__(kMomThreads, kMomBlocksPerSM)
+    __global__ void __launch_bounds__(kPairThreads, kMomBlocksPerSM)
       moments_deposit_kernel(const __grid_constant__ MomentParams m) {
       __shared__ __align__(16) uint32_t bucket[kMomBuckets]; // staged 16 bytes at a time
       __shared__ int64_t                logt[kLogEntries];
       __shared__ uint32_t               soff[kSeg ? kMomSharedSeg + 1 : 1];
       const int  slice = blockIdx.y;
       const int4 ms    = m.mslice[slice];
-      stage_log_table(m.log, kMomExtra, m.range[2 * slice + 1], logt, kMomThreads);
-      for (int i = threadIdx.x; i < kMomBuckets / 4; i += kMomThreads) {
+      stage_log_table(m.log, kMomExtra, m.range[2 * slice + 1], logt, kPairThreads);
+      for (int i = threadIdx.x; i < kMomBuckets / 4; i += kPairThreads) {
         reinterpret_cast<uint4*>(bucket)[i] = reinterpret_cast<const uint4*>(m.bucket + slice * kMomBuckets)[i];
       }
-      // the window's particles as offsets from its start; the segments' offsets clamped to it
-      const int64_t w0 = m.window, w1 = min(m.n, w0 + kMomWindow);
-      bool          bad = false;
-      if (kSeg) {
-        for (int i = threadIdx.x; i <= m.nseg; i += kMomThreads) {
-          // offsets must not decrease and must lie in [0, n]
-          const int64_t o = m.seg_off[i];
-          bad             = bad || o < 0 || o > m.n || (i > 0 && o < m.seg_off[i - 1]);
-          soff[i]         = static_cast<uint32_t>(max(min(o, w1), w0) - w0);
-        }
-      }
-      if (__syncthreads_or(bad)) {
-        if (threadIdx.x == 0 && blockIdx.x == 0 && slice == 0) {
-          atomicOr(m.fp.status, kDevBadOffsets);
-        }
-        return;
-      }
-      if (__syncthreads_or(*m.fp.status != kDevOk)) {
+      if (!stage_segments<kSeg>(m.in, m.fp.status, soff)) {
         return;
       }
       const int64_t  Pmin = m.range[2 * slice], Pmax = m.range[2 * slice + 1];
@@ -179,41 +148,14 @@ namespace rg {
       LogParams      lg  = m.log;
       lg.fx              = kMomExtra;
       const uint32_t first = kSeg ? soff[0] : 0u;
-      const uint32_t last  = kSeg ? soff[m.nseg] : static_cast<uint32_t>(w1 - w0);
-      const uint32_t step  = gridDim.x * kMomChunk, tid = threadIdx.x;
+      const uint32_t last  = kSeg ? soff[m.in.nseg] : static_cast<uint32_t>(min(m.in.n - m.in.window, kPairWindow));
+      const uint32_t step  = gridDim.x * kPairChunk, tid = threadIdx.x;
 
       constexpr int kSets = kE ? 2 : 3; // with E a third set spills (64.2 us against 60.5 for 4.3e6 particles)
-      using Loaded        = float2[kComps];
-      auto load = [&](uint32_t base, Loaded& to) {
-        if (base + kMomChunk <= last) {
-#pragma unroll
-          for (int c = 0; c < kComps; ++c) {
-            if (kE || c < 3 || c >= 6) {
-              const float* q = reinterpret_cast<const float*>(reinterpret_cast<const char*>(m.fp.comp[c]) +
-                                                              static_cast<uint64_t>(base + tid) * m.stride[c]);
-              to[c].x        = __ldg(q);
-              to[c].y        = __ldg(q + kMomThreads);
-            }
-          }
-        } else if (base < last) { // the last step: past the end, the last particle again (dropped by its index)
-          const uint32_t i0 = min(base + tid, last - 1), i1 = min(base + tid + kMomThreads, last - 1);
-#pragma unroll
-          for (int c = 0; c < kComps; ++c) {
-            if (kE || c < 3 || c >= 6) {
-              const char* q = reinterpret_cast<const char*>(m.fp.comp[c]);
-              to[c].x       = __ldg(reinterpret_cast<const float*>(q + static_cast<uint64_t>(i0) * m.stride[c]));
-              to[c].y       = __ldg(reinterpret_cast<const float*>(q + static_cast<uint64_t>(i1) * m.stride[c]));
-            }
-          }
-        }
-      };
       uint32_t useg = 0, uend = kSeg ? soff[1] : last; // the segment of the step's first particle, and its end
-      auto     add  = [&](uint32_t base, const Loaded& from) {
+      auto     add  = [&](uint32_t base, const float2 (&from)[kComps]) {
         f2 v[kComps];
-#pragma unroll
-        for (int c = 0; c < kComps; ++c) {
-          v[c] = (kE || c < 3 || c >= 6) ? pack2(from[c].x, from[c].y) : set2(0.0f);
-        }
+        to_pairs<kE>(from, v);
         const Place2 pl = place2<kE>(v, m.fp, lg, logt, Pmin, Pmax, m.L);
         if (kSeg) {
           while (uend <= base) { // base < last = soff[nseg]
@@ -243,10 +185,10 @@ namespace rg {
           idx[j] += origin + Rc[j] * row;
           idx[j] = Rc[j] < nc && emits(pl.A[j]) ? idx[j] : kNoEntry;
         }
-        if (base + kMomChunk > (kSeg ? uend : last)) { // the step crosses an end of its segment or of the particles
+        if (base + kPairChunk > (kSeg ? uend : last)) { // the step crosses an end of its segment or of the particles
 #pragma unroll
           for (int j = 0; j < 2; ++j) {
-            const uint32_t i = base + tid + j * kMomThreads;
+            const uint32_t i = base + tid + j * kPairThreads;
             if (i >= last) {
               idx[j] = kNoEntry;
             } else if (kSeg && idx[j] != kNoEntry) {
@@ -260,16 +202,16 @@ namespace rg {
         red_pair(m.hist, idx[0], pl.A[0], Rl[0]);
         red_pair(m.hist, idx[1], pl.A[1], Rl[1]);
       };
-      Loaded   set[kSets];
-      uint32_t base = first + blockIdx.x * kMomChunk;
+      float2   set[kSets][kComps];
+      uint32_t base = first + blockIdx.x * kPairChunk;
 #pragma unroll
       for (int k = 0; k < kSets - 1; ++k) {
-        load(base + k * step, set[k]);
+        load_pair<kE>(m.in, base + k * step, last, set[k]);
       }
       while (base < last) {
 #pragma unroll
         for (int k = 0; k < kSets; ++k) {
-          load(base + (kSets - 1) * step, set[(k + kSets - 1) % kSets]);
+          load_pair<kE>(m.in, base + (kSets - 1) * step, last, set[(k + kSets - 1) % kSets]);
           add(base, set[k]);
           base += step;
           if (base >= last) {
@@ -317,31 +259,12 @@ namespace rg {
              kFinWarps * (sizeof(float2) * kSliceBins + sizeof(float4) * bufs * row);
     }
 
-    // d 2^-k as (hi, lo): the top 24 significant bits cut, then the 29 below; 0 when d 2^-k < 2^-126
-    // (GB300's FP64 pipe would take longer over the subtraction d - hi than these integer steps).
-    __device__ __forceinline__ float2 split_double(double d, int k) {
-      const uint32_t h = static_cast<uint32_t>(__double2hiint(d)), l = static_cast<uint32_t>(__double2loint(d));
-      const int      e = static_cast<int>((h >> 20) & 0x7ffu) - 1023 + 127 - k; // biased FP32 exponent
-      const uint32_t sign = h & 0x80000000u;
-      float2         r;
-      r.x = __uint_as_float(sign | (static_cast<uint32_t>(e) << 23) | (__funnelshift_l(l, h, 3) & 0x7fffffu));
-      r.y = static_cast<float>(l & 0x1fffffffu) * __uint_as_float(sign | (static_cast<uint32_t>(e - 52) << 23));
-      r.y = e > 52 ? r.y : 0.0f;
-      return e >= 1 ? r : make_float2(0.0f, 0.0f);
-    }
-
     __device__ __forceinline__ ff2 shfl_up_ff2(ff2 a, int o) {
       return { { __shfl_up_sync(0xffffffffu, a.hi.v, o) }, { __shfl_up_sync(0xffffffffu, a.lo.v, o) } };
     }
 
     __device__ __forceinline__ ff2 shfl_down_ff2(ff2 a, int o) {
       return { { __shfl_down_sync(0xffffffffu, a.hi.v, o) }, { __shfl_down_sync(0xffffffffu, a.lo.v, o) } };
-    }
-
-    __device__ __forceinline__ ff2 ff_mul2(ff2 a, ff2 b) {
-      const f2 p = mul2(a.hi, b.hi);
-      const f2 e = sub2(fma2(a.hi, b.lo, mul2(a.lo, b.hi)), fma2(neg2(a.hi), b.hi, p));
-      return fast_two_sum2(p, e);
     }
 
     __device__ __forceinline__ void store_ff2(float4* to, ff2 a) {
@@ -788,9 +711,6 @@ namespace rg {
     fill_params(pl, comp, nullptr, nullptr, n, 1, m.fp);
     m.range   = pl->d_mrange;
     m.L       = pl->mom_L;
-    m.seg_off = d_off;
-    m.nseg    = d_off ? nseg : 1;
-    m.n       = n;
     m.mslice  = reinterpret_cast<const int4*>(pl->d_mslice);
     m.thr     = pl->d_thr;
     m.bucket  = pl->d_bucket;
@@ -799,9 +719,6 @@ namespace rg {
     fill_log_params(pl, m.log);
     DeviceContext* ctx = nullptr;
     RG_TRY(context(&ctx));
-    for (int c = 0; c < kComps; ++c) {
-      m.stride[c] = comp[c] ? 4u : 0u;
-    }
     if (n == 0 && !d_off) {
       return RG_OK;
     }
@@ -816,23 +733,19 @@ namespace rg {
       }
       RG_CUDA_TRY(cudaEventRecord(ev.first, s));
     }
-    for (m.window = 0; m.window < std::max<int64_t>(n, 1); m.window += kMomWindow) {
-      for (int c = 0; c < kComps; ++c) {
-        m.fp.comp[c] = comp[c] ? comp[c] + m.window : stand_in(pl, c);
-      }
-      const int64_t steps = (std::min(n - m.window, kMomWindow) + kMomChunk - 1) / kMomChunk;
-      const int     grid  = static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(steps, ctx->sms * kMomBlocksPerSM)));
-      const dim3    blocks(grid, pl->nslices);
+    for (int64_t w = 0; w < std::max<int64_t>(n, 1); w += kPairWindow) {
+      fill_streams(pl, comp, d_off, n, nseg, w, m.in);
+      const dim3 blocks(pair_grid(n, w, ctx->sms, kMomBlocksPerSM), pl->nslices);
       if (m.fp.has_e) {
         if (d_off) {
-          moments_deposit_kernel<true, true><<<blocks, kMomThreads, 0, s>>>(m);
+          moments_deposit_kernel<true, true><<<blocks, kPairThreads, 0, s>>>(m);
         } else {
-          moments_deposit_kernel<true, false><<<blocks, kMomThreads, 0, s>>>(m);
+          moments_deposit_kernel<true, false><<<blocks, kPairThreads, 0, s>>>(m);
         }
       } else if (d_off) {
-        moments_deposit_kernel<false, true><<<blocks, kMomThreads, 0, s>>>(m);
+        moments_deposit_kernel<false, true><<<blocks, kPairThreads, 0, s>>>(m);
       } else {
-        moments_deposit_kernel<false, false><<<blocks, kMomThreads, 0, s>>>(m);
+        moments_deposit_kernel<false, false><<<blocks, kPairThreads, 0, s>>>(m);
       }
     }
     RG_CUDA_TRY(cudaGetLastError());
@@ -913,11 +826,9 @@ namespace rg {
     cudaFree(pl->d_msum);
     cudaFree(pl->d_logt);
     cudaFree(pl->d_cells);
-    cudaFree(pl->d_coef64);
     cudaFree(pl->own_smooth.d_coef);
     pl->d_cells           = nullptr;
     pl->cells_cap         = 0;
-    pl->d_coef64          = nullptr;
     pl->own_smooth.d_coef = nullptr;
     pl->d_mslice = nullptr;
     pl->d_mrange = nullptr;

@@ -79,17 +79,6 @@ namespace rg {
     return __longlong_as_double(static_cast<long long>(d));
   }
 
-  // FP64 atomic add of a float: values of normal magnitude take the integer-built
-  // operand, subnormals the FP64 pipe, zeros nothing.
-  __device__ __forceinline__ void red_add_float(double* dst, float v) {
-    const float m = fabsf(v);
-    if (m >= 1.17549435e-38f) {
-      atomicAdd(dst, float_to_double_bits(v));
-    } else if (m > 0.0f) {
-      atomicAdd(dst, static_cast<double>(v));
-    }
-  }
-
   // G = 1 + u^2 and W = |u x B|^2 (no E field) as double-floats (relative error ~2^-46; a
   // host emulation over 2e6 random and nearly parallel u, B: 1e-14 and 2e-13), in
   // fewer operations than kinematics_ff: squares and products are exact pairs, sums of
@@ -176,20 +165,6 @@ namespace rg {
       A *= v[9];
     }
     return isfinite(A);
-  }
-
-  // Largest s in [0, nseg] with off[s] <= i (off non-decreasing).
-  __device__ __forceinline__ int segment_of(const int64_t* off, int nseg, int64_t i) {
-    int lo = 0, hi = nseg;
-    while (lo < hi) {
-      const int mid = (lo + hi + 1) >> 1;
-      if (off[mid] <= i) {
-        lo = mid;
-      } else {
-        hi = mid - 1;
-      }
-    }
-    return lo;
   }
 
 } // namespace rg

@@ -20,6 +20,8 @@
 #include "moments_common.cuh"
 #include "spectrum_plan.hpp"
 
+#include <algorithm>
+
 namespace rg {
 
   // ---- asynchronous copies global -> shared ------------------------------------------------
@@ -247,7 +249,7 @@ namespace rg {
   };
 
   // The scalar stage, for the particles the packed one leaves out (a call, not inlined: rare).
-  __device__ __noinline__ int64_t scalar_place(const float (&v)[kComps], const FusedParams& p, int fx, int64_t Pmin,
+  static __device__ __noinline__ int64_t scalar_place(const float (&v)[kComps], const FusedParams& p, int fx, int64_t Pmin,
                                                int64_t Pmax, int64_t L, float& A) {
     int64_t Q = 0;
     if (!moment_particle_stage(v, p, Pmin, Pmax, L, Q, A)) {
@@ -329,6 +331,7 @@ namespace rg {
           continue;
         }
         if (wh[j] == 0.0f && wl[j] == 0.0f) { // no emission: u parallel to B, or no field
+          o.Y[j] = -1;
           o.A[j] = 0.0f;
           continue;
         }
@@ -345,6 +348,126 @@ namespace rg {
       }
     }
     return o;
+  }
+
+  // ---- particle streams, two particles per thread ------------------------------------------
+  // What a kernel over pairs reads: the streams from the first particle of the launch's window of
+  // at most kPairWindow particles (32-bit indices within it), and the segments.
+  constexpr int     kPairThreads = 256;
+  constexpr int     kPairChunk   = 2 * kPairThreads;   // particles per block and step
+  constexpr int64_t kPairWindow  = int64_t(1) << 31;
+  constexpr int     kPairSharedSeg = 1024;             // segment offsets staged in shared memory
+
+  struct PairStreams {
+    const float*   comp[kComps];   // a stand-in where a stream is not given
+    uint32_t       stride[kComps]; // bytes between particles: 4, or 0 for a stand-in
+    const int64_t* seg_off;        // nseg + 1 particle offsets (device), or null: particles [0, n)
+    int            nseg;
+    int64_t        n;              // stream length
+    int64_t        window;         // the window's first particle
+  };
+
+  inline void fill_streams(const rg_spectrum_plan* pl, const float* const comp[kComps], const int64_t* d_off, int64_t n,
+                           int nseg, int64_t window, PairStreams& p) {
+    for (int c = 0; c < kComps; ++c) {
+      p.comp[c]   = comp[c] ? comp[c] + window : stand_in(pl, c);
+      p.stride[c] = comp[c] ? 4u : 0u;
+    }
+    p.seg_off = d_off;
+    p.nseg    = d_off ? nseg : 1;
+    p.n       = n;
+    p.window  = window;
+  }
+
+  // Blocks over the window's particles, at most per_sm per SM.
+  inline int pair_grid(int64_t n, int64_t window, int sms, int per_sm) {
+    const int64_t steps = (std::min(n - window, kPairWindow) + kPairChunk - 1) / kPairChunk;
+    return static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(steps, static_cast<int64_t>(sms) * per_sm)));
+  }
+
+  // Stages the segments' offsets, clamped to the window and relative to its start; false for the
+  // whole block if they decrease or leave [0, n], or if the status word is set.
+  template <bool kSeg>
+  __device__ __forceinline__ bool stage_segments(const PairStreams& p, unsigned* status, uint32_t* soff) {
+    const int64_t w0 = p.window, w1 = min(p.n, w0 + kPairWindow);
+    bool          bad = false;
+    if (kSeg) {
+      for (int i = threadIdx.x; i <= p.nseg; i += kPairThreads) {
+        const int64_t o = p.seg_off[i];
+        bad             = bad || o < 0 || o > p.n || (i > 0 && o < p.seg_off[i - 1]);
+        soff[i]         = static_cast<uint32_t>(max(min(o, w1), w0) - w0);
+      }
+    }
+    if (__syncthreads_or(bad)) {
+      if (threadIdx.x == 0 && blockIdx.x == 0 && blockIdx.y == 0) {
+        atomicOr(status, kDevBadOffsets);
+      }
+      return false;
+    }
+    return !__syncthreads_or(*status != kDevOk);
+  }
+
+  // Particles base + thread and base + thread + 256 (coalesced whatever the streams' alignment).
+  // Past the end the last particle again, to be dropped by its index; nothing from a base past it.
+  template <bool kE>
+  __device__ __forceinline__ void load_pair(const PairStreams& p, uint32_t base, uint32_t last, float2 (&to)[kComps]) {
+    if (base + kPairChunk <= last) {
+#pragma unroll
+      for (int c = 0; c < kComps; ++c) {
+        if (kE || c < 3 || c >= 6) {
+          const float* q = reinterpret_cast<const float*>(reinterpret_cast<const char*>(p.comp[c]) +
+                                                          static_cast<uint64_t>(base + threadIdx.x) * p.stride[c]);
+          to[c].x        = __ldg(q);
+          to[c].y        = __ldg(q + kPairThreads);
+        }
+      }
+    } else if (base < last) {
+      const uint32_t i0 = min(base + threadIdx.x, last - 1), i1 = min(base + threadIdx.x + kPairThreads, last - 1);
+#pragma unroll
+      for (int c = 0; c < kComps; ++c) {
+        if (kE || c < 3 || c >= 6) {
+          const char* q = reinterpret_cast<const char*>(p.comp[c]);
+          to[c].x       = __ldg(reinterpret_cast<const float*>(q + static_cast<uint64_t>(i0) * p.stride[c]));
+          to[c].y       = __ldg(reinterpret_cast<const float*>(q + static_cast<uint64_t>(i1) * p.stride[c]));
+        }
+      }
+    }
+  }
+
+  template <bool kE>
+  __device__ __forceinline__ void to_pairs(const float2 (&from)[kComps], f2 (&v)[kComps]) {
+#pragma unroll
+    for (int c = 0; c < kComps; ++c) {
+      v[c] = (kE || c < 3 || c >= 6) ? pack2(from[c].x, from[c].y) : set2(0.0f);
+    }
+  }
+
+  // FP64 add to global memory where `on`, without a branch.
+  __device__ __forceinline__ void red_add_if(bool on, double* p, double v) {
+    asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %2, 0;\n\t@q red.global.add.f64 [%0], %1;\n\t}" ::"l"(p), "d"(v),
+                 "r"(static_cast<uint32_t>(on))
+                 : "memory");
+  }
+
+  constexpr uint32_t kNoEntry = 0xffffffffu;
+
+  // d 2^-k as (hi, lo): the top 24 significant bits cut, then the 29 below; 0 when d 2^-k < 2^-126
+  // (GB300's FP64 pipe would take longer over the subtraction d - hi than these integer steps).
+  __device__ __forceinline__ float2 split_double(double d, int k) {
+    const uint32_t h = static_cast<uint32_t>(__double2hiint(d)), l = static_cast<uint32_t>(__double2loint(d));
+    const int      e = static_cast<int>((h >> 20) & 0x7ffu) - 1023 + 127 - k; // biased FP32 exponent
+    const uint32_t sign = h & 0x80000000u;
+    float2         r;
+    r.x = __uint_as_float(sign | (static_cast<uint32_t>(e) << 23) | (__funnelshift_l(l, h, 3) & 0x7fffffu));
+    r.y = static_cast<float>(l & 0x1fffffffu) * __uint_as_float(sign | (static_cast<uint32_t>(e - 52) << 23));
+    r.y = e > 52 ? r.y : 0.0f;
+    return e >= 1 ? r : make_float2(0.0f, 0.0f);
+  }
+
+  __device__ __forceinline__ ff2 ff_mul2(ff2 a, ff2 b) {
+    const f2 p = mul2(a.hi, b.hi);
+    const f2 e = sub2(fma2(a.hi, b.lo, mul2(a.lo, b.hi)), fma2(neg2(a.hi), b.hi, p));
+    return fast_two_sum2(p, e);
   }
 
 } // namespace rg

@@ -67,10 +67,8 @@ struct rg_spectrum_plan {
   bool                  aligned     = false;
   int64_t               sm_pmin = 0, sm_pmax = 0; // smallest / largest bin coordinate, fine units
   int                   sm_cells    = 0;
-  double*               d_cells     = nullptr; // nseg x cells x 4 doubles: the forward's folded cell
-                                               // moments, or (as float4) the adjoint's cell cubics
+  float4*               d_cells     = nullptr; // nseg x cells: the adjoint's cell cubics
   size_t                cells_cap   = 0;       // (segment, cell) entries
-  double2*              d_coef64    = nullptr; // per table segment: (c0, c1), (c2, c3), (c1, 2 c2), (3 c3, 0)
   // kernel timing (events bracketing each fused launch)
   bool                                             timing = false;
   std::vector<std::pair<cudaEvent_t, cudaEvent_t>> ev_used, ev_free;

@@ -304,3 +304,48 @@ def test_smooth_host_streaming_matches_device(gpu, oracle_lib, algo):
     plan.check()
     truth = oracle_lib.sync_smooth_f64(sub, bins, 1.0, 1.0, 1.0, coef, xmin, xmax)
     assert max_rel(dev.cpu().numpy(), truth) <= SPECTRUM_RTOL
+
+
+@pytest.mark.parametrize("n,nbins,efield", [(1, 2, False), (255, 33, False), (257, 64, True), (511, 512, False),
+                                            (513, 100, False), (1025, 700, True)])
+def test_moment_pair_edges(gpu, oracle_lib, n, nbins, efield):
+    """Particle counts around the kernels' 512-particle steps, streams that start off a 16-byte
+    boundary, zero weights (no emission, but a gradient) and momenta small enough for the
+    scalar gradient: spectrum and full gradient against FP64, with the placement record and
+    without."""
+    P = particles(n + 1, seed=3 * n + nbins, bfield="iso", weights=True, efield=efield, umax=1e3)
+    P = {k: v[1:].copy() for k, v in P.items()}
+    P["w"][::7] = 0.0
+    if n > 4 and not efield:
+        for k in ("ux", "uy", "uz"):
+            P[k][3] *= np.float32(1e-11)
+    bins = oracle_lib.logspace(1e-2, 1e6, nbins)
+    plan = rt.spectrum_plan(bins)
+    coef, xmin, xmax = plan_table(plan)
+    T = {}
+    for k, v in P.items():
+        full = torch.zeros(n + 1, device=gpu)
+        full[1:] = torch.from_numpy(v).to(gpu)
+        T[k] = full[1:]
+    prt = capi.particles([T["ux"], T["uy"], T["uz"]], b=[T["bx"], T["by"], T["bz"]],
+                         e=[T["ex"], T["ey"], T["ez"]] if efield else None, w=T["w"], n=n)
+    S64 = oracle_lib.sync_smooth_f64(P, bins, 1.0, 1.0, 1.0, coef, xmin, xmax)
+    gS = 1.0 / np.maximum(S64, 1e-6 * max(S64.max(), 1e-30))
+    gw64, gu64 = oracle_lib.sync_smooth_grad_f64(P, bins, 1.0, 1.0, 1.0, coef, gS, xmin, xmax)
+    g64 = np.vstack([gw64[None], gu64])
+    scale = np.maximum(np.max(np.abs(g64), axis=1, keepdims=True), 1e-30)
+    S = torch.full((nbins,), -1.0, device=gpu)
+    gout = torch.from_numpy(gS.astype(np.float32)).to(gpu)
+    place = torch.empty(2 * n, device=gpu, dtype=torch.int32)
+    for placed in (True, False):
+        g = [torch.full((n,), float("nan"), device=gpu) for _ in range(4)]
+        if placed:
+            plan.run_placed(prt, S, place)
+            plan.adjoint_placed(prt, place, gout, g[0], g[1:])
+        else:
+            plan.run(prt, S)
+            plan.adjoint(prt, gout, g[0], g[1:])
+        plan.check()
+        assert max_rel(S.cpu().numpy(), S64) <= SPECTRUM_RTOL
+        got = np.stack([t.cpu().numpy() for t in g]).astype(np.float64)
+        assert np.max(np.abs(got - g64) / scale) < 1e-4
