@@ -12,7 +12,7 @@
 // reciprocal may be the hardware's approximate one.  The remainder's error is below 2^-41
 // (r^4/4), a hundredth of the coordinate's unit.
 //
-// Every operation is the IEEE operation written (no contraction), and a particle whose
+// Every operation whose rounding error is taken is the IEEE operation written, and a particle whose
 // X is not a normal float (u parallel to B, no field, overflow, NaN) takes the scalar
 // stage instead.
 #pragma once
@@ -64,6 +64,9 @@ namespace rg {
     return r;
   }
 
+  // The compiler contracts a packed product that only one packed sum reads into an fma, .rn or not
+  // (measured: 489284 of 1048576 sums of three squares differ from the separately rounded ones).  A
+  // product whose rounding matters below is read again for its remainder, which keeps it a product.
   __device__ __forceinline__ f2 mul2(f2 a, f2 b) {
     f2 r;
     asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));

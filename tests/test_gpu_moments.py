@@ -180,3 +180,38 @@ def test_moments_edges_of_steps_and_rows(gpu, oracle_lib, table, n, nbins, wscal
     plan.check()
     truth = oracle_lib.sync_spectrum_f64(P, bins, 1.0, 1.0, 1.0, table)
     assert max_rel(out.cpu().numpy(), truth) <= SPECTRUM_RTOL
+
+
+@pytest.mark.parametrize("mode", ["reference", "smooth"])
+@pytest.mark.parametrize("efield", [False, True])
+@pytest.mark.parametrize("tilt", [2.0**-8, 2.0**-20])
+def test_moments_nearly_cancelling_force(gpu, oracle_lib, table, mode, efield, tilt):
+    """Fields almost parallel to the momentum, or an electric field that almost cancels u x B: the
+    force is the small difference of products, whose remainders decide it (a sum that took an
+    unrounded product instead would be off by the product's whole rounding error)."""
+    n   = 4001
+    P   = particles(n, seed=5, bfield="iso", weights=True, umax=1e3)
+    rng = np.random.default_rng(6)
+    u   = np.stack([P[k] for k in ("ux", "uy", "uz")]).astype(np.float64)
+    b   = np.stack([P[k] for k in ("bx", "by", "bz")]).astype(np.float64)
+    off = 1.0 + tilt * rng.uniform(-1.0, 1.0, (3, n))
+    if efield:
+        e = -np.cross(u.T, b.T).T / np.sqrt(1.0 + np.sum(u * u, axis=0)) * off
+        P.update({k: e[d].astype(np.float32) for d, k in enumerate(("ex", "ey", "ez"))})
+    else:
+        b = u / np.sqrt(np.sum(u * u, axis=0)) * off
+        P.update({k: b[d].astype(np.float32) for d, k in enumerate(("bx", "by", "bz"))})
+    bins = oracle_lib.logspace(1e-8, 1e6, 300)
+    T, prt = _device(P, gpu)
+    out = torch.full((300,), -1.0, device=gpu)
+    plan = capi.SpectrumPlan(bins, 1.0, 1.0, 1.0,
+                             capi.RG_TABLE_SMOOTH if mode == "smooth" else capi.RG_TABLE_REFERENCE)
+    plan.run(prt, out)
+    plan.check()
+    if mode == "reference":
+        truth = oracle_lib.sync_spectrum_f64(P, bins, 1.0, 1.0, 1.0, table)
+    else:
+        coef, lnx, dln = plan.smooth_table()
+        xmin, xmax = float(np.exp(lnx)), float(np.exp(lnx + coef.shape[0] * dln))
+        truth = oracle_lib.sync_smooth_f64(P, bins, 1.0, 1.0, 1.0, coef, xmin, xmax)
+    assert max_rel(out.cpu().numpy(), truth) <= SPECTRUM_RTOL
