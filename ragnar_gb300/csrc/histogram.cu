@@ -14,9 +14,17 @@
 // Log-spaced bins add float(1.0 / energy): for |u| energies that is the
 // correctly rounded reciprocal of sqrtf(Usqr) (double rounding of one division
 // of floats through double is innocuous); for sqrt(1 + Usqr) energies it is a
-// double-float Newton step of rsqrt rounded to float.  Sums are accumulated in
-// FP32 shared-memory bins (kSumCopies lane-indexed copies) flushed to FP64 every
-// chunk, then across blocks in FP64 in a fixed order.
+// double-float Newton step of rsqrt rounded to float.
+//
+// Only what the call asks for is accumulated: sums for log-spaced bins, counts otherwise or where
+// they are asked for.  Sums of many particles over up to about 220 bins without counts
+// (lane_warps): every lane of a warp has its own copy of the bins in shared memory, [bin][lane],
+// so a particle is one conflict-free load, add and store.  Shared-memory atomics set the pace
+// of the other kernel, which serves the rest: integer ones run at one lane per clock and SM on
+// random bins, float ones as compare-and-swap loops.  FP32 sums are flushed to FP64 every
+// kFlushLane particles of a lane (or kFlushParticles of a block), then summed across blocks in
+// FP64 in a fixed order.
+#include "pair_stage.cuh"
 #include "rg_common.cuh"
 #include "rg_internal.hpp"
 
@@ -25,6 +33,7 @@
 #include <cstring>
 #include <limits>
 #include <mutex>
+#include <type_traits>
 #include <vector>
 
 namespace rg {
@@ -66,6 +75,14 @@ namespace rg {
       return f;
     }
 
+    // The lane kernel's cells are coarser (its table has 8 bytes a cell) and carry their first
+    // threshold, so a cell with at most one threshold is one load.
+    constexpr int kLaneCells   = 2048;
+    constexpr int kLaneMaxWarps = 16;
+    constexpr int kLaneVectors = 4;    // groups of four particles in flight per thread (8: the same time)
+    constexpr int kFlushLane   = 1024; // particles per lane between flushes
+    constexpr size_t kLaneSmem = 226 * 1024;
+
     struct HistParams {
       const float*    ux;
       const float*    uy;
@@ -80,8 +97,12 @@ namespace rg {
       int             cell_shift;   // cell of a float = its bit pattern >> cell_shift
       int             cell_base;    // cell of thr[1]
       int             ncells;
-      unsigned long long* part_counts; // [grid][nbins]
-      double*         part_sums;       // [grid][nbins]
+      const uint2*    lcells;       // lane kernel: [lncells + 2]: below thr[1], the cells, above the last threshold:
+                                    // (128 x the bin of the cell's smallest float, next threshold's bits; bit 31 of
+                                    // the first: more than one threshold inside)
+      int             lshift, lbase, lncells;
+      unsigned long long* part_counts; // [grid][nbins], or null
+      double*         part_sums;       // [grid][nbins], or null
     };
 
     // Bin of one particle: start[ci] is the bin of the smallest float of its cell (entry
@@ -117,6 +138,20 @@ namespace rg {
       return __fmaf_rn(__fmul_rn(0.5f, r0), e, r0);
     }
 
+    // 1/|u|: rsqrt and one Newton step (within an ulp; the reference rounds this value through
+    // double, so the sums are compared with a tolerance anyway)
+    __device__ __forceinline__ float inverse_energy(float U, int fourvel) {
+      if (!fourvel) {
+        return inv_sqrt_one_plus(U);
+      }
+      if (U > 0.0f && U < 3.0e38f) {
+        const float r = rsqrtf(U);
+        return __fmul_rn(r, __fmaf_rn(__fmul_rn(-0.5f * U, r), r, 1.5f));
+      }
+      return __frcp_rn(sqrtf(U)); // 0 -> inf, inf -> 0, NaN -> NaN
+    }
+
+    template <bool kSum, bool kCount>
     __global__ void __launch_bounds__(kHistThreads)
       histogram_kernel(const __grid_constant__ HistParams p) {
       extern __shared__ __align__(16) unsigned char smem[];
@@ -154,19 +189,11 @@ namespace rg {
         auto          one = [&](float x, float y, float z) {
           const float U = __fadd_rn(__fadd_rn(__fmul_rn(x, x), __fmul_rn(y, y)), __fmul_rn(z, z));
           const int   k = bin_of(U, p, thr, start);
-          atomicAdd(&cnt[k], 1u);
-          if (p.log_spaced) {
-            // 1/|u|: rsqrt and one Newton step (within an ulp; the reference rounds this
-            // value through double, so the sums are compared with a tolerance anyway)
-            float v;
-            if (!p.fourvel) {
-              v = inv_sqrt_one_plus(U);
-            } else if (U > 0.0f && U < 3.0e38f) {
-              const float r = rsqrtf(U);
-              v             = __fmul_rn(r, __fmaf_rn(__fmul_rn(-0.5f * U, r), r, 1.5f));
-            } else {
-              v = __frcp_rn(sqrtf(U)); // 0 -> inf, inf -> 0, NaN -> NaN
-            }
+          if (kCount) {
+            atomicAdd(&cnt[k], 1u);
+          }
+          if (kSum) {
+            const float v = inverse_energy(U, p.fourvel);
             atomicAdd(&sum_l[k], v);
           }
         };
@@ -191,7 +218,7 @@ namespace rg {
             one(p.ux[i], p.uy[i], p.uz[i]);
           }
         }
-        if (p.log_spaced) {
+        if (kSum) {
           __syncthreads();
           for (int i = threadIdx.x; i < nb; i += blockDim.x) {
             double t = sum64[i];
@@ -205,8 +232,272 @@ namespace rg {
         __syncthreads();
       }
       for (int i = threadIdx.x; i < nb; i += blockDim.x) {
-        p.part_counts[static_cast<int64_t>(blockIdx.x) * nb + i] = cnt[i];
-        p.part_sums[static_cast<int64_t>(blockIdx.x) * nb + i]   = sum64[i];
+        if (kCount) {
+          p.part_counts[static_cast<int64_t>(blockIdx.x) * nb + i] = cnt[i];
+        }
+        if (kSum) {
+          p.part_sums[static_cast<int64_t>(blockIdx.x) * nb + i] = sum64[i];
+        }
+      }
+    }
+
+    // Energies whose reciprocal the packed expressions below give: 2^-126 <= Usqr < 2^100, as an
+    // interval of bit patterns (which leaves out NaN too).
+    constexpr uint32_t kOrdinaryMin  = 0x00800000u;
+    constexpr uint32_t kOrdinarySpan = 0x71800000u - kOrdinaryMin;
+
+    __device__ __forceinline__ f2 rsqrt2(float a, float b) {
+      asm("rsqrt.approx.ftz.f32 %0, %0;" : "+f"(a));
+      asm("rsqrt.approx.ftz.f32 %0, %0;" : "+f"(b));
+      return pack2(a, b);
+    }
+
+    // inv_sqrt_one_plus of two: r + r (1 - s r^2) / 2 with s = 1 + U in double-float.  r^2 = h + l and
+    // s.hi h - 1 are exact or rounded once, so the correction keeps its leading digits.
+    __device__ __forceinline__ f2 inv_sqrt_one_plus2(f2 U) {
+      const ff2 s = two_sum2(set2(1.0f), U);
+      float     a, b;
+      unpack2(s.hi, a, b);
+      const f2 r = rsqrt2(a, b);
+      const f2 h = mul2(r, r), l = fma2(r, r, neg2(h));
+      const f2 e = add2(fma2(s.hi, h, set2(-1.0f)), fma2(s.hi, l, mul2(s.lo, h))); // s r^2 - 1
+      return fma2(mul2(r, set2(-0.5f)), e, r);
+    }
+
+    // Any particle's bin by stepping over all thresholds (energies of 0, infinity and NaN, and
+    // cells with several thresholds).
+    __device__ __noinline__ int bin_by_steps(float U, const HistParams& p, const float* thr, int g) {
+      if (U != U) {
+        return p.nan_index;
+      }
+      while (g < p.nbins - 1 && thr[g + 1] <= U) {
+        ++g;
+      }
+      return g;
+    }
+
+    // Shared memory of the lane kernel with `warps` warps.
+    size_t lane_smem(int nb, int ncells, int warps) {
+      return (sizeof(double) + sizeof(float)) * nb + sizeof(uint2) * (ncells + 2) +
+             sizeof(float) * 32 * static_cast<size_t>(nb) * warps + 16;
+    }
+
+    // Warps of the lane kernel, or 0 where the atomics are faster: with fewer than seven warps on
+    // an SM the loads' latency is not hidden, and clearing and summing the copies takes about as
+    // long as a few million particles.  Per call, sums of |u|^-1 over log bins, lanes against
+    // atomics: 3.3e7 particles x 50 bins 99 / 164 us, 150: 104 / 140, 200: 121 / 139, 220 (7 warps):
+    // 128 / 141, 250 (6 warps): 162 / 138, 380 (4): 209 / 144; 200 bins x 8e6: 54.5 / 58.3, 4e6: 43.2 / 43.3,
+    // 1e6: 35.7 / 28.8.  Counts stay with the integer atomics (200 bins: 109 / 81).
+    constexpr int     kLaneMinWarps     = 7;
+    constexpr int64_t kLaneMinParticles = 6000000;
+
+    int lane_warps(int64_t n, int nb, int ncells) {
+      const size_t tables = lane_smem(nb, ncells, 0);
+      if (n < kLaneMinParticles || tables >= kLaneSmem) {
+        return 0;
+      }
+      const size_t w = (kLaneSmem - tables) / (sizeof(float) * 32 * nb);
+      return w < static_cast<size_t>(kLaneMinWarps) ? 0 : static_cast<int>(std::min<size_t>(w, kLaneMaxWarps));
+    }
+
+    // What bounds it: latency.  200 bins leave room for 8 warps on an SM (copies: 25.6 KB each), 33
+    // instructions a particle at 27 % of the issue slots, 49 % of the DRAM rate: 103 us for
+    // 3.3e7 particles x 200 bins against 120 us with atomics.  Eight particles of a thread are in
+    // flight at once (four, one addition after the other: 119 us).
+    __global__ void __launch_bounds__(32 * kLaneMaxWarps) histogram_lane_kernel(const __grid_constant__ HistParams p) {
+      extern __shared__ __align__(16) unsigned char smem[];
+      const int nb = p.nbins, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+      double*   sum64 = reinterpret_cast<double*>(smem);
+      uint2*    cells = reinterpret_cast<uint2*>(sum64 + nb);
+      float*    thr   = reinterpret_cast<float*>(cells + p.lncells + 2);
+      float*    copies = reinterpret_cast<float*>((reinterpret_cast<uintptr_t>(thr + nb) + 15) & ~uintptr_t(15));
+      const int per    = 32 * nb;
+      float*    mine   = copies + warp * per; // [nb][32]
+      for (int i = threadIdx.x; i < nb; i += blockDim.x) {
+        thr[i]   = p.thr[i];
+        sum64[i] = 0.0;
+      }
+      for (int i = threadIdx.x; i < p.lncells + 2; i += blockDim.x) {
+        cells[i] = p.lcells[i];
+      }
+      for (int i = threadIdx.x; i < warps * per / 4; i += blockDim.x) {
+        reinterpret_cast<uint4*>(copies)[i] = make_uint4(0u, 0u, 0u, 0u);
+      }
+      __syncthreads();
+
+      // 2 N particles of a lane: the bins and values of all of them first, then the additions in
+      // pairs (the two of a pair may share a bin).
+      const uint32_t copy0 = static_cast<uint32_t>(__cvta_generic_to_shared(mine + lane));
+      const uint32_t cell0 = static_cast<uint32_t>(__cvta_generic_to_shared(cells)) - 8u * static_cast<uint32_t>(p.lbase - 1);
+      const int      cmin = p.lbase - 1, cmax = p.lbase + p.lncells;
+      const bool     fourvel = p.fourvel != 0;
+      auto           add     = [&](auto const& x, auto const& y, auto const& z, auto count_tag) {
+        constexpr int N = decltype(count_tag)::value;
+        float         u[2 * N], v[2 * N];
+        uint32_t      k[2 * N];
+        uint32_t      many = 0u, far = 0u;
+#pragma unroll
+        for (int j = 0; j < N; ++j) {
+          // single products: the compiler contracts a packed product and sum, whatever their rounding
+          // modifiers, and Usqr has to be the reference's
+          float x0, x1, y0, y1, z0, z1;
+          unpack2(x[j], x0, x1);
+          unpack2(y[j], y0, y1);
+          unpack2(z[j], z0, z1);
+          u[2 * j]     = __fadd_rn(__fadd_rn(__fmul_rn(x0, x0), __fmul_rn(y0, y0)), __fmul_rn(z0, z0));
+          u[2 * j + 1] = __fadd_rn(__fadd_rn(__fmul_rn(x1, x1), __fmul_rn(y1, y1)), __fmul_rn(z1, z1));
+          const f2 U   = pack2(u[2 * j], u[2 * j + 1]);
+#pragma unroll
+          for (int h = 2 * j; h < 2 * j + 2; ++h) {
+            const uint32_t bits = __float_as_uint(u[h]);
+            uint32_t       cx, cy;
+            asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(cx), "=r"(cy) : "r"(cell0 + 8u * static_cast<uint32_t>(max(cmin, min(static_cast<int>(bits >> p.lshift), cmax)))));
+            k[h] = cx + (u[h] >= __uint_as_float(cy) ? 128u : 0u);
+            many |= cx;
+            far = max(far, bits - kOrdinaryMin);
+          }
+          if (fourvel) { // inverse_energy of an ordinary U
+            const f2 r = rsqrt2(u[2 * j], u[2 * j + 1]);
+            unpack2(mul2(r, fma2(mul2(mul2(U, set2(-0.5f)), r), r, set2(1.5f))), v[2 * j], v[2 * j + 1]);
+          } else {
+            unpack2(inv_sqrt_one_plus2(U), v[2 * j], v[2 * j + 1]);
+          }
+        }
+        if (static_cast<int>(many) < 0 || far >= kOrdinarySpan) {
+#pragma unroll
+          for (int h = 0; h < 2 * N; ++h) {
+            const uint32_t bits = __float_as_uint(u[h]);
+            const int      ci   = max(cmin, min(static_cast<int>(bits >> p.lshift), cmax)) - cmin;
+            k[h] = 128u * static_cast<uint32_t>(bin_by_steps(u[h], p, thr, static_cast<int>((cells[ci].x & 0x7fffffffu) >> 7)));
+            v[h] = inverse_energy(u[h], p.fourvel);
+          }
+        }
+#pragma unroll
+        for (int j = 0; j < N; ++j) {
+          const uint32_t k0 = k[2 * j], k1 = k[2 * j + 1];
+          float a, b;
+          asm volatile("ld.shared.f32 %0, [%1];" : "=f"(a) : "r"(copy0 + k0) : "memory");
+          asm volatile("ld.shared.f32 %0, [%1];" : "=f"(b) : "r"(copy0 + k1) : "memory");
+          a = __fadd_rn(a, v[2 * j]);
+          b = __fadd_rn(k0 == k1 ? a : b, v[2 * j + 1]);
+          asm volatile("st.shared.f32 [%0], %1;" ::"r"(copy0 + k0), "f"(a) : "memory");
+          asm volatile("st.shared.f32 [%0], %1;" ::"r"(copy0 + k1), "f"(b) : "memory");
+        }
+      };
+      auto add_one = [&](float x, float y, float z) {
+        const float U = __fadd_rn(__fadd_rn(__fmul_rn(x, x), __fmul_rn(y, y)), __fmul_rn(z, z));
+        const int   k = bin_by_steps(U, p, thr, static_cast<int>((cells[max(cmin, min(static_cast<int>(__float_as_uint(U) >> p.lshift), cmax)) - cmin].x & 0x7fffffffu) >> 7));
+        mine[k * 32 + lane] += inverse_energy(U, p.fourvel);
+      };
+      // The lanes' copies into the block's totals: a thread sums the 32 copies of its bins in four
+      // chains (starting at a different lane per bin, so that a warp's reads hit different banks),
+      // then the warps'.
+      auto flush = [&]() {
+        __syncwarp();
+        for (int b = lane; b < nb; b += 32) {
+          ff t[4];
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            t[c] = ff { 0.0f, 0.0f };
+          }
+#pragma unroll 2
+          for (int l = 0; l < 32; l += 4) {
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+              const int   at = b * 32 + ((l + c + b) & 31);
+              const float x  = mine[at];
+              const ff    s  = two_sum(t[c].hi, x);
+              // an infinite sum (an energy of 0) or NaN stays what it is: its remainder is NaN
+              t[c]     = ff { s.hi, isfinite(s.hi) ? __fadd_rn(t[c].lo, s.lo) : 0.0f };
+              mine[at] = 0.0f;
+            }
+          }
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            mine[b * 32 + 2 * c]     = t[c].hi;
+            mine[b * 32 + 2 * c + 1] = t[c].lo;
+          }
+        }
+        __syncthreads();
+        // four threads a bin sum the warps' pairs of one chain each
+        for (int i = threadIdx.x; i < ((4 * nb + 31) & ~31); i += blockDim.x) {
+          const int b = i >> 2, c = i & 3;
+          double    t = 0.0;
+          if (b < nb) {
+            for (int w = 0; w < warps; ++w) {
+              float* m = copies + w * per + b * 32 + 2 * c;
+              t += static_cast<double>(m[0]) + static_cast<double>(m[1]);
+              m[0] = 0.0f;
+              m[1] = 0.0f;
+            }
+          }
+          t += __shfl_xor_sync(0xffffffffu, t, 1);
+          t += __shfl_xor_sync(0xffffffffu, t, 2);
+          if (b < nb && c == 0) {
+            sum64[b] += t;
+          }
+        }
+        __syncthreads();
+      };
+
+      const int64_t T = static_cast<int64_t>(gridDim.x) * blockDim.x;
+      const int64_t t = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+      const bool    vec_ok = ((reinterpret_cast<uintptr_t>(p.ux) | reinterpret_cast<uintptr_t>(p.uy) |
+                            reinterpret_cast<uintptr_t>(p.uz)) & 15) == 0;
+      int           since = 0; // particles of a lane since the last flush (the same in every thread)
+      int64_t       done  = 0; // particles taken by the vector loop
+      if (vec_ok) {
+        const int64_t nv = p.n / 4;
+        done             = nv * 4;
+        // kLaneVectors groups in flight, taken two at a time: their registers are loaded again as
+        // soon as the two are added
+        float4 X[kLaneVectors], Y[kLaneVectors], Z[kLaneVectors];
+        auto   load = [&](int k, int64_t v) {
+          if (v < nv) {
+            X[k] = __ldcs(reinterpret_cast<const float4*>(p.ux) + v);
+            Y[k] = __ldcs(reinterpret_cast<const float4*>(p.uy) + v);
+            Z[k] = __ldcs(reinterpret_cast<const float4*>(p.uz) + v);
+          }
+        };
+#pragma unroll
+        for (int k = 0; k < kLaneVectors; ++k) {
+          load(k, k * T + t);
+        }
+        for (int64_t v0 = 0; v0 < nv; v0 += kLaneVectors * T) { // uniform over the grid
+#pragma unroll
+          for (int k = 0; k < kLaneVectors; k += 2) {
+            const int64_t v    = v0 + k * T + t;
+            const f2      x[4] = { pack2(X[k].x, X[k].y), pack2(X[k].z, X[k].w), pack2(X[k + 1].x, X[k + 1].y), pack2(X[k + 1].z, X[k + 1].w) };
+            const f2      y[4] = { pack2(Y[k].x, Y[k].y), pack2(Y[k].z, Y[k].w), pack2(Y[k + 1].x, Y[k + 1].y), pack2(Y[k + 1].z, Y[k + 1].w) };
+            const f2      z[4] = { pack2(Z[k].x, Z[k].y), pack2(Z[k].z, Z[k].w), pack2(Z[k + 1].x, Z[k + 1].y), pack2(Z[k + 1].z, Z[k + 1].w) };
+            if (v + T < nv) {
+              add(x, y, z, std::integral_constant<int, 4> {});
+            } else if (v < nv) {
+              add(x, y, z, std::integral_constant<int, 2> {});
+            }
+            load(k, v + kLaneVectors * T);
+            load(k + 1, v + (kLaneVectors + 1) * T);
+          }
+          since += 4 * kLaneVectors;
+          if (since >= kFlushLane) {
+            flush();
+            since = 0;
+          }
+        }
+      }
+      for (int64_t i0 = done; i0 < p.n; i0 += T) { // uniform over the grid
+        const int64_t i = i0 + t;
+        if (i < p.n) {
+          add_one(p.ux[i], p.uy[i], p.uz[i]);
+        }
+        if (++since >= kFlushLane) {
+          flush();
+          since = 0;
+        }
+      }
+      flush();
+      for (int b = threadIdx.x; b < nb; b += blockDim.x) {
+        p.part_sums[static_cast<int64_t>(blockIdx.x) * nb + b] = sum64[b];
       }
     }
 
@@ -228,8 +519,8 @@ namespace rg {
         // unrolled so that several rows' loads are in flight (the adds stay in row order)
 #pragma unroll 8
         for (int b = ty; b < grid; b += kHistReduceRows) {
-          c += pc[static_cast<int64_t>(b) * nbins + k];
-          s += ps[static_cast<int64_t>(b) * nbins + k];
+          c += pc ? pc[static_cast<int64_t>(b) * nbins + k] : 0ull;
+          s += ps ? ps[static_cast<int64_t>(b) * nbins + k] : 0.0;
         }
       }
       c_part[ty][threadIdx.x] = c;
@@ -297,7 +588,9 @@ namespace rg {
       float                               emin = 0, emax = 0;
       std::vector<uint16_t>               start; // cell table (see bin_of)
       int                                 cell_shift = 0, cell_base = 0, ncells = 0;
-      std::vector<std::pair<int, float*>> dev; // (device, thresholds then cell table on that device)
+      std::vector<uint2>                  lcells; // cell table of the lane kernel
+      int                                 lshift = 0, lbase = 0, lncells = 0;
+      std::vector<std::pair<int, float*>> dev; // (device, the lane kernel's cells, thresholds, cell table there)
     };
 
     uint32_t float_bits(float f) {
@@ -345,6 +638,41 @@ namespace rg {
       }
     }
 
+    // The lane kernel's cells over the same range (see HistParams::lcells).
+    void make_lane_cells(ThrEntry& e) {
+      const int      n   = static_cast<int>(e.thr.size());
+      const uint32_t inf = 0x7f800000u;
+      int            fin = 0; // thresholds thr[1..fin] are finite
+      while (fin + 1 < n && std::isfinite(e.thr[fin + 1])) {
+        ++fin;
+      }
+      e.lshift  = 0;
+      e.lbase   = 0;
+      e.lncells = 0;
+      if (fin == 0) { // no finite threshold: bin 0 for every finite energy
+        e.lcells.assign(2, make_uint2(0u, inf));
+        return;
+      }
+      const uint32_t lo = float_bits(e.thr[1]), hi = float_bits(e.thr[fin]);
+      while ((hi >> e.lshift) - (lo >> e.lshift) + 1 > static_cast<uint32_t>(kLaneCells)) {
+        ++e.lshift;
+      }
+      e.lbase   = static_cast<int>(lo >> e.lshift);
+      e.lncells = static_cast<int>((hi >> e.lshift) - (lo >> e.lshift) + 1);
+      e.lcells.assign(static_cast<std::size_t>(e.lncells) + 2, make_uint2(0u, inf));
+      int k = 1; // thr[1..k-1] <= the current cell's smallest float
+      for (int i = 1; i <= e.lncells; ++i) {
+        const uint32_t first = static_cast<uint32_t>(e.lbase + i - 1) << e.lshift;
+        while (k <= fin && float_bits(e.thr[k]) <= first) {
+          ++k;
+        }
+        const uint64_t next = static_cast<uint64_t>(first) + (uint64_t(1) << e.lshift);
+        const bool     many = k + 1 <= fin && float_bits(e.thr[k + 1]) < next;
+        e.lcells[i] = make_uint2(128u * static_cast<uint32_t>(k - 1) | (many ? 0x80000000u : 0u), k <= fin ? float_bits(e.thr[k]) : inf);
+      }
+      e.lcells[e.lncells + 1] = make_uint2(128u * static_cast<uint32_t>(fin), inf);
+    }
+
     constexpr std::size_t kThrCacheEntries = 16;
 
     std::mutex& thr_mutex() {
@@ -377,6 +705,8 @@ namespace rg {
   struct DeviceBins {
     const float*    thr   = nullptr;
     const uint16_t* start = nullptr;
+    const uint2*    lcells = nullptr;
+    int             lshift = 0, lbase = 0, lncells = 0;
     int             nan_index = 0, cell_shift = 0, cell_base = 0, ncells = 0;
   };
 
@@ -397,6 +727,7 @@ namespace rg {
       ThrEntry e;
       energy_thresholds(bins, n, fourvel, e.thr, e.nan_index, e.emin, e.emax);
       make_cells(e);
+      make_lane_cells(e);
       e.bins.assign(bins, bins + n);
       e.fourvel = fourvel;
       if (cache.size() >= kThrCacheEntries) {
@@ -417,10 +748,15 @@ namespace rg {
       }
     }
     if (!p) {
-      RG_CUDA_TRY(cudaMalloc(&p, sizeof(float) * n + sizeof(uint16_t) * e.start.size()));
-      cudaError_t err = cudaMemcpy(p, e.thr.data(), sizeof(float) * n, cudaMemcpyHostToDevice);
+      const size_t lbytes = sizeof(uint2) * e.lcells.size();
+      RG_CUDA_TRY(cudaMalloc(&p, lbytes + sizeof(float) * n + sizeof(uint16_t) * e.start.size()));
+      float*      t   = reinterpret_cast<float*>(reinterpret_cast<unsigned char*>(p) + lbytes);
+      cudaError_t err = cudaMemcpy(p, e.lcells.data(), lbytes, cudaMemcpyHostToDevice);
       if (err == cudaSuccess) {
-        err = cudaMemcpy(p + n, e.start.data(), sizeof(uint16_t) * e.start.size(), cudaMemcpyHostToDevice);
+        err = cudaMemcpy(t, e.thr.data(), sizeof(float) * n, cudaMemcpyHostToDevice);
+      }
+      if (err == cudaSuccess) {
+        err = cudaMemcpy(t + n, e.start.data(), sizeof(uint16_t) * e.start.size(), cudaMemcpyHostToDevice);
       }
       if (err != cudaSuccess) {
         cudaFree(p);
@@ -428,8 +764,12 @@ namespace rg {
       }
       e.dev.emplace_back(device, p);
     }
-    out.thr        = p;
-    out.start      = reinterpret_cast<const uint16_t*>(p + n);
+    out.lcells     = reinterpret_cast<const uint2*>(p);
+    out.thr        = reinterpret_cast<const float*>(out.lcells + e.lcells.size());
+    out.start      = reinterpret_cast<const uint16_t*>(out.thr + n);
+    out.lshift     = e.lshift;
+    out.lbase      = e.lbase;
+    out.lncells    = e.lncells;
     out.nan_index  = e.nan_index;
     out.cell_shift = e.cell_shift;
     out.cell_base  = e.cell_base;
@@ -482,22 +822,36 @@ int rg_energy_distribution(const float* ux, const float* uy, const float* uz, in
 
   rg::DeviceContext* ctx = nullptr;
   RG_TRY(rg::context(&ctx));
-  const size_t smem = (((2 + rg::kSumCopies) * sizeof(float) * nbins + 15) & ~size_t(15)) +
-                      sizeof(double) * nbins + sizeof(uint16_t) * (db.ncells + 1);
-  if (smem > 48 * 1024) {
-    RG_CUDA_TRY(cudaFuncSetAttribute(rg::histogram_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     static_cast<int>(smem)));
+  // what is accumulated, and by which kernel
+  const bool need_sum = log_spaced != 0, need_count = !need_sum || counts != nullptr;
+  const int  warps    = need_count ? 0 : rg::lane_warps(n, nbins, db.lncells);
+  size_t     smem     = 0;
+  int        G        = 0;
+  auto       kernel   = !need_sum    ? rg::histogram_kernel<false, true>
+                        : need_count ? rg::histogram_kernel<true, true>
+                                     : rg::histogram_kernel<true, false>;
+  if (warps > 0) {
+    static std::atomic<uint64_t> configured { 0 };
+    RG_CUDA_TRY(rg::ensure_max_dynamic_smem(rg::histogram_lane_kernel, static_cast<int>(rg::kLaneSmem), configured));
+    smem = rg::lane_smem(nbins, db.lncells, warps);
+    G    = ctx->sms * std::max(1, std::min(static_cast<int>(rg::kLaneSmem / smem), 2048 / (32 * rg::kLaneMaxWarps)));
+  } else {
+    smem = (((2 + rg::kSumCopies) * sizeof(float) * nbins + 15) & ~size_t(15)) + sizeof(double) * nbins +
+           sizeof(uint16_t) * (db.ncells + 1);
+    if (smem > 48 * 1024) {
+      RG_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+    }
+    int per_sm = 0;
+    RG_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, rg::kHistThreads, smem));
+    per_sm = std::max(1, std::min(per_sm, 8));
+    const int64_t want = std::max<int64_t>(1, (n + 4095) / 4096);
+    G = static_cast<int>(std::min<int64_t>(want, static_cast<int64_t>(ctx->sms) * per_sm));
   }
-  int per_sm = 0;
-  RG_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, rg::histogram_kernel,
-                                                            rg::kHistThreads, smem));
-  per_sm = std::max(1, std::min(per_sm, 8));
-  const int64_t want = std::max<int64_t>(1, (n + 4095) / 4096);
-  const int     G    = static_cast<int>(std::min<int64_t>(want, static_cast<int64_t>(ctx->sms) * per_sm));
 
   // one stream-ordered allocation for the per-block partials
-  const size_t   off_ps = sizeof(unsigned long long) * static_cast<size_t>(G) * nbins;
-  const size_t   bytes  = off_ps + sizeof(double) * static_cast<size_t>(G) * nbins;
+  const size_t   rows   = static_cast<size_t>(G) * nbins;
+  const size_t   off_ps = need_count ? sizeof(unsigned long long) * rows : 0;
+  const size_t   bytes  = off_ps + (need_sum ? sizeof(double) * rows : 0);
   unsigned char* buf    = nullptr;
   RG_CUDA_TRY(cudaMallocAsync(reinterpret_cast<void**>(&buf), bytes, s));
 
@@ -515,9 +869,17 @@ int rg_energy_distribution(const float* ux, const float* uy, const float* uz, in
   p.cell_shift = db.cell_shift;
   p.cell_base  = db.cell_base;
   p.ncells     = db.ncells;
-  p.part_counts = reinterpret_cast<unsigned long long*>(buf);
-  p.part_sums   = reinterpret_cast<double*>(buf + off_ps);
-  rg::histogram_kernel<<<G, rg::kHistThreads, smem, s>>>(p);
+  p.lcells     = db.lcells;
+  p.lshift     = db.lshift;
+  p.lbase      = db.lbase;
+  p.lncells    = db.lncells;
+  p.part_counts = need_count ? reinterpret_cast<unsigned long long*>(buf) : nullptr;
+  p.part_sums   = need_sum ? reinterpret_cast<double*>(buf + off_ps) : nullptr;
+  if (warps > 0) {
+    rg::histogram_lane_kernel<<<G, 32 * warps, smem, s>>>(p);
+  } else {
+    kernel<<<G, rg::kHistThreads, smem, s>>>(p);
+  }
   RG_CUDA_TRY(cudaGetLastError());
   rg::histogram_reduce_kernel<<<(nbins + 31) / 32, dim3(32, rg::kHistReduceRows), 0, s>>>(
     p.part_counts, p.part_sums, G, nbins, p.log_spaced, hist,

@@ -193,3 +193,40 @@ def test_more_than_2_pow_31_particles(gpu):
     np.testing.assert_array_equal(c, c1 + c2)
     m = h > 0
     assert np.max(np.abs(h1[m] + h2[m] - h[m]) / h[m]) < 1e-6
+
+
+@pytest.fixture(scope="module")
+def many():
+    """More particles than the per-lane histogram asks for, with NaN, one far above any bin and one at rest."""
+    P = particles(6_000_007, seed=77, umax=3e3)
+    u = [P[k] for k in ("ux", "uy", "uz")]
+    for i, v in enumerate((np.nan, 1e30, 0.0)):
+        for c in u:
+            c[10 + i] = 0.0
+        u[0][10 + i] = v
+    return u
+
+
+@pytest.mark.parametrize("n,offset", [(1, 0), (4099, 0), (200_001, 1), (6_000_003, 0), (6_000_000, 1)])
+@pytest.mark.parametrize("nb,log_spaced,fourvel", [(1, True, True), (33, True, False), (200, True, True), (220, True, False),
+                                                   (380, True, True), (200, False, True)])
+def test_without_counts(gpu, oracle_lib, many, n, offset, nb, log_spaced, fourvel):
+    """The histogram alone (no counts asked for): per-lane copies of the bins for many particles and
+    up to about 220 bins, atomics otherwise; groups of four and the remainder."""
+    u = [c[:n] for c in many]
+    bins = (oracle_lib.logspace(1e-2, 1e3, nb) if log_spaced else oracle_lib.linspace(0.5, 900.0, nb)) if nb > 1 \
+        else np.array([2.0], np.float32)
+    T = [torch.from_numpy(np.concatenate([np.zeros(offset, np.float32), c])).to(gpu)[offset:] for c in u]
+    hist = torch.full((nb,), -1.0, device=gpu)
+    capi.check(capi.lib().rg_energy_distribution(T[0].data_ptr(), T[1].data_ptr(), T[2].data_ptr(), n,
+                                                 bins.ctypes.data, nb, int(log_spaced), int(fourvel),
+                                                 hist.data_ptr(), None, 0))
+    torch.cuda.synchronize()
+    h = hist.cpu().numpy().astype(np.float64)
+    _, h64, cnt = oracle_lib.energy_distribution(*u, bins, log_spaced, fourvel)
+    if not log_spaced:
+        np.testing.assert_array_equal(h, cnt.astype(np.float32).astype(np.float64))
+        return
+    fin = np.isfinite(h64)
+    assert np.array_equal(np.isnan(h), np.isnan(h64)) and np.array_equal(np.isinf(h), np.isinf(h64))
+    assert np.all(np.abs(h[fin] - h64[fin]) <= 1e-6 * h64[fin])
