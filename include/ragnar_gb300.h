@@ -71,6 +71,15 @@ int rg_device_sm_count(int* sms);
  * deep_copy (array.hpp:21-30, array.cpp:46-51). */
 int rg_malloc(void** ptr, size_t bytes);
 int rg_free(void* ptr);
+
+/* Device memory for callers that order all work on a device's null stream (as the drop-in
+ * module does): blocks of up to 1 MB come from idle ones of the current device, of which at
+ * most 32 MB are kept, larger ones from rg_malloc.  A block given back may be handed out again
+ * at once: its next use on the null stream comes after the last one's.  `device` receives what
+ * rg_block_free needs.  rg_finalize gives the idle blocks back.  Callable from any thread. */
+int rg_block_malloc(void** ptr, size_t bytes, int32_t* device);
+int rg_block_free(void* ptr, size_t bytes, int32_t device);
+
 int rg_memcpy_htod(void* dst, const void* src, size_t bytes, void* stream);
 int rg_memcpy_dtoh(void* dst, const void* src, size_t bytes, void* stream);
 int rg_memcpy_dtod(void* dst, const void* src, size_t bytes, void* stream);

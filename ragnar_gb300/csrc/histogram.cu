@@ -853,7 +853,7 @@ int rg_energy_distribution(const float* ux, const float* uy, const float* uz, in
   const size_t   off_ps = need_count ? sizeof(unsigned long long) * rows : 0;
   const size_t   bytes  = off_ps + (need_sum ? sizeof(double) * rows : 0);
   unsigned char* buf    = nullptr;
-  RG_CUDA_TRY(cudaMallocAsync(reinterpret_cast<void**>(&buf), bytes, s));
+  RG_TRY(rg::scratch_alloc(reinterpret_cast<void**>(&buf), bytes, s));
 
   rg::HistParams p {};
   p.ux         = ux;

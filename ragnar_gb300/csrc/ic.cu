@@ -591,7 +591,7 @@ int rg_ic_spectrum(const float* gbins, const float* f, int32_t ng, int32_t log_s
   const size_t   off_part = off_pairs + up(sizeof(double) * static_cast<size_t>(splits) * ne);
   const size_t   bytes    = off_part + sizeof(double) * static_cast<size_t>(grid) * nslices * slice_w;
   unsigned char* buf      = nullptr;
-  RG_CUDA_TRY(cudaMallocAsync(reinterpret_cast<void**>(&buf), bytes, s));
+  RG_TRY(rg::scratch_alloc(reinterpret_cast<void**>(&buf), bytes, s));
   rg::IcParams p {};
   p.gb         = gbins;
   p.fp         = f;

@@ -117,6 +117,76 @@ namespace rg {
     }
   }
 
+  int scratch_alloc(void** p, size_t bytes, cudaStream_t s) {
+    DeviceContext* c = nullptr;
+    RG_TRY(context(&c));
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    RG_CUDA_TRY(cudaStreamIsCapturing(s, &capture));
+    if (capture != cudaStreamCaptureStatusNone) { // becomes an allocation of the graph
+      RG_CUDA_TRY(cudaMallocAsync(p, bytes, s));
+      return RG_OK;
+    }
+    {
+      std::lock_guard<std::mutex> lock(ctx_mutex());
+      if (!c->scratch) {
+        cudaMemPoolProps props {};
+        props.allocType     = cudaMemAllocationTypePinned;
+        props.handleTypes   = cudaMemHandleTypeNone;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id   = c->device;
+        uint64_t      keep  = kScratchKept;
+        cudaMemPool_t pool  = nullptr;
+        RG_CUDA_TRY(cudaMemPoolCreate(&pool, &props));
+        const cudaError_t e = cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+        if (e != cudaSuccess) {
+          cudaMemPoolDestroy(pool);
+          return cuda_error(e, "scratch pool");
+        }
+        c->scratch = pool;
+      }
+    }
+    RG_CUDA_TRY(cudaMallocFromPoolAsync(p, bytes, c->scratch, s));
+    return RG_OK;
+  }
+
+  // ---- blocks ordered on the null stream ----
+  namespace {
+    constexpr size_t kBlockMax  = size_t(1) << 20;
+    constexpr size_t kBlocksKept = size_t(32) << 20; // idle bytes over all devices
+
+    struct BlockPool {
+      std::mutex                                    mu;
+      std::map<std::pair<int, size_t>, std::vector<void*>> idle; // by device and size
+      size_t                                        bytes = 0;
+    };
+
+    BlockPool& block_pool() { // never destroyed, as the contexts
+      static auto* p = new BlockPool();
+      return *p;
+    }
+
+    // Four sizes per octave, 512 bytes at least.
+    size_t block_size(size_t bytes) {
+      size_t step = 512;
+      while (step * 8 < bytes) {
+        step *= 2;
+      }
+      return (bytes + step - 1) / step * step;
+    }
+
+    void free_idle_blocks() {
+      BlockPool&                  p = block_pool();
+      std::lock_guard<std::mutex> lock(p.mu);
+      for (auto& kv : p.idle) {
+        for (void* q : kv.second) {
+          cudaFree(q);
+        }
+      }
+      p.idle.clear();
+      p.bytes = 0;
+    }
+  } // namespace
+
   void free_staging(DeviceContext& c) {
     c.staging.reset();
   }
@@ -170,6 +240,8 @@ int rg_init(int device) {
 
 int rg_finalize(void) {
   rg::free_threshold_cache();
+  rg::free_plan_caches();
+  rg::free_idle_blocks();
   std::lock_guard<std::mutex> lock(rg::ctx_mutex());
   for (auto& kv : rg::contexts()) {
     int cur = 0;
@@ -177,6 +249,9 @@ int rg_finalize(void) {
     cudaSetDevice(kv.first);
     rg::free_staging(*kv.second);
     rg::free_tables(*kv.second);
+    if (kv.second->scratch) {
+      cudaMemPoolDestroy(kv.second->scratch); // outstanding scratch keeps its memory until it is freed
+    }
     cudaSetDevice(cur);
   }
   rg::contexts().clear();
@@ -222,6 +297,52 @@ int rg_free(void* ptr) {
     RG_CUDA_TRY(cudaFree(ptr));
   }
   return RG_OK;
+}
+
+int rg_block_malloc(void** ptr, size_t bytes, int32_t* device) {
+  *ptr = nullptr;
+  int dev = 0;
+  RG_CUDA_TRY(cudaGetDevice(&dev));
+  *device = dev;
+  if (bytes == 0 || bytes > rg::kBlockMax) {
+    return rg_malloc(ptr, bytes);
+  }
+  const size_t size = rg::block_size(bytes);
+  {
+    rg::BlockPool&              p = rg::block_pool();
+    std::lock_guard<std::mutex> lock(p.mu);
+    const auto                  it = p.idle.find({ dev, size });
+    if (it != p.idle.end() && !it->second.empty()) {
+      *ptr = it->second.back();
+      it->second.pop_back();
+      p.bytes -= size;
+      return RG_OK;
+    }
+  }
+  cudaError_t e = cudaMalloc(ptr, size);
+  if (e == cudaErrorMemoryAllocation) {
+    cudaGetLastError();
+    rg::free_idle_blocks();
+    e = cudaMalloc(ptr, size);
+  }
+  return e == cudaSuccess ? RG_OK : rg::cuda_error(e, "rg_block_malloc");
+}
+
+int rg_block_free(void* ptr, size_t bytes, int32_t device) {
+  if (!ptr) {
+    return RG_OK;
+  }
+  if (bytes <= rg::kBlockMax) {
+    const size_t                size = rg::block_size(bytes);
+    rg::BlockPool&              p    = rg::block_pool();
+    std::lock_guard<std::mutex> lock(p.mu);
+    if (p.bytes + size <= rg::kBlocksKept) {
+      p.idle[{ device, size }].push_back(ptr);
+      p.bytes += size;
+      return RG_OK;
+    }
+  }
+  return rg_free(ptr);
 }
 
 int rg_memcpy_htod(void* dst, const void* src, size_t bytes, void* stream) {

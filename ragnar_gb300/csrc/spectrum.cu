@@ -933,12 +933,46 @@ namespace rg {
       return RG_OK;
     }
 
-    std::mutex& oneshot_mutex() {
-      static std::mutex m;
-      return m;
+    // Plans of the calls that take none, keyed on everything a plan is made of: (device, bins,
+    // scalars).  Particle plans stay in the map (at most kParticlePlans).  A plan of
+    // rg_synchrotron_spectrum_from_dist, which returns when its result is there, is taken out of the
+    // list while a call uses it, so that calls of several threads or streams never share one (at
+    // most kDistPlans idle ones): making it anew costs eight allocations and five copies.
+    constexpr std::size_t kParticlePlans = 32, kDistPlans = 8;
+    using PlanKey = std::tuple<int, std::vector<float>, float, float, float>;
+
+    struct PlanCaches {
+      std::mutex                                            mu;
+      std::map<PlanKey, rg_spectrum_plan*>                  particles;
+      std::vector<std::pair<PlanKey, rg_spectrum_plan*>>    dist; // idle, most recent last
+    };
+
+    PlanCaches& plan_caches() { // never destroyed: its plans are device memory (rg_finalize frees them)
+      static auto* c = new PlanCaches();
+      return *c;
+    }
+
+    void free_particle_plans(PlanCaches& c) {
+      for (auto& kv : c.particles) {
+        rg_spectrum_plan_destroy(kv.second);
+      }
+      c.particles.clear();
     }
 
   } // namespace
+
+  void free_plan_caches() {
+    PlanCaches&                 c = plan_caches();
+    std::lock_guard<std::mutex> lock(c.mu);
+    if (!c.particles.empty()) {
+      cudaDeviceSynchronize();
+    }
+    free_particle_plans(c);
+    for (auto& kv : c.dist) {
+      rg_spectrum_plan_destroy(kv.second);
+    }
+    c.dist.clear();
+  }
 
   // A plan for particles or (source kSrcDist) for one tabulated distribution; only particle
   // plans over log-uniform bins take a bin-aligned smooth table.
@@ -1307,32 +1341,25 @@ int rg_spectrum_run_plain(const rg_spectrum_plan* cplan, const rg_particles* p, 
 
 int rg_synchrotron_spectrum(const rg_particles* p, const float* bins, int32_t nbins, float B0,
                             float g_syn, float e_syn_at_g_syn, float* out, void* stream) {
-  // plans are cached by (device, bins, scalars)
-  using Key = std::tuple<int, std::vector<float>, float, float, float>;
-  static std::map<Key, rg_spectrum_plan*> cache;
   if (nbins < 0 || (nbins > 0 && !bins)) {
     return rg::set_error(RG_ERR_ARGUMENT, "bins: need nbins >= 0 host values");
   }
   int dev = 0;
   RG_CUDA_TRY(cudaGetDevice(&dev));
-  Key               key { dev, std::vector<float>(bins, bins + nbins), B0, g_syn, e_syn_at_g_syn };
-  rg_spectrum_plan* pl = nullptr;
-  {
-    std::lock_guard<std::mutex> lock(rg::oneshot_mutex());
-    auto                        it = cache.find(key);
-    if (it == cache.end()) {
-      RG_TRY(rg_spectrum_plan_create(bins, nbins, B0, g_syn, e_syn_at_g_syn, RG_TABLE_REFERENCE, &pl));
-      if (cache.size() >= 32) {
-        RG_CUDA_TRY(cudaDeviceSynchronize());
-        for (auto& kv : cache) {
-          rg_spectrum_plan_destroy(kv.second);
-        }
-        cache.clear();
-      }
-      cache.emplace(key, pl);
-    } else {
-      pl = it->second;
+  rg::PlanKey                 key { dev, std::vector<float>(bins, bins + nbins), B0, g_syn, e_syn_at_g_syn };
+  rg::PlanCaches&             c  = rg::plan_caches();
+  rg_spectrum_plan*           pl = nullptr;
+  std::lock_guard<std::mutex> lock(c.mu); // also while the run's launches are queued: they share the plan's tables
+  auto                        it = c.particles.find(key);
+  if (it == c.particles.end()) {
+    RG_TRY(rg_spectrum_plan_create(bins, nbins, B0, g_syn, e_syn_at_g_syn, RG_TABLE_REFERENCE, &pl));
+    if (c.particles.size() >= rg::kParticlePlans) {
+      RG_CUDA_TRY(cudaDeviceSynchronize());
+      rg::free_particle_plans(c);
     }
+    c.particles.emplace(std::move(key), pl);
+  } else {
+    pl = it->second;
   }
   return rg_spectrum_run(pl, p, out, stream);
 }
@@ -1360,40 +1387,67 @@ int rg_synchrotron_spectrum_from_dist(const float* gbeta, const float* f, int32_
   if (ng < 0 || nbins < 0 || (ng > 0 && (!gbeta || !f)) || (nbins > 0 && !out)) {
     return rg::set_error(RG_ERR_ARGUMENT, "rg_synchrotron_spectrum_from_dist: bad arguments");
   }
-  auto pl        = std::make_unique<rg_spectrum_plan>();
-  pl->source     = rg::kSrcDist;
-  pl->log_spaced = log_spaced ? 1 : 0;
-  pl->g_syn      = g_syn;
-  pl->eps        = e_syn_at_g_syn;
-  int st         = rg::create_plan_common(pl.get(), bins, nbins);
-  // e_peak(g) = K0 gbeta^2 with K0 = eps / g^2 (synchrotron.hpp:78-79)
-  const double K0 = static_cast<double>(e_syn_at_g_syn) / (static_cast<double>(g_syn) * g_syn);
-  pl->zero        = !(K0 > 0.0) || !std::isfinite(K0);
-  pl->amp         = 1.0f;
-  if (st == RG_OK) {
-    double ln_xmin, dln;
-    int    nseg;
-    rg::table_geometry(pl.get(), ln_xmin, dln, nseg);
-    st = rg::plan_prepare_bins(pl.get(), ln_xmin, dln, nseg, pl->zero ? 0.0 : std::log(K0));
+  if (nbins > 0 && !bins) {
+    return rg::set_error(RG_ERR_ARGUMENT, "bins: need nbins >= 0 host values");
   }
-  auto s = static_cast<cudaStream_t>(stream);
+  int dev = 0;
+  RG_CUDA_TRY(cudaGetDevice(&dev));
+  rg::PlanKey       key { dev, std::vector<float>(bins, bins + nbins), log_spaced ? 1.0f : 0.0f, g_syn, e_syn_at_g_syn };
+  rg::PlanCaches&   c = rg::plan_caches();
+  rg_spectrum_plan* pl = nullptr;
+  {
+    std::lock_guard<std::mutex> lock(c.mu);
+    for (auto it = c.dist.begin(); it != c.dist.end(); ++it) {
+      if (it->first == key) {
+        pl = it->second;
+        c.dist.erase(it);
+        break;
+      }
+    }
+  }
+  int st = RG_OK;
+  if (!pl) {
+    pl             = new rg_spectrum_plan();
+    pl->source     = rg::kSrcDist;
+    pl->log_spaced = log_spaced ? 1 : 0;
+    pl->g_syn      = g_syn;
+    pl->eps        = e_syn_at_g_syn;
+    st             = rg::create_plan_common(pl, bins, nbins);
+    // e_peak(g) = K0 gbeta^2 with K0 = eps / g^2 (synchrotron.hpp:78-79)
+    const double K0 = static_cast<double>(e_syn_at_g_syn) / (static_cast<double>(g_syn) * g_syn);
+    pl->zero        = !(K0 > 0.0) || !std::isfinite(K0);
+    pl->amp         = 1.0f;
+    if (st == RG_OK) {
+      double ln_xmin, dln;
+      int    nseg;
+      rg::table_geometry(pl, ln_xmin, dln, nseg);
+      st = rg::plan_prepare_bins(pl, ln_xmin, dln, nseg, pl->zero ? 0.0 : std::log(K0));
+    }
+  }
   if (st == RG_OK) {
     const float* comp[rg::kComps] = {};
     comp[0]                       = gbeta;
     comp[1]                       = f;
-    st                            = rg::run_fused(pl.get(), comp, nullptr, ng, 1, out, s);
+    st = rg::run_fused(pl, comp, nullptr, ng, 1, out, static_cast<cudaStream_t>(stream));
   }
   if (st == RG_OK) {
-    const cudaError_t e = cudaStreamSynchronize(s);
-    if (e != cudaSuccess) {
-      st = rg::cuda_error(e, "rg_synchrotron_spectrum_from_dist");
+    st = rg_spectrum_plan_check(pl, stream); // waits for the result
+  }
+  if (st != RG_OK) {
+    rg_spectrum_plan_destroy(pl);
+    return st;
+  }
+  rg_spectrum_plan* old = nullptr;
+  {
+    std::lock_guard<std::mutex> lock(c.mu);
+    if (c.dist.size() >= rg::kDistPlans) {
+      old = c.dist.front().second;
+      c.dist.erase(c.dist.begin());
     }
+    c.dist.emplace_back(std::move(key), pl);
   }
-  if (st == RG_OK) {
-    st = rg_spectrum_plan_check(pl.get(), stream);
-  }
-  rg_spectrum_plan_destroy(pl.release());
-  return st;
+  rg_spectrum_plan_destroy(old);
+  return RG_OK;
 }
 
 } // extern "C"

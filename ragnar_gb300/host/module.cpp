@@ -64,7 +64,9 @@ namespace rgh {
   template <class T>
   py::array_t<T> as_array(const Array1D<T>& a) {
     py::array_t<T> out(static_cast<py::ssize_t>(a.n));
-    if (a.n) {
+    if (a.host) {
+      std::copy(a.host->begin(), a.host->end(), out.mutable_data());
+    } else if (a.n) {
       check(rg_memcpy_dtoh(out.mutable_data(), a.data(), a.n * sizeof(T), nullptr));
       check(rg_stream_synchronize(nullptr));
     }
@@ -296,7 +298,7 @@ namespace rgh {
 
   template <unsigned short D>
   Array1D<float> component(Particles<D>& P, int c, const char* name) {
-    Array1D<float> out(P.nactive());
+    Array1D<float> out(P.nactive(), false);
     if (P.nactive()) {
       check(rg_memcpy_dtod(out.data(), P.comp(c), P.nactive() * sizeof(float), nullptr));
       check(rg_stream_synchronize(nullptr));
@@ -311,7 +313,7 @@ namespace rgh {
       py::print("Computing energy distribution for", P.label(), "...", "end"_a = "", "flush"_a = true);
     }
     const auto     hb = bins.to_host();
-    Array1D<float> hist(bins.extent());
+    Array1D<float> hist(bins.extent(), false);
     if (!hb.empty()) {
       const auto v = P.view();
       for (int d = 0; d < 3; ++d) {
@@ -345,14 +347,14 @@ namespace rgh {
     if (bins.unit != EnergyUnits::mec2 and bins.unit != EnergyUnits::mpc2) {
       throw std::runtime_error("bins_e_syn must be in units of mc^2");
     }
-    const auto     hb = bins.to_host();
-    Array1D<float> out(bins.extent());
+    const auto hb = bins.to_host();
     if (P.is_allocated()) {
       for (int d = 0; d < 3; ++d) {
         P.comp(Particles<D>::kU + d);
       }
     }
     const rg_particles v = P.view();
+    Array1D<float>     out(bins.extent(), v.n <= 0);
     if (!hb.empty() && v.n > 0) {
       py::gil_scoped_release nogil;
       check(rg_synchrotron_spectrum(&v, hb.data(), static_cast<int32_t>(hb.size()), B0, g_syn, eps,
@@ -422,7 +424,7 @@ namespace rgh {
                 "threads", "end"_a = "", "flush"_a = true);
     }
     const auto     hb = bins.to_host();
-    Array1D<float> out(bins.extent());
+    Array1D<float> out(bins.extent(), false);
     if (!hb.empty()) {
       py::gil_scoped_release nogil;
       check(rg_synchrotron_spectrum_from_dist(
@@ -451,7 +453,7 @@ namespace rgh {
                 human(static_cast<double>(dist_prtls.f.extent()) * dist_soft.f.extent() * bins_e_ic.extent()),
                 "threads", "end"_a = "", "flush"_a = true);
     }
-    Array1D<float> out(bins_e_ic.extent());
+    Array1D<float> out(bins_e_ic.extent(), false);
     if (out.n > 0) {
       py::gil_scoped_release nogil;
       check(rg_ic_spectrum(dist_prtls.bins.data(), dist_prtls.f.data(), static_cast<int32_t>(dist_prtls.f.extent()),

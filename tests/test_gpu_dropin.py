@@ -280,3 +280,46 @@ def test_batched_extension(oracle_lib):
     P = {"ux": u[0], "uy": u[1], "uz": u[2], "bx": b[0], "by": b[1], "bz": b[2]}
     truth = oracle_lib.sync_spectrum_batched_f64(P, offs, g["iso_bins"], 1, 1, 1, table)
     assert max_rel(S[0], truth[0]) <= 1e-5 and np.all(S[1] == 0) and max_rel(S[2], truth[2]) <= 1e-5
+
+
+# --- memory behind the calls ---------------------------------------------------------
+def _dist_call(k, n=300):
+    dist = rg.TabulatedDistribution(rg.Logbins(1.0, 1e4, n), rg.PlawGenerator(-2.0 - 0.01 * k, 1.0, 1e4))
+    bins = rg.Logbins(1e-2 * (1.0 + k), 1e6, 200, rg.EnergyUnits.mec2)
+    return rg.SynchrotronSpectrumFromDist(dist, bins, 1.0, 1.0).as_array()
+
+
+def test_distribution_calls_of_several_threads():
+    """More grids than plans are kept, from four threads at a time and again after Finalize: every
+    call gives what a single one gave."""
+    from concurrent.futures import ThreadPoolExecutor  # noqa: PLC0415
+
+    want = [_dist_call(k) for k in range(12)]
+    assert all(np.any(w > 0) for w in want)
+    with ThreadPoolExecutor(4) as pool:
+        got = list(pool.map(_dist_call, [k % 12 for k in range(96)]))
+    for k, g in enumerate(got):
+        np.testing.assert_array_equal(g, want[k % 12])
+    rg.Finalize()
+    rg.Initialize()
+    for k in (11, 0):
+        np.testing.assert_array_equal(_dist_call(k), want[k])
+
+
+@pytest.mark.parametrize("n", [1, 127, 128, 129, 65536, 65537, 262144, 262145])
+def test_arrays_reuse_memory_without_traces(n):
+    """Arrays around the sizes at which blocks change class, at which values stay on the host and at
+    which the driver allocates: values survive the reuse of memory that others gave back, and
+    components that nobody wrote are zero."""
+    for rep in range(3):
+        a = np.arange(n, dtype=np.float32) + rep
+        keep = [rg.Array1D_f(a + k) for k in range(4)]
+        del keep[1]
+        keep.append(rg.Array1D_f(a - 1))
+        for arr, off in zip(keep, (0, 2, 3, -1)):
+            np.testing.assert_array_equal(arr.as_array(), a + np.float32(off))
+        p = rg.Particles_3D("p")
+        p.fromArrays({"U1": a + 1.0, "U2": a + 1.0, "U3": a + 1.0})
+        assert not p.B(1).as_array().any()
+        assert not rg.SynchrotronSpectrum_3D(p, rg.Logbins(1e-2, 1e2, 50, rg.EnergyUnits.mec2), 1.0, 1.0,
+                                             1.0).as_array().any()
