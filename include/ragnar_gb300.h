@@ -321,6 +321,13 @@ int rg_synchrotron_spectrum_from_dist(const float* gbeta, const float* f, int32_
                                       float g_syn, float e_syn_at_g_syn, float* out,
                                       void* stream);
 
+/* Misfit of n spectrum values S to T (device): mean of (ln S - ln T)^2 over those above `floor`
+ * times the largest of both arrays.  inv_count: 1 / (number of values that count, at least 1);
+ * r[i] = dloss/dS[i] = 2 (ln S - ln T) / S inv_count and a[i] = 1 / S where value i counts, else 0,
+ * so that dr/dS = 2 a^2 inv_count - r a and da/dS = -a^2. */
+int rg_log_mse(const float* S, const float* T, int64_t n, float floor, float* r, float* a, float* loss,
+               float* inv_count, void* stream);
+
 /* --------------------------------------------------------------------------
  * Many distributions at once on the tensor cores
  * ------------------------------------------------------------------------ */

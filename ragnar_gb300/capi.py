@@ -67,6 +67,8 @@ def _declare(L: ctypes.CDLL) -> None:
         "rg_device_sm_count": [ctypes.POINTER(_int)],
         "rg_malloc": [ctypes.POINTER(_vp), ctypes.c_size_t],
         "rg_free": [_vp],
+        "rg_block_malloc": [ctypes.POINTER(_vp), ctypes.c_size_t, ctypes.POINTER(_i32)],
+        "rg_block_free": [_vp, ctypes.c_size_t, _i32],
         "rg_memcpy_htod": [_vp, _vp, ctypes.c_size_t, _vp],
         "rg_memcpy_dtoh": [_vp, _vp, ctypes.c_size_t, _vp],
         "rg_memcpy_dtod": [_vp, _vp, ctypes.c_size_t, _vp],
@@ -103,6 +105,7 @@ def _declare(L: ctypes.CDLL) -> None:
         "rg_dist_plan_create": [_vp, _i32, _f32, _f32, _i32, _i32, ctypes.POINTER(_vp)],
         "rg_dist_run": [_vp, _vp, _vp, _i32, _vp, _vp],
         "rg_dist_adjoint": [_vp, _vp, _vp, _i32, _vp, _vp, _vp],
+        "rg_log_mse": [_vp, _vp, _i64, _f32, _vp, _vp, _vp, _vp, _vp],
         "rg_fromdist_plan_create": [_vp, _i32, _i32, _vp, _i32, _f32, _f32, _i32, _i32, _i32,
                                     ctypes.POINTER(_vp)],
         "rg_fromdist_plan_destroy": [_vp],

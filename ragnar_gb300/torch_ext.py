@@ -124,10 +124,59 @@ def synchrotron_from_dist(plan: capi.DistPlan, gbeta, f):
     return _FromDist.apply(plan, gbeta, f)
 
 
+class _LogMse(torch.autograd.Function):
+    """The misfit and the two arrays its derivatives are made of, its gradient r and a = 1 / S on the
+    c bins that count.  They are outputs, saved as such: a backward that is differentiated again
+    reaches S through them, to any order (dr/dS = 2 a^2 / c - r a, da/dS = -a^2), and S itself is not
+    kept."""
+
+    @staticmethod
+    def forward(ctx, S, S_target, floor):
+        r, a = torch.empty_like(S), torch.empty_like(S)
+        loss, inv = S.new_empty(()), S.new_empty(())
+        capi.check(capi.lib().rg_log_mse(S.data_ptr(), S_target.data_ptr(), S.numel(), floor, r.data_ptr(),
+                                         a.data_ptr(), loss.data_ptr(), inv.data_ptr(), _stream(S.device)))
+        ctx.set_materialize_grads(False)
+        ctx.save_for_backward(r, a, inv)
+        return loss, r, a
+
+    @staticmethod
+    def backward(ctx, g, gr, ga):
+        r, a, inv = ctx.saved_tensors
+        gS = None if g is None else r * g
+        if gr is not None:
+            gr = gr * (2 * inv * a * a - r * a)
+            gS = gr if gS is None else gS + gr
+        if ga is not None:
+            ga = ga * (a * a)
+            gS = -ga if gS is None else gS - ga
+        return gS, None, None
+
+
+def _plain_cuda(*tensors) -> bool:
+    """Contiguous float32 tensors of the current CUDA device, and nothing that looks at the single
+    operations: no tensor subclass, function transform, dual level, tracer or mode."""
+    dev = torch.cuda.current_device() if tensors[0].is_cuda else -1
+    return (all(type(t) is torch.Tensor and t.is_cuda and t.device.index == dev and t.dtype == torch.float32
+                and t.is_contiguous() for t in tensors)
+            and torch._C._functorch.peek_interpreter_stack() is None
+            and torch.autograd.forward_ad._current_level < 0
+            and torch._C._len_torch_dispatch_stack() == 0
+            and torch._C._len_torch_function_stack() == 0
+            and not torch.jit.is_tracing() and not torch.compiler.is_compiling())
+
+
 def log_mse(S, S_target, floor: float = 1e-12):
     """mean of (log S - log S_target)^2 over the bins where both spectra exceed
     `floor` times their peak (bins with a vanishing spectrum are left out: their
-    1/S weight would overflow and carries no information)."""
+    1/S weight would overflow and carries no information).
+
+    Plain CUDA spectra against a constant target take rg_log_mse (one launch for a spectrum, three
+    for many); anything else these tensor operations."""
+    if (isinstance(floor, (int, float)) and floor >= 0 and type(S) is torch.Tensor and type(S_target) is torch.Tensor
+            and not S_target.requires_grad and S.shape == S_target.shape and S.numel() > 0
+            and _plain_cuda(S, S_target)):
+        return _LogMse.apply(S, S_target, float(floor))[0]
     m = (S > floor * S.detach().max()) & (S_target > floor * S_target.max())
     d = torch.log(torch.where(m, S, torch.ones_like(S))) - torch.log(
         torch.where(m, S_target, torch.ones_like(S_target)))
