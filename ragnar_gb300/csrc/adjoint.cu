@@ -62,7 +62,7 @@ namespace rg {
 
       const int     tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
       const int     G        = gridDim.x, b = blockIdx.x;
-      const int64_t n_items  = total_items(p.item_prefix, p.nseg, p.n_single);
+      const int64_t n_items  = total_items(p.item_prefix, p.nseg, p.n_single, p.chunk);
       const int64_t it_begin = static_cast<int64_t>(b) * n_items / G;
       const int64_t it_end   = static_cast<int64_t>(b + 1) * n_items / G;
       if (it_begin >= it_end) {
@@ -318,8 +318,7 @@ namespace rg {
       }
       int G = pl->grid;
       if (!d_off) {
-        const int64_t items = (n_single + kChunk - 1) / kChunk;
-        G = static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(items, pl->grid)));
+        G = item_blocks(n_single, pl->grid);
         if (n_single == 0) {
           return RG_OK;
         }

@@ -844,7 +844,9 @@ int rg_energy_distribution(const float* ux, const float* uy, const float* uz, in
     int per_sm = 0;
     RG_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, rg::kHistThreads, smem));
     per_sm = std::max(1, std::min(per_sm, 8));
-    const int64_t want = std::max<int64_t>(1, (n + 4095) / 4096);
+    // at least 4096 particles a block, or 1024 while that leaves room on the chip (a call on 1e3
+    // particles 20 -> 14 us, 1e4 24 -> 13, 1e5 24 -> 15, 1e6 28 -> 23)
+    const int64_t want = std::max<int64_t>({ 1, (n + 4095) / 4096, std::min<int64_t>((n + 1023) / 1024, 2 * ctx->sms) });
     G = static_cast<int>(std::min<int64_t>(want, static_cast<int64_t>(ctx->sms) * per_sm));
   }
 

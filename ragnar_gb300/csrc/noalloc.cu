@@ -41,7 +41,7 @@ namespace rg {
 
   int launch_fused_reference(int K, const FusedParams& fp, int grid, cudaStream_t s);
   int preload_reference_kernels();
-  int launch_reduce_single(const double* partials, int grid, int64_t n, int nbins, const float* ebins,
+  int launch_reduce_single(const double* partials, int grid, int64_t n, int chunk, int nbins, const float* ebins,
                            const uint8_t* valid, const unsigned* status, float* out, cudaStream_t s);
   int build_reference_table_into(int n, float xmin, float xmax, float* d_x, float* d_y, float2* d_coef,
                                  float* d_grids, double& ln_xmin, double& dln, cudaStream_t s);
@@ -243,12 +243,12 @@ int rg_synchrotron_spectrum_noalloc(const rg_particles* p, const float* bins, in
   fp.partials    = reinterpret_cast<double*>(b + kOffPartials);
   fp.nslices     = 1;
   fp.status      = reinterpret_cast<unsigned*>(b + kOffStatus);
-  const int64_t items = (p->n + kChunk - 1) / kChunk;
-  const int     grid  = static_cast<int>(
-    std::max<int64_t>(1, std::min<int64_t>(items, std::min(kNoAllocMaxGrid, d.sms * kBlocksPerSM))));
+  const int blocks = std::min(kNoAllocMaxGrid, d.sms * kBlocksPerSM);
+  const int grid   = item_blocks(p->n, blocks);
+  fp.chunk         = item_size(p->n, blocks);
   const int K = std::max(1, (nbins + 31) / 32);
   RG_TRY(launch_fused_reference(K, fp, grid, s));
-  RG_TRY(launch_reduce_single(fp.partials, grid, p->n, nbins, reinterpret_cast<const float*>(b + kOffEbins),
+  RG_TRY(launch_reduce_single(fp.partials, grid, p->n, fp.chunk, nbins, reinterpret_cast<const float*>(b + kOffEbins),
                               reinterpret_cast<const uint8_t*>(b + kOffValid), fp.status, out, s));
   return RG_OK;
 }

@@ -55,16 +55,19 @@ namespace rg {
   namespace {
 
     // Rows of 32 bins combined per pass of flush_block: the pass's scratch, kFlushRows x
-    // kWarps x 32 doubles, is the 8 KB of the two (q, A) buffers.
+    // kWarps x 32 double-floats, is the 8 KB of the two (q, A) buffers.
     constexpr int kFlushRows = 4;
-    static_assert(kFlushRows * kWarps * 32 * sizeof(double) <= 2 * kChunk * sizeof(int2),
+    static_assert(kFlushRows * kWarps * 32 * sizeof(float2) <= 2 * kChunk * sizeof(int2),
                   "flush scratch must fit the (q, A) buffers");
 
-    // Sums the warps' double-float accumulators of one segment in warp order (FP64) and
-    // writes the block's partial row; the accumulators are cleared.  Called by the whole
-    // block at a point where no warp reads the (q, A) buffers that serve as scratch.
+    // Sums the warps' double-float accumulators of one segment in warp order and writes the
+    // block's partial row; the accumulators are cleared.  Called by the whole block at a point
+    // where no warp reads the (q, A) buffers that serve as scratch.  The warps are summed in
+    // double-floats and only the row's value is FP64: GB300 adds FP64 at 2 lanes a clock, and one FP64
+    // value per warp and bin took 3 to 7 us a block (one distribution of 5e3 nodes 25.0 -> 18.8 us).
+    // The loop over warps is not unrolled: unrolled, it costs the kernel's main loop 3 %.
     template <int K>
-    __device__ __forceinline__ void flush_block(float (&hi)[K], float (&lo)[K], double* scratch, double* dst,
+    __device__ __forceinline__ void flush_block(float (&hi)[K], float (&lo)[K], float2* scratch, double* dst,
                                                 int tid, bool accumulate) {
       const int lane = tid & 31, warp = tid >> 5;
 #pragma unroll
@@ -72,20 +75,21 @@ namespace rg {
 #pragma unroll
         for (int r = 0; r < kFlushRows; ++r) {
           if (k0 + r < K) {
-            scratch[(r * kWarps + warp) * 32 + lane] =
-              static_cast<double>(hi[k0 + r]) + static_cast<double>(lo[k0 + r]);
+            scratch[(r * kWarps + warp) * 32 + lane] = make_float2(hi[k0 + r], lo[k0 + r]);
           }
         }
         __syncthreads();
         const int r = tid >> 5;
         if (r < kFlushRows && k0 + r < K) {
-          double t = 0.0;
-#pragma unroll
+          ff t { 0.0f, 0.0f };
+#pragma unroll 1
           for (int w = 0; w < kWarps; ++w) {
-            t += scratch[(r * kWarps + w) * 32 + lane];
+            const float2 v = scratch[(r * kWarps + w) * 32 + lane];
+            t              = ff_add(t, ff { v.x, v.y });
           }
-          double* d = dst + (k0 + r) * 32 + lane;
-          *d        = accumulate ? *d + t : t;
+          const double v = static_cast<double>(t.hi) + static_cast<double>(t.lo);
+          double*      d = dst + (k0 + r) * 32 + lane;
+          *d             = accumulate ? *d + v : v;
         }
         __syncthreads();
       }
@@ -112,7 +116,7 @@ namespace rg {
       const int     tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
       const int     slice    = blockIdx.y;
       const int     G        = gridDim.x, b = blockIdx.x;
-      const int64_t n_items  = total_items(p.item_prefix, p.nseg, p.n_single);
+      const int64_t n_items  = total_items(p.item_prefix, p.nseg, p.n_single, p.chunk);
       const int64_t it_begin = static_cast<int64_t>(b) * n_items / G;
       const int64_t it_end   = static_cast<int64_t>(b + 1) * n_items / G;
       if (it_begin >= it_end) {
@@ -194,7 +198,7 @@ namespace rg {
           // block-uniform (info[st] is shared); every warp is past the previous item's
           // evaluation (the barrier above), so the (q, A) buffers are free
           if (cur_seg >= 0) {
-            flush_block<K>(hi, lo, reinterpret_cast<double*>(qa), block_partial(p, b, cur_seg, slice), tid,
+            flush_block<K>(hi, lo, reinterpret_cast<float2*>(qa), block_partial(p, b, cur_seg, slice), tid,
                            p.accumulate != 0);
           }
           cur_seg = I.seg;
@@ -254,7 +258,7 @@ namespace rg {
       }
       if (cur_seg >= 0) {
         __syncthreads(); // every warp is done reading the last item's (q, A)
-        flush_block<K>(hi, lo, reinterpret_cast<double*>(qa), block_partial(p, b, cur_seg, slice), tid,
+        flush_block<K>(hi, lo, reinterpret_cast<float2*>(qa), block_partial(p, b, cur_seg, slice), tid,
                        p.accumulate != 0);
       }
     }
@@ -323,6 +327,7 @@ namespace rg {
       const double*   partials;
       const int64_t*  item_prefix; // or null: one segment
       int64_t         n_single;
+      int             chunk; // particles per item of the launch
       int             grid;
       int             nslices;
       int             nseg;
@@ -350,7 +355,7 @@ namespace rg {
       bool       active = false;
       double     sum    = 0.0;
       if (bin < r.nbins && !failed) {
-        const int64_t n_items = total_items(r.item_prefix, r.nseg, r.n_single);
+        const int64_t n_items = total_items(r.item_prefix, r.nseg, r.n_single, r.chunk);
         const int64_t i0      = items_before(r.item_prefix, s);
         const int64_t i1      = r.item_prefix ? r.item_prefix[s + 1] : n_items;
         if (i1 > i0 && r.valid[bin]) {
@@ -786,6 +791,7 @@ namespace rg {
     fp.seg_off     = d_off;
     fp.item_prefix = d_prefix;
     fp.n_single    = n_single;
+    fp.chunk       = d_off ? kChunk : item_size(n_single, pl->grid);
     fp.nseg        = nseg;
     fp.P           = pl->d_P;
     fp.Prange      = pl->d_Prange;
@@ -826,12 +832,13 @@ namespace rg {
     return RG_OK;
   }
 
-  int launch_reduce_single(const double* partials, int grid, int64_t n, int nbins, const float* ebins,
+  int launch_reduce_single(const double* partials, int grid, int64_t n, int chunk, int nbins, const float* ebins,
                            const uint8_t* valid, const unsigned* status, float* out, cudaStream_t s) {
     ReduceParams rp {};
     rp.partials    = partials;
     rp.item_prefix = nullptr;
     rp.n_single    = n;
+    rp.chunk       = chunk;
     rp.grid        = grid;
     rp.nslices     = 1;
     rp.nseg        = 1;
@@ -861,6 +868,7 @@ namespace rg {
       rp.partials    = pl->d_partials;
       rp.item_prefix = d_prefix;
       rp.n_single    = n_single;
+      rp.chunk       = d_prefix ? kChunk : item_size(n_single, pl->grid);
       rp.grid        = grid;
       rp.nslices     = pl->nslices;
       rp.nseg        = nseg;
@@ -873,12 +881,6 @@ namespace rg {
       reduce_partials_kernel<<<rgrid, dim3(32, kReduceRows), 0, s>>>(rp);
       RG_CUDA_TRY(cudaGetLastError());
       return RG_OK;
-    }
-
-    // Blocks of the fused kernel over a single segment of n particles.
-    int single_segment_grid(const rg_spectrum_plan* pl, int64_t n) {
-      const int64_t items = (n + kChunk - 1) / kChunk;
-      return static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(items, pl->grid)));
     }
 
     // Launches fused + reduce.  `d_off` (device, nseg + 1) may be null for a
@@ -909,7 +911,7 @@ namespace rg {
       FusedParams fp;
       const int   nslots = fill_params(pl, comp, d_off, d_prefix, n_single, nseg, fp);
       // a single segment with fewer items than blocks uses fewer blocks
-      const int G = d_off ? pl->grid : single_segment_grid(pl, n_single);
+      const int G = d_off ? pl->grid : item_blocks(n_single, pl->grid);
       const bool any = d_off ? true : n_single > 0;
       if (any) {
         RG_TRY(timed_launch(pl, fp, dim3(G, pl->nslices), fused_smem(pl->table_mode, fp.hseg, nslots), s));
@@ -927,7 +929,7 @@ namespace rg {
       const int   nslots = fill_params(pl, comp, nullptr, nullptr, n, 1, fp);
       fp.accumulate      = accumulate ? 1 : 0;
       if (n > 0) {
-        RG_TRY(timed_launch(pl, fp, dim3(single_segment_grid(pl, n), pl->nslices),
+        RG_TRY(timed_launch(pl, fp, dim3(item_blocks(n, pl->grid), pl->nslices),
                             fused_smem(pl->table_mode, fp.hseg, nslots), s));
       }
       return RG_OK;
@@ -1281,7 +1283,7 @@ int rg_spectrum_run_host(rg_spectrum_plan* pl, const rg_particles* p, float* out
   }
   // the rows the chunks accumulated: as many blocks as the first (largest) chunk used
   const int64_t first = std::min(kStageChunk, n);
-  return rg::reduce_rows(pl, nullptr, first, rg::single_segment_grid(pl, first), 1, out, s);
+  return rg::reduce_rows(pl, nullptr, first, rg::item_blocks(first, pl->grid), 1, out, s);
 }
 
 int rg_spectrum_run_plain(const rg_spectrum_plan* cplan, const rg_particles* p, float* out,

@@ -459,3 +459,32 @@ def test_host_streaming_from_two_threads(gpu, oracle_lib, algo):
     for i in range(2):
         plans[i].check(streams[i].cuda_stream)
         same(outs[i].cpu(), alone[i], algo)
+
+
+@pytest.mark.parametrize("n", [1, 3, 31, 33, 9727, 9729, 20001, 155647, 155649])
+@pytest.mark.parametrize("source", ["particles", "dist"])
+def test_fused_item_sizes(gpu, oracle_lib, n, source):
+    """The fused kernel over one segment, with work items of 32 to 512 particles: sizes around the
+    smallest item, one item per block and the largest, on 40 and 513 bins, against FP64."""
+    table = oracle_lib.tabulate_ffunc()
+    for nbins in (40, 513):
+        bins = oracle_lib.logspace(1e-2, 1e6, nbins)
+        out = torch.full((nbins,), -1.0, device=gpu)
+        if source == "particles":
+            P = particles(n, seed=n, bfield="iso", weights=True)
+            T = {k: torch.from_numpy(v).to(gpu) for k, v in P.items()}
+            prt = capi.particles([T["ux"], T["uy"], T["uz"]], b=[T["bx"], T["by"], T["bz"]], w=T["w"])
+            plan = capi.SpectrumPlan(bins, 1.0, 1.0, 1.0)
+            plan.set_algorithm(capi.RG_ALGO_DIRECT)
+            plan.run(prt, out)
+            plan.check()
+            want = oracle_lib.sync_spectrum_f64(P, bins, 1.0, 1.0, 1.0, table)
+        else:
+            g = np.geomspace(1.0, 1e4, n).astype(np.float32) if n > 1 else np.array([30.0], np.float32)
+            f = (g.astype(np.float64) ** -2.2).astype(np.float32)
+            plan = capi.DistPlan(bins, 1.0, 1.0, True, capi.RG_TABLE_REFERENCE)
+            gd, fd = torch.from_numpy(g).to(gpu), torch.from_numpy(f).to(gpu)
+            plan.run_dist(gd, fd, out)
+            plan.check()
+            want = oracle_lib.sync_from_dist_f64(g, f, True, bins, 1.0, 1.0, table)[0]
+        assert max_rel(out.cpu().numpy(), want) <= SPECTRUM_RTOL
