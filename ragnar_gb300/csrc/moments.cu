@@ -241,22 +241,20 @@ namespace rg {
 
     constexpr int kFinWarps = 8;
     constexpr int kFinThreads = 32 * kFinWarps;
-    constexpr int kFinAhead = 8; // rows of up to 32 x kFinAhead entries are fetched one row ahead
 
     // A bin as the finish kernel reads it: (sorted position, Dc), and -Dl and 1 - Dl in segment
     // units as double-floats.
     struct FinBin {
       int    pos, Dc;
       float  nDh, nDl, mDh, mDl;
-      float2 pad;
     };
 
     // Shared memory: coefficients, bins, and per warp the bins' sums, the row (overwritten by the
-    // sums below) and the sums above; rows fetched ahead have a second buffer.
+    // sums below) and the sums above.
     size_t finish_smem(int max_bins, int nseg_tab) {
-      const size_t row = max_bins + 1, bufs = row <= 32 * kFinAhead ? 3 : 2;
-      return sizeof(float4) * (nseg_tab + 2) + sizeof(FinBin) * kSliceBins +
-             kFinWarps * (sizeof(float2) * kSliceBins + sizeof(float4) * bufs * row);
+      const size_t row = max_bins + 1, groups = (max_bins + 31) & ~31;
+      return sizeof(float4) * (nseg_tab + 2) + sizeof(FinBin) * groups +
+             kFinWarps * (sizeof(float2) * groups + sizeof(float4) * 2 * row);
     }
 
     __device__ __forceinline__ ff2 shfl_up_ff2(ff2 a, int o) {
@@ -275,35 +273,35 @@ namespace rg {
     }
 
     // One warp per cell row, kFinWarps rows in flight per block, blockIdx.y = (segment, slice).
-    // The row is copied to shared memory (coalesced, one row ahead for short rows) and set back to
-    // zero; a lane takes C consecutive entries (M0, and M1 in segment units, as packed
+    // The row is copied to shared memory (coalesced) and set back to zero; a lane takes C consecutive entries (M0, and M1 in segment units, as packed
     // double-floats scaled by a power of two), and the warp leaves the row's sums below (L) and
     // above (U) every threshold in shared memory.  U is summed from the row's end, not as
     // total - L, so that a bin with no particle above its threshold gets an exact zero.  Then
     // lanes own bins in the order of their cells, so that whole groups of 32 skip the cells their
     // table segments do not reach.  Double-floats (2^-44) because the FP64 pipe issues 1.6
     // operations per clock and SM: the FP64 scan and reduce kernels this replaces took 503 and
-    // 449 us for 256 spectra of 200 bins (this kernel 170 us, and no memset of 350 MB before the
-    // run).  Blocks add their bins' sums in FP64; the last block of a (segment, slice) writes the
+    // 449 us for 256 spectra of 200 bins (this kernel 124 us, and no memset of 350 MB before the
+    // run).  What bounds it is the latency of its chains: rows fetched one ahead take a third buffer, and
+    // with it two blocks fit an SM (146 us) instead of three.  Blocks add their bins' sums in FP64; the last block of a (segment, slice) writes the
     // spectrum.
     template <int C>
     __global__ void __launch_bounds__(kFinThreads) moments_finish_kernel(const __grid_constant__ MomentFinishParams r) {
       extern __shared__ __align__(16) unsigned char smem[];
       __shared__ int   wscale[kFinWarps];
       __shared__ bool  last;
-      constexpr bool   kAhead = C <= kFinAhead;
       const int  seg = blockIdx.y / r.nslices, slice = blockIdx.y % r.nslices;
       const int4 ms  = r.mslice[slice];
       const int  nv = ms.x, row = nv + 1, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+      const int  groups = (nv + 31) & ~31; // bins in groups of 32
       float4*    coef  = reinterpret_cast<float4*>(smem);
       FinBin*    bins  = reinterpret_cast<FinBin*>(coef + r.nseg_tab + 2);
-      float2*    sums  = reinterpret_cast<float2*>(bins + kSliceBins); // [kFinWarps][kSliceBins]
-      float2*    acc   = sums + warp * kSliceBins;
-      float4*    bufs  = reinterpret_cast<float4*>(sums + kFinWarps * kSliceBins) + (kAhead ? 3 : 2) * warp * row;
-      float4*    Us    = bufs + (kAhead ? 2 : 1) * row;
+      float2*    sums  = reinterpret_cast<float2*>(bins + groups); // [kFinWarps][groups]
+      float2*    acc   = sums + warp * groups;
+      float4*    buf   = reinterpret_cast<float4*>(sums + kFinWarps * groups) + 2 * warp * row;
+      float4*    Us    = buf + row;
       double2*   hist  = r.hist + seg * r.per_seg + ms.z;
       const int  c0 = blockIdx.x * kFinWarps + warp, cstep = gridDim.x * kFinWarps;
-      auto fetch = [&](int c, float4* buf) {
+      auto fetch = [&](int c) {
         if (c < ms.y) {
           double2* h = hist + static_cast<int64_t>(c) * row;
           for (int j = lane; j < row; j += 32) {
@@ -312,39 +310,30 @@ namespace rg {
         }
         copies_commit();
       };
-      fetch(c0, bufs);
+      fetch(c0);
       const bool failed = *r.status != kDevOk;
       for (int i = threadIdx.x; i < r.nseg_tab + 2; i += kFinThreads) {
         coef[i] = r.coef[i];
       }
-      for (int i = threadIdx.x; i < kSliceBins; i += kFinThreads) {
+      for (int i = threadIdx.x; i < groups; i += kFinThreads) {
         const int4  b  = r.bins[slice * kSliceBins + i];
         const float un = 1.0f / (1u << kMomFrac);
         const int   m  = (1 << kMomFrac) - b.z;
         const float dh = static_cast<float>(b.z), mh = static_cast<float>(m);
         bins[i] = FinBin { b.x, b.y, -dh * un, static_cast<float>(static_cast<int>(dh) - b.z) * un, mh * un,
-                           static_cast<float>(m - static_cast<int>(mh)) * un, make_float2(0.0f, 0.0f) };
+                           static_cast<float>(m - static_cast<int>(mh)) * un };
       }
-      for (int i = lane; i < kSliceBins; i += 32) {
+      for (int i = lane; i < groups; i += 32) {
         acc[i] = make_float2(0.0f, 0.0f);
       }
       __syncthreads();
       int scale = -2000; // this warp's sums hold their value times 2^-scale
-      int which = 0;
 #pragma unroll 1
       for (int c = c0; c < ms.y; c += cstep) {
-        float4* buf = bufs + (kAhead ? which * row : 0);
-        if (kAhead) {
-          fetch(c + cstep, bufs + (which ^ 1) * row);
-          which ^= 1;
-          copies_wait<1>();
-        } else {
-          if (c != c0) {
-            __syncwarp();
-            fetch(c, buf);
-          }
-          copies_wait<0>();
+        if (c != c0) {
+          fetch(c);
         }
+        copies_wait<0>();
         __syncwarp(); // every lane's copies of this row have landed
         double2* h = hist + static_cast<int64_t>(c) * row;
         double2  d[C];
@@ -368,7 +357,7 @@ namespace rg {
         if (top - 1023 > scale + 40) { // room for sums 2^40 above the first row's largest entry
           const int   down = top - 1023 - scale;
           const float f    = down > 126 ? 0.0f : __uint_as_float(static_cast<uint32_t>(127 - down) << 23);
-          for (int i = lane; i < kSliceBins; i += 32) {
+          for (int i = lane; i < groups; i += 32) {
             acc[i] = make_float2(acc[i].x * f, acc[i].y * f);
           }
           scale = top - 1023;
@@ -438,7 +427,7 @@ namespace rg {
             acc[q + lane]  = make_float2(n.hi, n.lo);
           }
         }
-        __syncwarp(); // the buffers are reused
+        __syncwarp(); // the row's buffer takes the next row
       }
       copies_wait<0>();
       // the block's sums, at its warps' largest scale, one FP64 add per bin
@@ -460,7 +449,7 @@ namespace rg {
           for (int w = 0; w < kFinWarps; ++w) {
             const int    down = top - wscale[w];
             const float  f    = down > 126 ? 0.0f : __uint_as_float(static_cast<uint32_t>(127 - down) << 23);
-            const float2 a    = sums[w * kSliceBins + i];
+            const float2 a    = sums[w * groups + i];
             t                 = ff_add(t, ff { a.x * f, a.y * f });
           }
           if (t.hi != 0.0f) {
@@ -758,6 +747,26 @@ namespace rg {
 
   namespace {
 
+    // Blocks per (segment, slice): those with which the waves of `resident` blocks take the fewest rows
+    // of a warp, a block's setup and epilogue counted as kFinSetup rows (256 spectra: 5 blocks each,
+    // 124 us; counted as 6, 3 blocks: 138 us).
+    constexpr size_t kFinSmSmem = 227 * 1024;
+    constexpr int    kFinSetup  = 1;
+    int finish_blocks(int rows, int cells, int resident) {
+      const int most = std::max(1, (cells + kFinWarps - 1) / kFinWarps);
+      int       best = 1;
+      int64_t   least = std::numeric_limits<int64_t>::max();
+      for (int gx = 1; gx <= most; ++gx) {
+        const int64_t waves = (static_cast<int64_t>(rows) * gx + resident - 1) / resident;
+        const int64_t cost  = waves * ((cells + kFinWarps * gx - 1) / (kFinWarps * gx) + kFinSetup);
+        if (cost < least) {
+          least = cost;
+          best  = gx;
+        }
+      }
+      return best;
+    }
+
     template <int C>
     int launch_finish(const MomentFinishParams& r, dim3 grid, size_t smem, cudaStream_t s) {
       static std::atomic<uint64_t> configured { 0 };
@@ -791,11 +800,10 @@ namespace rg {
     r.acc      = pl->d_msum;
     r.done     = reinterpret_cast<unsigned*>(pl->d_msum + pl->msum_cap * kSliceBins);
     r.out      = out;
-    // a row per warp for few spectra; with many, more rows per warp and about four blocks per SM
-    const int rows = nseg * pl->nslices;
-    const int gx   = std::max(1, std::min((max_cells(pl) + kFinWarps - 1) / kFinWarps, (4 * ctx->sms + rows - 1) / rows));
-    const int nv   = max_valid(pl);
-    const size_t smem = finish_smem(nv, r.nseg_tab);
+    const int    rows   = nseg * pl->nslices;
+    const int    nv     = max_valid(pl);
+    const size_t smem   = finish_smem(nv, r.nseg_tab);
+    const int    gx     = finish_blocks(rows, max_cells(pl), ctx->sms * std::max(1, static_cast<int>(kFinSmSmem / (smem + 1024))));
     const dim3   grid(gx, rows);
     int          st = RG_OK;
     switch ((nv + 1 + 31) / 32) {
