@@ -17,13 +17,13 @@
 // double-float Newton step of rsqrt rounded to float.
 //
 // Only what the call asks for is accumulated: sums for log-spaced bins, counts otherwise or where
-// they are asked for.  Sums of many particles over up to about 220 bins without counts
-// (lane_warps): every lane of a warp has its own copy of the bins in shared memory, [bin][lane],
-// so a particle is one conflict-free load, add and store.  Shared-memory atomics set the pace
-// of the other kernel, which serves the rest: integer ones run at one lane per clock and SM on
-// random bins, float ones as compare-and-swap loops.  FP32 sums are flushed to FP64 every
-// kFlushLane particles of a lane (or kFlushParticles of a block), then summed across blocks in
-// FP64 in a fixed order.
+// they are asked for.  Sums of many particles over up to about 320 bins without counts
+// (lane_warps): each of 16 lanes of a warp has its own copy of the bins in shared memory,
+// [bin][copy], and the warp's halves add one after the other, so a particle is one conflict-free
+// load, add and store.  Shared-memory atomics set the pace of the other kernel, which serves the
+// rest: integer ones run at one lane per clock and SM on random bins, float ones as compare-and-swap
+// loops.  FP32 sums are flushed to double-floats every kFlushLane particles of a lane (or
+// kFlushParticles of a block), and blocks are summed in FP64 in a fixed order.
 #include "pair_stage.cuh"
 #include "rg_common.cuh"
 #include "rg_internal.hpp"
@@ -47,7 +47,7 @@ namespace rg {
     // 3.3e7 particles; 16 copies were slower).
     constexpr int kSumCopies     = 4;
     constexpr int kHistMaxBins   = 4096;
-    constexpr int kFlushParticles = 4096; // per block between FP32 -> FP64 flushes
+    constexpr int kFlushParticles = 4096; // per block between flushes of the FP32 sums
     // Cells of the bin lookup: the finest cells of float bit patterns (bits >> shift)
     // such that [thr[1], the largest finite threshold] spans at most kMaxCells of them
     // (64 cells per octave for 200 log bins over five decades: at most one threshold
@@ -79,8 +79,10 @@ namespace rg {
     // threshold, so a cell with at most one threshold is one load.
     constexpr int kLaneCells   = 2048;
     constexpr int kLaneMaxWarps = 16;
-    constexpr int kLaneVectors = 4;    // groups of four particles in flight per thread (8: the same time)
-    constexpr int kFlushLane   = 1024; // particles per lane between flushes
+    constexpr int kLaneCopies  = 16;   // copies of the bins per warp, lane l adding into copy l mod kLaneCopies
+    constexpr int kLaneVectors = 4;    // groups of four particles in flight per thread
+    constexpr int kFlushLane   = 512; // particles per lane between flushes
+    constexpr uint32_t kLaneRow = sizeof(float) * kLaneCopies; // bytes of a bin's copies
     constexpr size_t kLaneSmem = 226 * 1024;
 
     struct HistParams {
@@ -98,7 +100,7 @@ namespace rg {
       int             cell_base;    // cell of thr[1]
       int             ncells;
       const uint2*    lcells;       // lane kernel: [lncells + 2]: below thr[1], the cells, above the last threshold:
-                                    // (128 x the bin of the cell's smallest float, next threshold's bits; bit 31 of
+                                    // (kLaneRow x the bin of the cell's smallest float, next threshold's bits; bit 31 of
                                     // the first: more than one threshold inside)
       int             lshift, lbase, lncells;
       unsigned long long* part_counts; // [grid][nbins], or null
@@ -151,6 +153,14 @@ namespace rg {
       return __frcp_rn(sqrtf(U)); // 0 -> inf, inf -> 0, NaN -> NaN
     }
 
+    // t + (hi, lo) in double-float: infinite and NaN sums (an energy of 0) stay what they are, with no
+    // low part.  The flushes below sum in this form because GB300 adds FP64 at 2 lanes a clock: with
+    // FP64 sums 3.3e7 particles took 360 us over 2000 bins (now 198) and 161 over 600 (now 133).
+    __device__ __forceinline__ ff sum_add(ff t, float hi, float lo) {
+      const ff s = two_sum(t.hi, hi);
+      return { s.hi, isfinite(s.hi) ? __fadd_rn(t.lo, __fadd_rn(s.lo, lo)) : 0.0f };
+    }
+
     template <bool kSum, bool kCount>
     __global__ void __launch_bounds__(kHistThreads)
       histogram_kernel(const __grid_constant__ HistParams p) {
@@ -160,12 +170,12 @@ namespace rg {
       unsigned* cnt     = reinterpret_cast<unsigned*>(thr + nb);
       constexpr int kC = kSumCopies;
       float*    sum32   = reinterpret_cast<float*>(cnt + nb); // [kC][nb]
-      double*   sum64   = reinterpret_cast<double*>(smem + (((2 + kC) * sizeof(float) * nb + 15) & ~size_t(15)));
-      uint16_t* start   = reinterpret_cast<uint16_t*>(sum64 + nb);
+      float2*   total   = reinterpret_cast<float2*>(smem + (((2 + kC) * sizeof(float) * nb + 15) & ~size_t(15)));
+      uint16_t* start   = reinterpret_cast<uint16_t*>(total + nb);
       for (int i = threadIdx.x; i < nb; i += blockDim.x) {
         thr[i]   = p.thr[i];
         cnt[i]   = 0u;
-        sum64[i] = 0.0;
+        total[i] = make_float2(0.0f, 0.0f);
       }
       for (int i = threadIdx.x; i < kC * nb; i += blockDim.x) {
         sum32[i] = 0.0f;
@@ -221,12 +231,13 @@ namespace rg {
         if (kSum) {
           __syncthreads();
           for (int i = threadIdx.x; i < nb; i += blockDim.x) {
-            double t = sum64[i];
+            ff t { total[i].x, total[i].y };
+#pragma unroll
             for (int c = 0; c < kC; ++c) {
-              t += static_cast<double>(sum32[c * nb + i]);
+              t                 = sum_add(t, sum32[c * nb + i], 0.0f);
               sum32[c * nb + i] = 0.0f;
             }
-            sum64[i] = t;
+            total[i] = make_float2(t.hi, t.lo);
           }
         }
         __syncthreads();
@@ -236,7 +247,7 @@ namespace rg {
           p.part_counts[static_cast<int64_t>(blockIdx.x) * nb + i] = cnt[i];
         }
         if (kSum) {
-          p.part_sums[static_cast<int64_t>(blockIdx.x) * nb + i] = sum64[i];
+          p.part_sums[static_cast<int64_t>(blockIdx.x) * nb + i] = static_cast<double>(total[i].x) + static_cast<double>(total[i].y);
         }
       }
     }
@@ -264,6 +275,24 @@ namespace rg {
       return fma2(mul2(r, set2(-0.5f)), e, r);
     }
 
+    // shared [k0] += v0, then [k1] += v1 (which may be the same bin) where `on`
+    __device__ __forceinline__ void add_pair(uint32_t k0, uint32_t k1, float v0, float v1, bool on) {
+      asm volatile("{\n"
+                   "  .reg .pred p, q;\n"
+                   "  .reg .f32 a, b;\n"
+                   "  setp.ne.u32 p, %4, 0;\n"
+                   "  setp.eq.u32 q, %0, %1;\n"
+                   "  @p ld.shared.f32 a, [%0];\n"
+                   "  @p ld.shared.f32 b, [%1];\n"
+                   "  add.rn.f32 a, a, %2;\n"
+                   "  selp.f32 b, a, b, q;\n"
+                   "  add.rn.f32 b, b, %3;\n"
+                   "  @p st.shared.f32 [%0], a;\n"
+                   "  @p st.shared.f32 [%1], b;\n"
+                   "}" ::"r"(k0), "r"(k1), "f"(v0), "f"(v1), "r"(static_cast<uint32_t>(on))
+                   : "memory");
+    }
+
     // Any particle's bin by stepping over all thresholds (energies of 0, infinity and NaN, and
     // cells with several thresholds).
     __device__ __noinline__ int bin_by_steps(float U, const HistParams& p, const float* thr, int g) {
@@ -278,44 +307,44 @@ namespace rg {
 
     // Shared memory of the lane kernel with `warps` warps.
     size_t lane_smem(int nb, int ncells, int warps) {
-      return (sizeof(double) + sizeof(float)) * nb + sizeof(uint2) * (ncells + 2) +
-             sizeof(float) * 32 * static_cast<size_t>(nb) * warps + 16;
+      return (sizeof(float2) + sizeof(float)) * nb + sizeof(uint2) * (ncells + 2) +
+             sizeof(float) * kLaneCopies * static_cast<size_t>(nb) * warps + 16;
     }
 
-    // Warps of the lane kernel, or 0 where the atomics are faster: with fewer than seven warps on
-    // an SM the loads' latency is not hidden, and clearing and summing the copies takes about as
-    // long as a few million particles.  Per call, sums of |u|^-1 over log bins, lanes against
-    // atomics: 3.3e7 particles x 50 bins 99 / 164 us, 150: 104 / 140, 200: 121 / 139, 220 (7 warps):
-    // 128 / 141, 250 (6 warps): 162 / 138, 380 (4): 209 / 144; 200 bins x 8e6: 54.5 / 58.3, 4e6: 43.2 / 43.3,
-    // 1e6: 35.7 / 28.8.  Counts stay with the integer atomics (200 bins: 109 / 81).
-    constexpr int     kLaneMinWarps     = 7;
-    constexpr int64_t kLaneMinParticles = 6000000;
+    // Warps of the lane kernel, or 0 where the atomics are faster: with fewer than ten warps on an SM
+    // latencies are not hidden, and clearing and summing the copies takes as long as a million
+    // particles.  Per call, sums of |u|^-1 over log bins, lanes against atomics: 3.3e7 particles x 25
+    // bins 97 / 185 us, 50: 92 / 155, 100: 94 / 139, 200: 89 / 128, 300 (10 warps): 114 / 128, 380
+    // (8 warps): 138 / 128; 200 bins x 8e6: 37.9 / 51.1, 3e6: 27.6 / 30.9, 1e6: 23.4 / 23.2.  Counts stay
+    // with the integer atomics (200 bins: 77).
+    constexpr int     kLaneMinWarps     = 10;
+    constexpr int64_t kLaneMinParticles = 2000000;
 
     int lane_warps(int64_t n, int nb, int ncells) {
       const size_t tables = lane_smem(nb, ncells, 0);
       if (n < kLaneMinParticles || tables >= kLaneSmem) {
         return 0;
       }
-      const size_t w = (kLaneSmem - tables) / (sizeof(float) * 32 * nb);
+      const size_t w = (kLaneSmem - tables) / (sizeof(float) * kLaneCopies * nb);
       return w < static_cast<size_t>(kLaneMinWarps) ? 0 : static_cast<int>(std::min<size_t>(w, kLaneMaxWarps));
     }
 
-    // What bounds it: latency.  200 bins leave room for 8 warps on an SM (copies: 25.6 KB each), 33
-    // instructions a particle at 27 % of the issue slots, 49 % of the DRAM rate: 103 us for
-    // 3.3e7 particles x 200 bins against 120 us with atomics.  Eight particles of a thread are in
-    // flight at once (four, one addition after the other: 119 us).
+    // What bounds it: latency.  200 bins leave room for 16 warps on an SM (copies: 12.8 KB each).  3.3e7
+    // particles x 200 bins with 1/|u|: 89 us a call (4.4 TB/s) against 128 us with atomics and 139 us with
+    // atomics and FP64 flushes.  A copy per lane leaves 8 warps: 121 us; two groups of four at a
+    // time spill: 123 us before the flushes were in double-floats, one group 103 us.
     __global__ void __launch_bounds__(32 * kLaneMaxWarps) histogram_lane_kernel(const __grid_constant__ HistParams p) {
       extern __shared__ __align__(16) unsigned char smem[];
       const int nb = p.nbins, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
-      double*   sum64 = reinterpret_cast<double*>(smem);
-      uint2*    cells = reinterpret_cast<uint2*>(sum64 + nb);
+      float2*   total = reinterpret_cast<float2*>(smem);
+      uint2*    cells = reinterpret_cast<uint2*>(total + nb);
       float*    thr   = reinterpret_cast<float*>(cells + p.lncells + 2);
       float*    copies = reinterpret_cast<float*>((reinterpret_cast<uintptr_t>(thr + nb) + 15) & ~uintptr_t(15));
-      const int per    = 32 * nb;
-      float*    mine   = copies + warp * per; // [nb][32]
+      const int per    = kLaneCopies * nb;
+      float*    mine   = copies + warp * per; // [nb][kLaneCopies]
       for (int i = threadIdx.x; i < nb; i += blockDim.x) {
         thr[i]   = p.thr[i];
-        sum64[i] = 0.0;
+        total[i] = make_float2(0.0f, 0.0f);
       }
       for (int i = threadIdx.x; i < p.lncells + 2; i += blockDim.x) {
         cells[i] = p.lcells[i];
@@ -327,7 +356,8 @@ namespace rg {
 
       // 2 N particles of a lane: the bins and values of all of them first, then the additions in
       // pairs (the two of a pair may share a bin).
-      const uint32_t copy0 = static_cast<uint32_t>(__cvta_generic_to_shared(mine + lane));
+      const uint32_t copy0 = static_cast<uint32_t>(__cvta_generic_to_shared(mine + (lane & (kLaneCopies - 1))));
+      const uint32_t upper = lane >> 4; // lanes l and l + 16 share a copy: the lower ones add first
       const uint32_t cell0 = static_cast<uint32_t>(__cvta_generic_to_shared(cells)) - 8u * static_cast<uint32_t>(p.lbase - 1);
       const int      cmin = p.lbase - 1, cmax = p.lbase + p.lncells;
       const bool     fourvel = p.fourvel != 0;
@@ -352,7 +382,7 @@ namespace rg {
             const uint32_t bits = __float_as_uint(u[h]);
             uint32_t       cx, cy;
             asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(cx), "=r"(cy) : "r"(cell0 + 8u * static_cast<uint32_t>(max(cmin, min(static_cast<int>(bits >> p.lshift), cmax)))));
-            k[h] = cx + (u[h] >= __uint_as_float(cy) ? 128u : 0u);
+            k[h] = copy0 + cx + (u[h] >= __uint_as_float(cy) ? kLaneRow : 0u);
             many |= cx;
             far = max(far, bits - kOrdinaryMin);
           }
@@ -368,28 +398,40 @@ namespace rg {
           for (int h = 0; h < 2 * N; ++h) {
             const uint32_t bits = __float_as_uint(u[h]);
             const int      ci   = max(cmin, min(static_cast<int>(bits >> p.lshift), cmax)) - cmin;
-            k[h] = 128u * static_cast<uint32_t>(bin_by_steps(u[h], p, thr, static_cast<int>((cells[ci].x & 0x7fffffffu) >> 7)));
+            k[h] = copy0 + kLaneRow * static_cast<uint32_t>(bin_by_steps(u[h], p, thr, static_cast<int>((cells[ci].x & 0x7fffffffu) / kLaneRow)));
             v[h] = inverse_energy(u[h], p.fourvel);
           }
         }
 #pragma unroll
-        for (int j = 0; j < N; ++j) {
-          const uint32_t k0 = k[2 * j], k1 = k[2 * j + 1];
-          float a, b;
-          asm volatile("ld.shared.f32 %0, [%1];" : "=f"(a) : "r"(copy0 + k0) : "memory");
-          asm volatile("ld.shared.f32 %0, [%1];" : "=f"(b) : "r"(copy0 + k1) : "memory");
-          a = __fadd_rn(a, v[2 * j]);
-          b = __fadd_rn(k0 == k1 ? a : b, v[2 * j + 1]);
-          asm volatile("st.shared.f32 [%0], %1;" ::"r"(copy0 + k0), "f"(a) : "memory");
-          asm volatile("st.shared.f32 [%0], %1;" ::"r"(copy0 + k1), "f"(b) : "memory");
+        for (uint32_t half = 0; half < 2; ++half) {
+#pragma unroll
+          for (int j = 0; j < N; ++j) {
+            add_pair(k[2 * j], k[2 * j + 1], v[2 * j], v[2 * j + 1], upper == half);
+          }
+          __syncwarp();
         }
       };
-      auto add_one = [&](float x, float y, float z) {
-        const float U = __fadd_rn(__fadd_rn(__fmul_rn(x, x), __fmul_rn(y, y)), __fmul_rn(z, z));
-        const int   k = bin_by_steps(U, p, thr, static_cast<int>((cells[max(cmin, min(static_cast<int>(__float_as_uint(U) >> p.lshift), cmax)) - cmin].x & 0x7fffffffu) >> 7));
-        mine[k * 32 + lane] += inverse_energy(U, p.fourvel);
+      auto add_one = [&](bool live, float x, float y, float z) {
+        uint32_t at = copy0;
+        float    v  = 0.0f;
+        if (live) {
+          const float U  = __fadd_rn(__fadd_rn(__fmul_rn(x, x), __fmul_rn(y, y)), __fmul_rn(z, z));
+          const int   ci = max(cmin, min(static_cast<int>(__float_as_uint(U) >> p.lshift), cmax)) - cmin;
+          at = copy0 + kLaneRow * static_cast<uint32_t>(bin_by_steps(U, p, thr, static_cast<int>((cells[ci].x & 0x7fffffffu) / kLaneRow)));
+          v  = inverse_energy(U, p.fourvel);
+        }
+        __syncwarp();
+#pragma unroll
+        for (uint32_t half = 0; half < 2; ++half) {
+          if (live && upper == half) {
+            float a;
+            asm volatile("ld.shared.f32 %0, [%1];" : "=f"(a) : "r"(at) : "memory");
+            asm volatile("st.shared.f32 [%0], %1;" ::"r"(at), "f"(__fadd_rn(a, v)) : "memory");
+          }
+          __syncwarp();
+        }
       };
-      // The lanes' copies into the block's totals: a thread sums the 32 copies of its bins in four
+      // The lanes' copies into the block's totals: a thread sums the copies of its bins in four
       // chains (starting at a different lane per bin, so that a warp's reads hit different banks),
       // then the warps'.
       auto flush = [&]() {
@@ -401,40 +443,40 @@ namespace rg {
             t[c] = ff { 0.0f, 0.0f };
           }
 #pragma unroll 2
-          for (int l = 0; l < 32; l += 4) {
+          for (int l = 0; l < kLaneCopies; l += 4) {
 #pragma unroll
             for (int c = 0; c < 4; ++c) {
-              const int   at = b * 32 + ((l + c + b) & 31);
-              const float x  = mine[at];
-              const ff    s  = two_sum(t[c].hi, x);
-              // an infinite sum (an energy of 0) or NaN stays what it is: its remainder is NaN
-              t[c]     = ff { s.hi, isfinite(s.hi) ? __fadd_rn(t[c].lo, s.lo) : 0.0f };
-              mine[at] = 0.0f;
+              const int at = b * kLaneCopies + ((l + c + b) & (kLaneCopies - 1));
+              t[c]         = sum_add(t[c], mine[at], 0.0f);
+              mine[at]     = 0.0f;
             }
           }
 #pragma unroll
           for (int c = 0; c < 4; ++c) {
-            mine[b * 32 + 2 * c]     = t[c].hi;
-            mine[b * 32 + 2 * c + 1] = t[c].lo;
+            mine[b * kLaneCopies + 2 * c]     = t[c].hi;
+            mine[b * kLaneCopies + 2 * c + 1] = t[c].lo;
           }
         }
         __syncthreads();
         // four threads a bin sum the warps' pairs of one chain each
         for (int i = threadIdx.x; i < ((4 * nb + 31) & ~31); i += blockDim.x) {
           const int b = i >> 2, c = i & 3;
-          double    t = 0.0;
+          ff        t { 0.0f, 0.0f };
           if (b < nb) {
             for (int w = 0; w < warps; ++w) {
-              float* m = copies + w * per + b * 32 + 2 * c;
-              t += static_cast<double>(m[0]) + static_cast<double>(m[1]);
-              m[0] = 0.0f;
-              m[1] = 0.0f;
+              float* m = copies + w * per + b * kLaneCopies + 2 * c;
+              t        = sum_add(t, m[0], m[1]);
+              m[0]     = 0.0f;
+              m[1]     = 0.0f;
             }
           }
-          t += __shfl_xor_sync(0xffffffffu, t, 1);
-          t += __shfl_xor_sync(0xffffffffu, t, 2);
+#pragma unroll
+          for (int o = 1; o < 4; o <<= 1) {
+            t = sum_add(t, __shfl_xor_sync(0xffffffffu, t.hi, o), __shfl_xor_sync(0xffffffffu, t.lo, o));
+          }
           if (b < nb && c == 0) {
-            sum64[b] += t;
+            t        = sum_add(t, total[b].x, total[b].y);
+            total[b] = make_float2(t.hi, t.lo);
           }
         }
         __syncthreads();
@@ -449,8 +491,7 @@ namespace rg {
       if (vec_ok) {
         const int64_t nv = p.n / 4;
         done             = nv * 4;
-        // kLaneVectors groups in flight, taken two at a time: their registers are loaded again as
-        // soon as the two are added
+        // kLaneVectors groups in flight: a group's registers are loaded again as soon as it is added
         float4 X[kLaneVectors], Y[kLaneVectors], Z[kLaneVectors];
         auto   load = [&](int k, int64_t v) {
           if (v < nv) {
@@ -465,18 +506,21 @@ namespace rg {
         }
         for (int64_t v0 = 0; v0 < nv; v0 += kLaneVectors * T) { // uniform over the grid
 #pragma unroll
-          for (int k = 0; k < kLaneVectors; k += 2) {
+          for (int k = 0; k < kLaneVectors; ++k) {
             const int64_t v    = v0 + k * T + t;
-            const f2      x[4] = { pack2(X[k].x, X[k].y), pack2(X[k].z, X[k].w), pack2(X[k + 1].x, X[k + 1].y), pack2(X[k + 1].z, X[k + 1].w) };
-            const f2      y[4] = { pack2(Y[k].x, Y[k].y), pack2(Y[k].z, Y[k].w), pack2(Y[k + 1].x, Y[k + 1].y), pack2(Y[k + 1].z, Y[k + 1].w) };
-            const f2      z[4] = { pack2(Z[k].x, Z[k].y), pack2(Z[k].z, Z[k].w), pack2(Z[k + 1].x, Z[k + 1].y), pack2(Z[k + 1].z, Z[k + 1].w) };
-            if (v + T < nv) {
-              add(x, y, z, std::integral_constant<int, 4> {});
-            } else if (v < nv) {
+            const f2      x[2] = { pack2(X[k].x, X[k].y), pack2(X[k].z, X[k].w) };
+            const f2      y[2] = { pack2(Y[k].x, Y[k].y), pack2(Y[k].z, Y[k].w) };
+            const f2      z[2] = { pack2(Z[k].x, Z[k].y), pack2(Z[k].z, Z[k].w) };
+            if (v - lane + 31 < nv) { // the whole warp has a group
               add(x, y, z, std::integral_constant<int, 2> {});
+            } else {
+#pragma unroll 1
+              for (int i = 0; i < 4; ++i) {
+                const int64_t g = 4 * v + i;
+                add_one(v < nv, v < nv ? p.ux[g] : 0.0f, v < nv ? p.uy[g] : 0.0f, v < nv ? p.uz[g] : 0.0f);
+              }
             }
             load(k, v + kLaneVectors * T);
-            load(k + 1, v + (kLaneVectors + 1) * T);
           }
           since += 4 * kLaneVectors;
           if (since >= kFlushLane) {
@@ -486,10 +530,9 @@ namespace rg {
         }
       }
       for (int64_t i0 = done; i0 < p.n; i0 += T) { // uniform over the grid
-        const int64_t i = i0 + t;
-        if (i < p.n) {
-          add_one(p.ux[i], p.uy[i], p.uz[i]);
-        }
+        const int64_t i    = i0 + t;
+        const bool    live = i < p.n;
+        add_one(live, live ? p.ux[i] : 0.0f, live ? p.uy[i] : 0.0f, live ? p.uz[i] : 0.0f);
         if (++since >= kFlushLane) {
           flush();
           since = 0;
@@ -497,7 +540,7 @@ namespace rg {
       }
       flush();
       for (int b = threadIdx.x; b < nb; b += blockDim.x) {
-        p.part_sums[static_cast<int64_t>(blockIdx.x) * nb + b] = sum64[b];
+        p.part_sums[static_cast<int64_t>(blockIdx.x) * nb + b] = static_cast<double>(total[b].x) + static_cast<double>(total[b].y);
       }
     }
 
@@ -668,9 +711,9 @@ namespace rg {
         }
         const uint64_t next = static_cast<uint64_t>(first) + (uint64_t(1) << e.lshift);
         const bool     many = k + 1 <= fin && float_bits(e.thr[k + 1]) < next;
-        e.lcells[i] = make_uint2(128u * static_cast<uint32_t>(k - 1) | (many ? 0x80000000u : 0u), k <= fin ? float_bits(e.thr[k]) : inf);
+        e.lcells[i] = make_uint2(kLaneRow * static_cast<uint32_t>(k - 1) | (many ? 0x80000000u : 0u), k <= fin ? float_bits(e.thr[k]) : inf);
       }
-      e.lcells[e.lncells + 1] = make_uint2(128u * static_cast<uint32_t>(fin), inf);
+      e.lcells[e.lncells + 1] = make_uint2(kLaneRow * static_cast<uint32_t>(fin), inf);
     }
 
     constexpr std::size_t kThrCacheEntries = 16;
@@ -836,7 +879,7 @@ int rg_energy_distribution(const float* ux, const float* uy, const float* uz, in
     smem = rg::lane_smem(nbins, db.lncells, warps);
     G    = ctx->sms * std::max(1, std::min(static_cast<int>(rg::kLaneSmem / smem), 2048 / (32 * rg::kLaneMaxWarps)));
   } else {
-    smem = (((2 + rg::kSumCopies) * sizeof(float) * nbins + 15) & ~size_t(15)) + sizeof(double) * nbins +
+    smem = (((2 + rg::kSumCopies) * sizeof(float) * nbins + 15) & ~size_t(15)) + sizeof(float2) * nbins +
            sizeof(uint16_t) * (db.ncells + 1);
     if (smem > 48 * 1024) {
       RG_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
