@@ -1,7 +1,6 @@
-// Device pieces of the moment spectra (moments.cu, moments_smooth.cu): the particle
-// stage with a finer 64-bit table coordinate and the FP64 operands of the moment
-// atomics, built with integer instructions (GB300 issues FP64 arithmetic and 64-bit
-// conversions at a small fraction of the FP32 rate).
+// Device pieces of the moment spectra (moments.cu, moments_smooth.cu): the scalar particle
+// stage with a finer 64-bit table coordinate, which the packed one (pair_stage.cuh) leaves its
+// exceptional particles to, and the logarithm it shares with the IC pairs (ic.cu).
 #pragma once
 
 #include "spectrum_common.cuh"
@@ -49,11 +48,8 @@ namespace rg {
     return o;
   }
 
-  // GB300 issues FP64 arithmetic and 64-bit conversions at a small fraction of the FP32
-  // rate, so the deposit builds its FP64 values and 64-bit integers with integer
-  // instructions only.
-
-  // round(x) as a 64-bit integer for a finite float x with |x| < 2^62.
+  // round(x) as a 64-bit integer for a finite float x with |x| < 2^62, by integer instructions
+  // (GB300 converts to 64 bits at a small fraction of the FP32 rate).
   __device__ __forceinline__ int64_t float_to_ll_rn(float x) {
     if (fabsf(x) < 4194304.0f) { // |x| < 2^22: round through the 1.5 2^23 shifter
       return static_cast<int64_t>(__float_as_int(__fadd_rn(x, 12582912.0f)) - 0x4B400000);
@@ -68,15 +64,6 @@ namespace rg {
       v = static_cast<int64_t>((m + 1) >> 1);
     }
     return (b >> 31) ? -v : v;
-  }
-
-  // The double equal to a float of normal magnitude (either sign), from its bits.
-  __device__ __forceinline__ double float_to_double_bits(float a) {
-    const uint32_t b = __float_as_uint(a);
-    const uint64_t d = (static_cast<uint64_t>(b >> 31) << 63) |
-                       (static_cast<uint64_t>(((b >> 23) & 0xffu) + 896u) << 52) |
-                       (static_cast<uint64_t>(b & 0x7fffffu) << 29);
-    return __longlong_as_double(static_cast<long long>(d));
   }
 
   // G = 1 + u^2 and W = |u x B|^2 (no E field) as double-floats (relative error ~2^-46; a

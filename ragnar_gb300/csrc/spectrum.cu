@@ -745,7 +745,7 @@ namespace rg {
       if (pl->hist_cap != cap || pl->msum_cap != sums) {
         RG_CUDA_TRY(cudaStreamSynchronize(nullptr)); // zeroed before any stream's run
       }
-      // the smooth moment path's per-cell scratch (folded moments, adjoint cubics)
+      // the smooth moment path's per-cell scratch (the adjoint's cubics)
       if (pl->aligned) {
         RG_TRY(smooth_reserve_cells(pl, static_cast<size_t>(max_seg) * pl->sm_cells));
       }
