@@ -100,7 +100,7 @@ namespace rg {
 
       int seg_hint = 0;
       if (tid == 0) {
-        info[0] = item_info(p, it_begin, seg_hint);
+        info[0] = item_info(p, p.chunk, it_begin, seg_hint);
         if (p.use_tma) {
           issue_stage(p, info[0], stage, &mbar[0]);
         }
@@ -110,7 +110,7 @@ namespace rg {
       for (int64_t i = it_begin, it = 0; i < it_end; ++i, ++it) {
         const int st = static_cast<int>(it & 1);
         if (tid == 0 && i + 1 < it_end) {
-          info[st ^ 1] = item_info(p, i + 1, seg_hint);
+          info[st ^ 1] = item_info(p, p.chunk, i + 1, seg_hint);
           if (p.use_tma) {
             fence_proxy_async_smem();
             issue_stage(p, info[st ^ 1], stage + (st ^ 1) * stage_floats, &mbar[st ^ 1]);

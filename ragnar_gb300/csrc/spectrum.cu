@@ -55,41 +55,56 @@ namespace rg {
   namespace {
 
     // Rows of 32 bins combined per pass of flush_block: the pass's scratch, kFlushRows x
-    // kWarps x 32 double-floats, is the 8 KB of the two (q, A) buffers.
+    // kWarps x 32 doubles, is the 8 KB of the two (q, A) buffers.
     constexpr int kFlushRows = 4;
-    static_assert(kFlushRows * kWarps * 32 * sizeof(float2) <= 2 * kChunk * sizeof(int2),
+    static_assert(kFlushRows * kWarps * 32 * sizeof(double) <= 2 * kChunk * sizeof(int2),
                   "flush scratch must fit the (q, A) buffers");
 
     // Sums the warps' double-float accumulators of one segment in warp order and writes the
     // block's partial row; the accumulators are cleared.  Called by the whole block at a point
-    // where no warp reads the (q, A) buffers that serve as scratch.  The warps are summed in
-    // double-floats and only the row's value is FP64: GB300 adds FP64 at 2 lanes a clock, and one FP64
-    // value per warp and bin took 3 to 7 us a block (one distribution of 5e3 nodes 25.0 -> 18.8 us).
-    // The loop over warps is not unrolled: unrolled, it costs the kernel's main loop 3 %.
-    template <int K>
-    __device__ __forceinline__ void flush_block(float (&hi)[K], float (&lo)[K], float2* scratch, double* dst,
+    // where no warp reads the (q, A) buffers that serve as scratch.  GB300 adds FP64 at 2 lanes a
+    // clock, so one FP64 value per warp and bin takes 3 to 7 us a block: kShort sums the warps in
+    // double-floats and forms one FP64 value per bin (a distribution of 5e3 nodes 25.0 -> 18.8 us).
+    // Longer runs keep the FP64 sums, which do not show there, while the code of the other costs the
+    // kernel's main loop registers (8e6 particles x 512 bins: 1.137 against 1.208 ms).
+    template <int K, bool kShort>
+    __device__ __forceinline__ void flush_block(float (&hi)[K], float (&lo)[K], double* scratch, double* dst,
                                                 int tid, bool accumulate) {
       const int lane = tid & 31, warp = tid >> 5;
+      float2*   pairs = reinterpret_cast<float2*>(scratch);
 #pragma unroll
       for (int k0 = 0; k0 < K; k0 += kFlushRows) {
 #pragma unroll
         for (int r = 0; r < kFlushRows; ++r) {
           if (k0 + r < K) {
-            scratch[(r * kWarps + warp) * 32 + lane] = make_float2(hi[k0 + r], lo[k0 + r]);
+            const int i = (r * kWarps + warp) * 32 + lane;
+            if (kShort) {
+              pairs[i] = make_float2(hi[k0 + r], lo[k0 + r]);
+            } else {
+              scratch[i] = static_cast<double>(hi[k0 + r]) + static_cast<double>(lo[k0 + r]);
+            }
           }
         }
         __syncthreads();
         const int r = tid >> 5;
         if (r < kFlushRows && k0 + r < K) {
-          ff t { 0.0f, 0.0f };
-#pragma unroll 1
-          for (int w = 0; w < kWarps; ++w) {
-            const float2 v = scratch[(r * kWarps + w) * 32 + lane];
-            t              = ff_add(t, ff { v.x, v.y });
+          double t = 0.0;
+          if (kShort) {
+            ff sum { 0.0f, 0.0f };
+#pragma unroll
+            for (int w = 0; w < kWarps; ++w) {
+              const float2 v = pairs[(r * kWarps + w) * 32 + lane];
+              sum            = ff_add(sum, ff { v.x, v.y });
+            }
+            t = static_cast<double>(sum.hi) + static_cast<double>(sum.lo);
+          } else {
+#pragma unroll
+            for (int w = 0; w < kWarps; ++w) {
+              t += scratch[(r * kWarps + w) * 32 + lane];
+            }
           }
-          const double v = static_cast<double>(t.hi) + static_cast<double>(t.lo);
-          double*      d = dst + (k0 + r) * 32 + lane;
-          *d             = accumulate ? *d + v : v;
+          double* d = dst + (k0 + r) * 32 + lane;
+          *d        = accumulate ? *d + t : t;
         }
         __syncthreads();
       }
@@ -100,7 +115,7 @@ namespace rg {
       }
     }
 
-    template <int K, int MODE>
+    template <int K, int MODE, bool kShort>
     __global__ void __launch_bounds__(kThreads, kBlocksPerSM)
       fused_spectrum_kernel(const __grid_constant__ FusedParams p) {
       extern __shared__ __align__(128) unsigned char smem[];
@@ -114,9 +129,9 @@ namespace rg {
       __shared__ ItemInfo info[2];
 
       const int     tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-      const int     slice    = blockIdx.y;
+      const int     slice    = blockIdx.y, chunk = kShort ? p.chunk : kChunk;
       const int     G        = gridDim.x, b = blockIdx.x;
-      const int64_t n_items  = total_items(p.item_prefix, p.nseg, p.n_single, p.chunk);
+      const int64_t n_items  = total_items(p.item_prefix, p.nseg, p.n_single, chunk);
       const int64_t it_begin = static_cast<int64_t>(b) * n_items / G;
       const int64_t it_end   = static_cast<int64_t>(b + 1) * n_items / G;
       if (it_begin >= it_end) {
@@ -155,7 +170,7 @@ namespace rg {
 
       int seg_hint = 0;
       if (tid == 0) {
-        info[0] = item_info(p, it_begin, seg_hint);
+        info[0] = item_info(p, chunk, it_begin, seg_hint);
         if (p.use_tma) {
           issue_stage(p, info[0], stage, &mbar[0]);
         }
@@ -173,7 +188,7 @@ namespace rg {
       for (int64_t i = it_begin, it = 0; i < it_end; ++i, ++it) {
         const int st = static_cast<int>(it & 1);
         if (tid == 0 && i + 1 < it_end) {
-          info[st ^ 1] = item_info(p, i + 1, seg_hint);
+          info[st ^ 1] = item_info(p, chunk, i + 1, seg_hint);
           if (p.use_tma) {
             fence_proxy_async_smem();
             issue_stage(p, info[st ^ 1], stage + (st ^ 1) * stage_floats, &mbar[st ^ 1]);
@@ -198,7 +213,7 @@ namespace rg {
           // block-uniform (info[st] is shared); every warp is past the previous item's
           // evaluation (the barrier above), so the (q, A) buffers are free
           if (cur_seg >= 0) {
-            flush_block<K>(hi, lo, reinterpret_cast<float2*>(qa), block_partial(p, b, cur_seg, slice), tid,
+            flush_block<K, kShort>(hi, lo, reinterpret_cast<double*>(qa), block_partial(p, b, cur_seg, slice), tid,
                            p.accumulate != 0);
           }
           cur_seg = I.seg;
@@ -258,7 +273,7 @@ namespace rg {
       }
       if (cur_seg >= 0) {
         __syncthreads(); // every warp is done reading the last item's (q, A)
-        flush_block<K>(hi, lo, reinterpret_cast<float2*>(qa), block_partial(p, b, cur_seg, slice), tid,
+        flush_block<K, kShort>(hi, lo, reinterpret_cast<double*>(qa), block_partial(p, b, cur_seg, slice), tid,
                        p.accumulate != 0);
       }
     }
@@ -537,21 +552,28 @@ namespace rg {
     }
 
     // Sets the kernel's shared-memory limit once per device (which also loads it).
-    template <int K, int MODE>
+    template <int K, int MODE, bool kShort>
     cudaError_t configure_fused_k() {
       static std::atomic<uint64_t> configured { 0 };
-      return ensure_max_dynamic_smem(fused_spectrum_kernel<K, MODE>,
+      return ensure_max_dynamic_smem(fused_spectrum_kernel<K, MODE, kShort>,
                                      static_cast<int>(fused_smem(MODE, kSmoothMaxSegments, kComps)), configured);
     }
 
-    template <int K, int MODE>
-    cudaError_t launch_fused_k(const FusedParams& fp, dim3 grid, size_t smem, cudaStream_t s) {
-      const cudaError_t e = configure_fused_k<K, MODE>();
+    template <int K, int MODE, bool kShort>
+    cudaError_t launch_fused_as(const FusedParams& fp, dim3 grid, size_t smem, cudaStream_t s) {
+      const cudaError_t e = configure_fused_k<K, MODE, kShort>();
       if (e != cudaSuccess) {
         return e;
       }
-      fused_spectrum_kernel<K, MODE><<<grid, kThreads, smem, s>>>(fp);
+      fused_spectrum_kernel<K, MODE, kShort><<<grid, kThreads, smem, s>>>(fp);
       return cudaGetLastError();
+    }
+
+    // The short form where a block has one item of less than kChunk particles (item_size).
+    template <int K, int MODE>
+    cudaError_t launch_fused_k(const FusedParams& fp, dim3 grid, size_t smem, cudaStream_t s) {
+      return fp.chunk < kChunk ? launch_fused_as<K, MODE, true>(fp, grid, smem, s)
+                               : launch_fused_as<K, MODE, false>(fp, grid, smem, s);
     }
 
     template <int MODE>
@@ -822,7 +844,9 @@ namespace rg {
   // current device, so that a later launch needs no module load (a load reserves device
   // memory for the code under CUDA's lazy loading).
   int preload_reference_kernels() {
-#define RG_K_LOAD(k) RG_CUDA_TRY((configure_fused_k<k, kModeRef>()));
+#define RG_K_LOAD(k)                                    \
+  RG_CUDA_TRY((configure_fused_k<k, kModeRef, false>())); \
+  RG_CUDA_TRY((configure_fused_k<k, kModeRef, true>()));
     RG_K_LOAD(1) RG_K_LOAD(2) RG_K_LOAD(3) RG_K_LOAD(4) RG_K_LOAD(5) RG_K_LOAD(6) RG_K_LOAD(7) RG_K_LOAD(8)
     RG_K_LOAD(9) RG_K_LOAD(10) RG_K_LOAD(11) RG_K_LOAD(12) RG_K_LOAD(13) RG_K_LOAD(14) RG_K_LOAD(15)
     RG_K_LOAD(16)

@@ -230,7 +230,7 @@ namespace rg {
     return static_cast<uint32_t>(Pmin - L);
   }
 
-  __device__ __forceinline__ ItemInfo item_info(const FusedParams& p, int64_t i, int& seg_hint) {
+  __device__ __forceinline__ ItemInfo item_info(const FusedParams& p, int chunk, int64_t i, int& seg_hint) {
     int s = seg_hint;
     while (s + 1 < p.nseg && items_before(p.item_prefix, s + 1) <= i) {
       ++s;
@@ -239,8 +239,8 @@ namespace rg {
     const int64_t c = i - items_before(p.item_prefix, s);
     ItemInfo      I;
     I.seg    = s;
-    I.pstart = seg_begin(p, s) + c * p.chunk;
-    I.pend   = min(I.pstart + p.chunk, seg_end(p, s));
+    I.pstart = seg_begin(p, s) + c * chunk;
+    I.pend   = min(I.pstart + chunk, seg_end(p, s));
     I.np     = static_cast<int>(I.pend - I.pstart);
     I.a0     = I.pstart & ~int64_t(3);
     I.a1     = I.pend & ~int64_t(3);
