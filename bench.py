@@ -17,7 +17,7 @@ rg_spectrum_run_host, H2D of the inputs and D2H of the spectra inside the timed
 region every step, steps pipelined; the step-synchronous figure and a copy-only /
 kernel-only breakdown beside it).  The plans sum by interval moments (the default
 for reference-table particle plans): one particle stage per particle deposits FP64
-moments per (table cell, bin interval), then a scan and a per-bin reduce; the
+moments per (table cell, bin interval), and a finish kernel sums them per bin; the
 roofline is that of the deposit kernel (HBM: 28 algorithmic bytes per particle).
 The fused per-eval kernel (every particle x bin pair in FP32) runs the same step
 as a side case with its FP32-issue roofline.  Also: per-species error of the
@@ -77,7 +77,7 @@ def parse_args():
                          "1024 gamma bins x 1024 photon bins, 4 tcgen05 GEMM launches; 'histogram' = "
                          "energyDistribution of 3.3e7 particles into 200 log bins, 4 calls; 'ic' = "
                          "ICSpectrum 1024 x 1024 x 1024, 4 calls; 'moments' = one 2^24-particle species "
-                         "x 512 bins by interval moments, 4 runs (deposit, scan, reduce); 'smooth' / "
+                         "x 512 bins by interval moments, 4 runs (deposit, finish); 'smooth' / "
                          "'smooth_moments' = the smooth table, 4 forward + 4 adjoint runs, fused kernels on "
                          "2^22 particles / cell moments on 2^24 particles")
     return ap.parse_args()
@@ -374,7 +374,7 @@ def run_ours(args, rank, world, local_rank):
         plan_p.run(prt_p, out_p, stream)
 
     evals_per_step = NSPECIES * n_per * NBINS
-    launches_per_step = 6  # deposit + scan + reduce, for the e+- batch and for the protons
+    launches_per_step = 4  # deposit + finish, for the e+- batch and for the protons
 
     for _ in range(max(args.warmup, 3)):
         step()
@@ -543,7 +543,7 @@ def run_ours(args, rank, world, local_rank):
         extra["fromdist_gemm_4096x1024x1024"] = guarded(fromdist_gemm_case, torch, capi, device, peak_bf16)
         extra["fromdist_gemm_4096x1024x1024"]["peak_source"] = peak_src
         extra["adam_fit_1024x512x512"] = guarded(adam_fit_case, torch, capi, device)
-        extra["ic_1024x1024x1024"] = guarded(ic_case, torch, capi, device, clocks.get("sm_mhz") or 2070.0)
+        extra["ic_1024x1024x1024"] = guarded(ic_case, torch, capi, device)
         add_wavefront_rooflines(extra, sms, clocks.get("sm_mhz") or 2070.0)
         fa = extra["fwd_adjoint_1e7x512"]
         if "moments" in fa:
@@ -1181,11 +1181,11 @@ def dropin_module_case(torch, comps, n, reps=3):
             "energyDistribution_ms": t_h * 1e3, "energyDistribution_particles_per_s": n / t_h}
 
 
-def ic_case(torch, capi, device, clk_mhz=2070.0):
+def ic_case(torch, capi, device):
     """ICSpectrum of a 1024-bin particle power law (index -2 on [1e2, 1e7], exp cutoff at
     3e6) on a 1024-bin soft-photon field (1e-9..1e-3 mec2, dN/dE ~ E^-1) into 1024 IC bins
-    1e-3..1e7: 1.07e9 (gamma, soft photon, IC bin) evals.  Bound: one MUFU lg2 per eval
-    (16 per SM per clock)."""
+    1e-3..1e7: the sum over 1.07e9 (gamma, soft photon, IC bin) triples, taken as 1.05e6
+    (gamma, IC bin) pairs over suffix sums of the photons."""
     import numpy as np  # noqa: PLC0415
 
     n = 1024
@@ -1203,12 +1203,9 @@ def ic_case(torch, capi, device, clk_mhz=2070.0):
                                              t[3].data_ptr(), n, t[4].data_ptr(), n, out.data_ptr(), stream))
 
     dt = timed(torch, run, 10)
-    sms = torch.cuda.get_device_properties(device).multi_processor_count
     evals = float(n) ** 3
-    peak = sms * 16 * clk_mhz * 1e6
     return {"gamma_bins": n, "soft_photon_bins": n, "ic_bins": n, "ms": dt * 1e3, "evals_per_s": evals / dt,
-            "mufu_peak_evals_per_s": peak, "frac_of_mufu_peak": evals / dt / peak,
-            "finite": bool(torch.isfinite(out).all())}
+            "pairs_per_s": float(n) ** 2 / dt, "finite": bool(torch.isfinite(out).all())}
 
 
 def histogram_case(torch, capi, device, comps, n, reps=10):
@@ -1256,7 +1253,7 @@ def profile_case():
 
 
 def profile_case_moments():
-    """4 runs of the interval-moment path (deposit, scan, reduce) on 2^24 particles of
+    """4 runs of the interval-moment path (deposit, finish) on 2^24 particles of
     the dump-scale e- species x 512 bins (inputs 470 MB, above the L2)."""
     import torch  # noqa: PLC0415
 

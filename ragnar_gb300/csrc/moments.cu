@@ -123,7 +123,7 @@ namespace rg {
     // that are not given read a constant with a stride of 0, so the loads carry no tests.
     // Measured on 9.9e7 dump particles x 512 bins: 0.88 ms in two launches (1.13e11 particles/s,
     // 3.2 TB/s) against 1.45 ms for one particle per thread with scalar double-floats, 444
-    // instructions a particle and two reduction requests; now 185 and one.  Without the
+    // instructions a particle and two reduction requests; now 171 and one.  Without the
     // reductions it would take 0.65 ms, the reductions alone 0.69 ms: the L2's reduction requests
     // and the loads behind them set its pace.  Also measured: three blocks per SM 0.95 ms, loads
     // staged through shared memory by cp.async 0.93 ms, entries scattered over the table no gain.
