@@ -90,8 +90,8 @@ namespace rg {
   // Particles per work item of one segment of n particles: kChunk where that gives every block an
   // item, fewer for smaller sets, so that they use the whole chip (a multiple of 4 for the
   // 16-byte staging).  One distribution on 512 bins, with the flush in double-floats: 1e3 nodes 28.9 ->
-  // 18.7 us, 5e3 29.0 -> 18.8, 5e4 31.1 -> 27.0, 155e3 43.3 -> 39.3; particles on 200 bins: 1e3
-  // 22.9 -> 16.7 us, 1e5 33.2 -> 29.0.  (Half as many blocks: 155e3 nodes 43.3 us.)
+  // 18.7 us, 5e3 29.0 -> 18.8, 5e4 31.1 -> 25.1; particles on 200 bins: 1e3
+  // 22.9 -> 16.7 us, 1e5 33.2 -> 29.0.
   inline int item_size(int64_t n, int blocks) {
     const int64_t each = (n + blocks - 1) / blocks;
     return static_cast<int>(each >= kChunk ? kChunk : each <= kChunkMin ? kChunkMin : (each + 3) & ~int64_t(3));
