@@ -76,7 +76,7 @@ namespace rg {
     }
 
     // The lane kernel's cells are coarser (its table has 8 bytes a cell) and carry their first
-    // threshold, so a cell with at most one threshold is one load.
+    // threshold: each holds one at most, so a lookup is one load and one comparison.
     constexpr int kLaneCells   = 2048;
     constexpr int kLaneMaxWarps = 16;
     constexpr int kLaneCopies  = 16;   // copies of the bins per warp, lane l adding into copy l mod kLaneCopies
@@ -100,8 +100,7 @@ namespace rg {
       int             cell_base;    // cell of thr[1]
       int             ncells;
       const uint2*    lcells;       // lane kernel: [lncells + 2]: below thr[1], the cells, above the last threshold:
-                                    // (kLaneRow x the bin of the cell's smallest float, next threshold's bits; bit 31 of
-                                    // the first: more than one threshold inside)
+                                    // (kLaneRow x the bin of the cell's smallest float, next threshold's bits)
       int             lshift, lbase, lncells;
       unsigned long long* part_counts; // [grid][nbins], or null
       double*         part_sums;       // [grid][nbins], or null
@@ -293,8 +292,7 @@ namespace rg {
                    : "memory");
     }
 
-    // Any particle's bin by stepping over all thresholds (energies of 0, infinity and NaN, and
-    // cells with several thresholds).
+    // Any particle's bin by stepping over the thresholds from g (energies of 0, infinity and NaN).
     __device__ __noinline__ int bin_by_steps(float U, const HistParams& p, const float* thr, int g) {
       if (U != U) {
         return p.nan_index;
@@ -316,13 +314,16 @@ namespace rg {
     // particles.  Per call, sums of |u|^-1 over log bins, lanes against atomics: 3.3e7 particles x 25
     // bins 97 / 185 us, 50: 92 / 155, 100: 94 / 139, 200: 89 / 128, 300 (10 warps): 114 / 128, 380
     // (8 warps): 138 / 128; 200 bins x 8e6: 37.9 / 51.1, 3e6: 27.6 / 30.9, 1e6: 23.4 / 23.2.  Counts stay
-    // with the integer atomics (200 bins: 77).
+    // with the integer atomics (200 bins: 77); streams off a 16-byte boundary,
+    // and bins so uneven that a cell holds several thresholds, go to the atomics kernel too.
     constexpr int     kLaneMinWarps     = 10;
     constexpr int64_t kLaneMinParticles = 2000000;
 
-    int lane_warps(int64_t n, int nb, int ncells) {
+    int lane_warps(const float* ux, const float* uy, const float* uz, int64_t n, int nb, int ncells) {
       const size_t tables = lane_smem(nb, ncells, 0);
-      if (n < kLaneMinParticles || tables >= kLaneSmem) {
+      const bool   aligned = ((reinterpret_cast<uintptr_t>(ux) | reinterpret_cast<uintptr_t>(uy) |
+                             reinterpret_cast<uintptr_t>(uz)) & 15) == 0;
+      if (!aligned || n < kLaneMinParticles || tables >= kLaneSmem) {
         return 0;
       }
       const size_t w = (kLaneSmem - tables) / (sizeof(float) * kLaneCopies * nb);
@@ -365,7 +366,7 @@ namespace rg {
         constexpr int N = decltype(count_tag)::value;
         float         u[2 * N], v[2 * N];
         uint32_t      k[2 * N];
-        uint32_t      many = 0u, far = 0u;
+        uint32_t      far = 0u;
 #pragma unroll
         for (int j = 0; j < N; ++j) {
           // single products: the compiler contracts a packed product and sum, whatever their rounding
@@ -383,7 +384,6 @@ namespace rg {
             uint32_t       cx, cy;
             asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(cx), "=r"(cy) : "r"(cell0 + 8u * static_cast<uint32_t>(max(cmin, min(static_cast<int>(bits >> p.lshift), cmax)))));
             k[h] = copy0 + cx + (u[h] >= __uint_as_float(cy) ? kLaneRow : 0u);
-            many |= cx;
             far = max(far, bits - kOrdinaryMin);
           }
           if (fourvel) { // inverse_energy of an ordinary U
@@ -393,12 +393,12 @@ namespace rg {
             unpack2(inv_sqrt_one_plus2(U), v[2 * j], v[2 * j + 1]);
           }
         }
-        if (static_cast<int>(many) < 0 || far >= kOrdinarySpan) {
+        if (far >= kOrdinarySpan) {
 #pragma unroll
           for (int h = 0; h < 2 * N; ++h) {
             const uint32_t bits = __float_as_uint(u[h]);
             const int      ci   = max(cmin, min(static_cast<int>(bits >> p.lshift), cmax)) - cmin;
-            k[h] = copy0 + kLaneRow * static_cast<uint32_t>(bin_by_steps(u[h], p, thr, static_cast<int>((cells[ci].x & 0x7fffffffu) / kLaneRow)));
+            k[h] = copy0 + kLaneRow * static_cast<uint32_t>(bin_by_steps(u[h], p, thr, static_cast<int>(cells[ci].x / kLaneRow)));
             v[h] = inverse_energy(u[h], p.fourvel);
           }
         }
@@ -417,7 +417,7 @@ namespace rg {
         if (live) {
           const float U  = __fadd_rn(__fadd_rn(__fmul_rn(x, x), __fmul_rn(y, y)), __fmul_rn(z, z));
           const int   ci = max(cmin, min(static_cast<int>(__float_as_uint(U) >> p.lshift), cmax)) - cmin;
-          at = copy0 + kLaneRow * static_cast<uint32_t>(bin_by_steps(U, p, thr, static_cast<int>((cells[ci].x & 0x7fffffffu) / kLaneRow)));
+          at = copy0 + kLaneRow * static_cast<uint32_t>(bin_by_steps(U, p, thr, static_cast<int>(cells[ci].x / kLaneRow)));
           v  = inverse_energy(U, p.fourvel);
         }
         __syncwarp();
@@ -484,59 +484,49 @@ namespace rg {
 
       const int64_t T = static_cast<int64_t>(gridDim.x) * blockDim.x;
       const int64_t t = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-      const bool    vec_ok = ((reinterpret_cast<uintptr_t>(p.ux) | reinterpret_cast<uintptr_t>(p.uy) |
-                            reinterpret_cast<uintptr_t>(p.uz)) & 15) == 0;
-      int           since = 0; // particles of a lane since the last flush (the same in every thread)
-      int64_t       done  = 0; // particles taken by the vector loop
-      if (vec_ok) {
-        const int64_t nv = p.n / 4;
-        done             = nv * 4;
-        // kLaneVectors groups in flight: a group's registers are loaded again as soon as it is added
-        float4 X[kLaneVectors], Y[kLaneVectors], Z[kLaneVectors];
-        auto   load = [&](int k, int64_t v) {
-          if (v < nv) {
-            X[k] = __ldcs(reinterpret_cast<const float4*>(p.ux) + v);
-            Y[k] = __ldcs(reinterpret_cast<const float4*>(p.uy) + v);
-            Z[k] = __ldcs(reinterpret_cast<const float4*>(p.uz) + v);
-          }
-        };
+      const int64_t nv = p.n / 4; // groups of four, loaded as 16 bytes (lane_warps asks for the alignment)
+      int           since = 0;    // particles of a lane since the last flush (the same in every thread)
+      // kLaneVectors groups in flight: a group's registers are loaded again as soon as it is added
+      float4 X[kLaneVectors], Y[kLaneVectors], Z[kLaneVectors];
+      auto   load = [&](int k, int64_t v) {
+        if (v < nv) {
+          X[k] = __ldcs(reinterpret_cast<const float4*>(p.ux) + v);
+          Y[k] = __ldcs(reinterpret_cast<const float4*>(p.uy) + v);
+          Z[k] = __ldcs(reinterpret_cast<const float4*>(p.uz) + v);
+        }
+      };
+#pragma unroll
+      for (int k = 0; k < kLaneVectors; ++k) {
+        load(k, k * T + t);
+      }
+      for (int64_t v0 = 0; v0 < nv; v0 += kLaneVectors * T) { // uniform over the grid
 #pragma unroll
         for (int k = 0; k < kLaneVectors; ++k) {
-          load(k, k * T + t);
-        }
-        for (int64_t v0 = 0; v0 < nv; v0 += kLaneVectors * T) { // uniform over the grid
-#pragma unroll
-          for (int k = 0; k < kLaneVectors; ++k) {
-            const int64_t v    = v0 + k * T + t;
-            const f2      x[2] = { pack2(X[k].x, X[k].y), pack2(X[k].z, X[k].w) };
-            const f2      y[2] = { pack2(Y[k].x, Y[k].y), pack2(Y[k].z, Y[k].w) };
-            const f2      z[2] = { pack2(Z[k].x, Z[k].y), pack2(Z[k].z, Z[k].w) };
-            if (v - lane + 31 < nv) { // the whole warp has a group
-              add(x, y, z, std::integral_constant<int, 2> {});
-            } else {
+          const int64_t v    = v0 + k * T + t;
+          const f2      x[2] = { pack2(X[k].x, X[k].y), pack2(X[k].z, X[k].w) };
+          const f2      y[2] = { pack2(Y[k].x, Y[k].y), pack2(Y[k].z, Y[k].w) };
+          const f2      z[2] = { pack2(Z[k].x, Z[k].y), pack2(Z[k].z, Z[k].w) };
+          if (v - lane + 31 < nv) { // the whole warp has a group
+            add(x, y, z, std::integral_constant<int, 2> {});
+          } else {
 #pragma unroll 1
-              for (int i = 0; i < 4; ++i) {
-                const int64_t g = 4 * v + i;
-                add_one(v < nv, v < nv ? p.ux[g] : 0.0f, v < nv ? p.uy[g] : 0.0f, v < nv ? p.uz[g] : 0.0f);
-              }
+            for (int i = 0; i < 4; ++i) {
+              const int64_t g = 4 * v + i;
+              add_one(v < nv, v < nv ? p.ux[g] : 0.0f, v < nv ? p.uy[g] : 0.0f, v < nv ? p.uz[g] : 0.0f);
             }
-            load(k, v + kLaneVectors * T);
           }
-          since += 4 * kLaneVectors;
-          if (since >= kFlushLane) {
-            flush();
-            since = 0;
-          }
+          load(k, v + kLaneVectors * T);
         }
-      }
-      for (int64_t i0 = done; i0 < p.n; i0 += T) { // uniform over the grid
-        const int64_t i    = i0 + t;
-        const bool    live = i < p.n;
-        add_one(live, live ? p.ux[i] : 0.0f, live ? p.uy[i] : 0.0f, live ? p.uz[i] : 0.0f);
-        if (++since >= kFlushLane) {
+        since += 4 * kLaneVectors;
+        if (since >= kFlushLane) {
           flush();
           since = 0;
         }
+      }
+      { // the remainder
+        const int64_t i    = 4 * nv + t;
+        const bool    live = i < p.n;
+        add_one(live, live ? p.ux[i] : 0.0f, live ? p.uy[i] : 0.0f, live ? p.uz[i] : 0.0f);
       }
       flush();
       for (int b = threadIdx.x; b < nb; b += blockDim.x) {
@@ -681,28 +671,32 @@ namespace rg {
       }
     }
 
-    // The lane kernel's cells over the same range (see HistParams::lcells).
+    // The lane kernel's cells from the first threshold above 0 to the last finite one (see
+    // HistParams::lcells); none, and no lane kernel, where a cell would hold several thresholds.
     void make_lane_cells(ThrEntry& e) {
       const int      n   = static_cast<int>(e.thr.size());
       const uint32_t inf = 0x7f800000u;
-      int            fin = 0; // thresholds thr[1..fin] are finite
+      int            zero = 0, fin = 0; // thresholds thr[1..zero] are 0, thr[1..fin] finite
       while (fin + 1 < n && std::isfinite(e.thr[fin + 1])) {
         ++fin;
+      }
+      while (zero < fin && e.thr[zero + 1] == 0.0f) {
+        ++zero;
       }
       e.lshift  = 0;
       e.lbase   = 0;
       e.lncells = 0;
-      if (fin == 0) { // no finite threshold: bin 0 for every finite energy
-        e.lcells.assign(2, make_uint2(0u, inf));
+      e.lcells.assign(2, make_uint2(kLaneRow * static_cast<uint32_t>(zero), inf));
+      if (fin == zero) { // no threshold above 0: one bin for every finite energy
         return;
       }
-      const uint32_t lo = float_bits(e.thr[1]), hi = float_bits(e.thr[fin]);
+      const uint32_t lo = float_bits(e.thr[zero + 1]), hi = float_bits(e.thr[fin]);
       while ((hi >> e.lshift) - (lo >> e.lshift) + 1 > static_cast<uint32_t>(kLaneCells)) {
         ++e.lshift;
       }
       e.lbase   = static_cast<int>(lo >> e.lshift);
       e.lncells = static_cast<int>((hi >> e.lshift) - (lo >> e.lshift) + 1);
-      e.lcells.assign(static_cast<std::size_t>(e.lncells) + 2, make_uint2(0u, inf));
+      e.lcells.resize(static_cast<std::size_t>(e.lncells) + 2);
       int k = 1; // thr[1..k-1] <= the current cell's smallest float
       for (int i = 1; i <= e.lncells; ++i) {
         const uint32_t first = static_cast<uint32_t>(e.lbase + i - 1) << e.lshift;
@@ -710,8 +704,11 @@ namespace rg {
           ++k;
         }
         const uint64_t next = static_cast<uint64_t>(first) + (uint64_t(1) << e.lshift);
-        const bool     many = k + 1 <= fin && float_bits(e.thr[k + 1]) < next;
-        e.lcells[i] = make_uint2(kLaneRow * static_cast<uint32_t>(k - 1) | (many ? 0x80000000u : 0u), k <= fin ? float_bits(e.thr[k]) : inf);
+        if (k + 1 <= fin && float_bits(e.thr[k + 1]) < next) {
+          e.lcells.clear();
+          return;
+        }
+        e.lcells[i] = make_uint2(kLaneRow * static_cast<uint32_t>(k - 1), k <= fin ? float_bits(e.thr[k]) : inf);
       }
       e.lcells[e.lncells + 1] = make_uint2(kLaneRow * static_cast<uint32_t>(fin), inf);
     }
@@ -807,8 +804,8 @@ namespace rg {
       }
       e.dev.emplace_back(device, p);
     }
-    out.lcells     = reinterpret_cast<const uint2*>(p);
-    out.thr        = reinterpret_cast<const float*>(out.lcells + e.lcells.size());
+    out.lcells     = e.lcells.empty() ? nullptr : reinterpret_cast<const uint2*>(p);
+    out.thr        = reinterpret_cast<const float*>(reinterpret_cast<const uint2*>(p) + e.lcells.size());
     out.start      = reinterpret_cast<const uint16_t*>(out.thr + n);
     out.lshift     = e.lshift;
     out.lbase      = e.lbase;
@@ -867,7 +864,7 @@ int rg_energy_distribution(const float* ux, const float* uy, const float* uz, in
   RG_TRY(rg::context(&ctx));
   // what is accumulated, and by which kernel
   const bool need_sum = log_spaced != 0, need_count = !need_sum || counts != nullptr;
-  const int  warps    = need_count ? 0 : rg::lane_warps(n, nbins, db.lncells);
+  const int  warps    = need_count || !db.lcells ? 0 : rg::lane_warps(ux, uy, uz, n, nbins, db.lncells);
   size_t     smem     = 0;
   int        G        = 0;
   auto       kernel   = !need_sum    ? rg::histogram_kernel<false, true>

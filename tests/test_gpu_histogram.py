@@ -209,7 +209,7 @@ def many():
 
 @pytest.mark.parametrize("n,offset", [(1, 0), (4099, 0), (200_001, 1), (6_000_003, 0), (6_000_000, 1)])
 @pytest.mark.parametrize("nb,log_spaced,fourvel", [(1, True, True), (33, True, False), (200, True, True), (220, True, False),
-                                                   (380, True, True), (200, False, True)])
+                                                   (300, True, False), (380, True, True), (200, False, True)])
 def test_without_counts(gpu, oracle_lib, many, n, offset, nb, log_spaced, fourvel):
     """The histogram alone (no counts asked for): per-lane copies of the bins for many particles and
     up to about 220 bins, atomics otherwise; groups of four and the remainder."""
