@@ -153,17 +153,25 @@ class _LogMse(torch.autograd.Function):
         return gS, None, None
 
 
+def _unwatched() -> bool:
+    """Nothing looks at the single operations: no function transform, dual level, tracer or mode.  What
+    tells is private to torch; where one of the names is gone, the answer is no."""
+    try:
+        return (torch._C._functorch.peek_interpreter_stack() is None
+                and torch.autograd.forward_ad._current_level < 0
+                and torch._C._len_torch_dispatch_stack() == 0
+                and torch._C._len_torch_function_stack() == 0
+                and not torch.jit.is_tracing() and not torch.compiler.is_compiling())
+    except (AttributeError, TypeError):
+        return False
+
+
 def _plain_cuda(*tensors) -> bool:
-    """Contiguous float32 tensors of the current CUDA device, and nothing that looks at the single
-    operations: no tensor subclass, function transform, dual level, tracer or mode."""
+    """Contiguous float32 tensors of the current CUDA device, no subclasses, and _unwatched."""
     dev = torch.cuda.current_device() if tensors[0].is_cuda else -1
     return (all(type(t) is torch.Tensor and t.is_cuda and t.device.index == dev and t.dtype == torch.float32
                 and t.is_contiguous() for t in tensors)
-            and torch._C._functorch.peek_interpreter_stack() is None
-            and torch.autograd.forward_ad._current_level < 0
-            and torch._C._len_torch_dispatch_stack() == 0
-            and torch._C._len_torch_function_stack() == 0
-            and not torch.jit.is_tracing() and not torch.compiler.is_compiling())
+            and _unwatched())
 
 
 def log_mse(S, S_target, floor: float = 1e-12):

@@ -174,3 +174,16 @@ def test_placed_entry_points_reject_bad_arguments():
     assert L.rg_spectrum_adjoint_placed(None, ctypes.byref(p), 8, 8, None, None, None, None,
                                         None) == capi.RG_ERR_ARGUMENT
     assert b"rg_spectrum_adjoint_placed" in L.rg_last_error()
+
+
+def test_log_mse_without_torchs_private_names(monkeypatch):
+    """log_mse looks at private names of torch before it leaves the tensor operations; where one is gone
+    (another release), it keeps them instead of failing."""
+    torch = pytest.importorskip("torch")
+    rt = pytest.importorskip("ragnar_gb300.torch_ext")
+    assert rt._unwatched()
+    for owner, name in ((torch._C, "_len_torch_dispatch_stack"), (torch._C, "_len_torch_function_stack"),
+                        (torch._C._functorch, "peek_interpreter_stack"), (torch.autograd.forward_ad, "_current_level")):
+        with monkeypatch.context() as m:
+            m.delattr(owner, name)
+            assert not rt._unwatched()
