@@ -167,10 +167,11 @@ def _unwatched() -> bool:
 
 
 def _plain_cuda(*tensors) -> bool:
-    """Contiguous float32 tensors of the current CUDA device, no subclasses, and _unwatched."""
+    """Contiguous float32 tensors of the current CUDA device whose memory holds their values (no negated
+    views), no subclasses, and _unwatched."""
     dev = torch.cuda.current_device() if tensors[0].is_cuda else -1
     return (all(type(t) is torch.Tensor and t.is_cuda and t.device.index == dev and t.dtype == torch.float32
-                and t.is_contiguous() for t in tensors)
+                and t.is_contiguous() and not t.is_neg() for t in tensors)
             and _unwatched())
 
 

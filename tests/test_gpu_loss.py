@@ -101,3 +101,11 @@ def test_forms_that_keep_the_tensor_operations(gpu):
     total += 1.0
     (h,) = torch.autograd.grad(total, S)
     assert torch.equal(h, g)
+
+
+def test_negated_view(gpu):
+    """The imaginary part of a conjugate is a view whose memory holds the opposite values."""
+    z = torch.tensor([1.0 - 2.0j], device=gpu)
+    S, T = z.conj().imag, torch.tensor([3.0], device=gpu)
+    assert S.is_neg() and S.is_contiguous() and S.dtype == torch.float32
+    assert abs(float(rt.log_mse(S, T)) - np.log(2.0 / 3.0) ** 2) <= 1e-6
