@@ -127,7 +127,7 @@ def synchrotron_from_dist(plan: capi.DistPlan, gbeta, f):
 class _LogMse(torch.autograd.Function):
     """The misfit and the two arrays its derivatives are made of, its gradient r and a = 1 / S on the
     c bins that count.  They are outputs, saved as such: a backward that is differentiated again
-    reaches S through them, to any order (dr/dS = 2 a^2 / c - r a, da/dS = -a^2), and S itself is not
+    reaches S through them, to any order (dr/dS = a (2 a / c - r), da/dS = -a^2), and S itself is not
     kept."""
 
     @staticmethod
@@ -144,11 +144,12 @@ class _LogMse(torch.autograd.Function):
     def backward(ctx, g, gr, ga):
         r, a, inv = ctx.saved_tensors
         gS = None if g is None else r * g
+        # the incoming vectors take one factor a first: a a is 1 / S^2, which is no float for S of 1e-20 or 1e23
         if gr is not None:
-            gr = gr * (2 * inv * a * a - r * a)
+            gr = (gr * a) * (2 * inv * a - r)
             gS = gr if gS is None else gS + gr
         if ga is not None:
-            ga = ga * (a * a)
+            ga = (ga * a) * a
             gS = -ga if gS is None else gS - ga
         return gS, None, None
 

@@ -109,3 +109,22 @@ def test_negated_view(gpu):
     S, T = z.conj().imag, torch.tensor([3.0], device=gpu)
     assert S.is_neg() and S.is_contiguous() and S.dtype == torch.float32
     assert abs(float(rt.log_mse(S, T)) - np.log(2.0 / 3.0) ** 2) <= 1e-6
+
+
+@pytest.mark.parametrize("scale", [1e-24, 1e-22, 1e-12, 1e12, 1e20, 1e22, 1e24])
+def test_hessian_vector_product_far_from_one(gpu, scale):
+    """A vector of the spectrum's own size: the product is about 1 / S, although 1 / S^2 is not a float.
+    Its terms are products of six FP32 factors with |d| up to 2.3, and differ by at most that factor
+    from the largest of them: 1e-5 of it."""
+    rng = np.random.default_rng(8)
+    s = scale * 10.0 ** rng.uniform(-0.5, 0.5, 64)
+    t = s * 10.0 ** rng.uniform(-1.0, 1.0, 64)
+    v = s * rng.uniform(0.5, 1.5, 64)
+    S = torch.from_numpy(s.astype(np.float32)).to(gpu).requires_grad_(True)
+    T, V = (torch.from_numpy(x.astype(np.float32)).to(gpu) for x in (t, v))
+    S64 = S.detach().double().requires_grad_(True)
+    (g,) = torch.autograd.grad(rt.log_mse(S, T), S, create_graph=True)
+    (h,) = torch.autograd.grad((g * V).sum(), S)
+    (g64,) = torch.autograd.grad(_formula(S64, T.double()), S64, create_graph=True)
+    (h64,) = torch.autograd.grad((g64 * V.double()).sum(), S64)
+    assert float((h.double() - h64).abs().max()) <= 1e-5 * float(h64.abs().max())
