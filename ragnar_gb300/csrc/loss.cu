@@ -107,7 +107,7 @@ namespace rg {
       return v;
     }
 
-    // c r and a of the same values, and their part of the sum and the count.
+    // d (0 where a value does not count) and a of the same values, and their part of the sum and the count.
     __device__ __forceinline__ Sum terms(const LossParams& p, float2 peak, int64_t i, int64_t step) {
       const float lowS = __fmul_rn(p.floor, peak.x), lowT = __fmul_rn(p.floor, peak.y);
       Sum         t { { 0.0f, 0.0f }, 0u };
@@ -115,7 +115,7 @@ namespace rg {
         const float s = p.S[i], y = p.T[i];
         const bool  m = s > lowS && y > lowT;
         const float d = m ? logf(s) - logf(y) : 0.0f;
-        p.r[i]        = m ? __fdiv_rn(d + d, s) : 0.0f;
+        p.r[i]        = d;
         p.a[i]        = m ? __frcp_rn(s) : 0.0f;
         t.v           = ff_add(t.v, two_prod(d, d));
         t.count += m ? 1u : 0u;
@@ -123,7 +123,8 @@ namespace rg {
       return t;
     }
 
-    // The loss and 1 / c, and r with it.
+    // The loss and 1 / c, and r = (2 d / c) / S from the d that terms left in its place: 2 d / S itself is
+    // above the float range for spectra near its lower end.
     __device__ __forceinline__ void finish(const LossParams& p, double2 t, float* inv, int64_t i, int64_t step) {
       if (threadIdx.x == 0) {
         const double count = fmax(t.y, 1.0);
@@ -135,7 +136,8 @@ namespace rg {
       }
       __syncthreads();
       for (; i < p.n; i += step) {
-        p.r[i] *= *inv;
+        const float d = p.r[i];
+        p.r[i]        = d != 0.0f ? __fdiv_rn(__fmul_rn(d + d, *inv), p.S[i]) : 0.0f;
       }
     }
 

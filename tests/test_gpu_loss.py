@@ -128,3 +128,15 @@ def test_hessian_vector_product_far_from_one(gpu, scale):
     (g64,) = torch.autograd.grad(_formula(S64, T.double()), S64, create_graph=True)
     (h64,) = torch.autograd.grad((g64 * V.double()).sum(), S64)
     assert float((h.double() - h64).abs().max()) <= 1e-5 * float(h64.abs().max())
+
+
+def test_gradient_of_spectra_near_the_smallest_float(gpu):
+    """2 (ln S - ln T) / S is above the float range where the gradient, its share of 512 values, is not."""
+    rng = np.random.default_rng(10)
+    S = torch.from_numpy((3e-38 * rng.uniform(1.0, 9.0, 512)).astype(np.float32)).to(gpu).requires_grad_(True)
+    T = (S.detach() * 1e4).contiguous()
+    (g,) = torch.autograd.grad(rt.log_mse(S, T), S)
+    S64 = S.detach().double().requires_grad_(True)
+    (g64,) = torch.autograd.grad(_formula(S64, T.double()), S64)
+    assert float(g64.abs().max()) < 3e38 and float((2 * torch.log(S64 / T.double()) / S64).abs().max()) > 3.5e38
+    assert float((g.double() - g64).abs().max()) <= 1e-5 * float(g64.abs().max())
