@@ -141,7 +141,7 @@ namespace rg {
       // in order over the whole table (each block decides for itself) or, above kRankMax, over
       // this block's photons
       bool out_of_order = false;
-      for (int k = rank ? static_cast<int>(threadIdx.x) : s; k + 1 < p.ns; k += kPrepThreads) {
+      for (int k = rank ? static_cast<int>(threadIdx.x) : s; k < p.ns - 1; k += kPrepThreads) {
         out_of_order = out_of_order || ic_inv4(p.es[k]) < ic_inv4(p.es[k + 1]);
         if (!rank) {
           break;
@@ -182,14 +182,15 @@ namespace rg {
           const LnParts l = ln_parts(ff { e, 0.0f }); // ln i = -ln(4 e)
           lni             = -((static_cast<double>(l.e) + 2.0) * M_LN2 + ff_to_double(ff { l.h, l.l }));
         }
-        const double wi = w * i;
-        p.sums.i4[at]   = make_float2(iv.hi, iv.lo);
-        p.terms[at]             = w;
-        p.terms[p.ns + at]      = wi;
-        p.terms[2 * static_cast<int64_t>(p.ns) + at] = wi * i;
-        p.terms[3 * static_cast<int64_t>(p.ns) + at] = wi * lni;
-        p.terms[4 * static_cast<int64_t>(p.ns) + at] = lni;
-        p.terms[5 * static_cast<int64_t>(p.ns) + at] = ri;
+        const double  wi = w * i;
+        const int64_t ns = p.ns; // 6 ns entries: more than 2^31 from 3.6e8 photons
+        p.sums.i4[at]        = make_float2(iv.hi, iv.lo);
+        p.terms[at]          = w;
+        p.terms[ns + at]     = wi;
+        p.terms[2 * ns + at] = wi * i;
+        p.terms[3 * ns + at] = wi * lni;
+        p.terms[4 * ns + at] = lni;
+        p.terms[5 * ns + at] = ri;
       }
       const int all = __syncthreads_and(ok);
       if (threadIdx.x == 0) {
@@ -354,7 +355,7 @@ namespace rg {
           // the first photon with q <= 1 (1 / (4 e_s) descends)
           int j = 0, n = p.ns;
           while (j < n) {
-            const int mid = (j + n) >> 1;
+            const int mid = j + ((n - j) >> 1);
             if (__fmul_rn(z.hi, __ldg(p.inv4es + mid)) <= 1.0f) {
               n = mid;
             } else {
