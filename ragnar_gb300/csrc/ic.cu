@@ -84,7 +84,10 @@ namespace rg {
       float*       inv4es_min; // min over s of 1 / (4 e_s) (positive values), one float
       float*       ws;      // ns: f_s / e_s
       double*      terms;   // [6][ns]: w, w i, w i^2, w i ln i, ln i, 1 / i with i = 1 / (4 e_s)
-      int*         block_ok; // per block of ic_terms_kernel: its photons are in order and in range
+      float2*      blocks;  // per block of ic_terms_kernel: smallest i (as inv4es_min), 1 if its photons are in order and in range
+      int          nblocks;
+      double*      tiles;   // [4][ntiles]: sums of the first four terms over a tile of kTile photons (more than one tile)
+      int          ntiles;
       int*         regular; // 1: the pair kernel runs, 0: the direct kernel
       IcSums       sums;
       int          ns;
@@ -100,6 +103,7 @@ namespace rg {
 
     constexpr int kPrepThreads = 256;
     constexpr int kPrepItems   = 4; // photons per thread and tile
+    constexpr int kTile        = kPrepThreads * kPrepItems;
     constexpr int kRankMax     = 16384; // photons that are ranked when they are out of order
     constexpr int kRankTile    = 1024;
     // energies and |weights| of a regular table: far enough from the ends of the float range for
@@ -126,6 +130,50 @@ namespace rg {
     // finite, or 1 / (4 e) above the float range): masked photons come first in the order.
     __device__ __forceinline__ float ic_inv4(float e) {
       return (e > 0.0f && isfinite(e)) ? __frcp_rn(__fmul_rn(4.0f, e)) : __int_as_float(0x7f800000);
+    }
+
+    // Of photons without a positive 1 / (4 e_s): above any such value of a positive float.
+    __device__ __forceinline__ float no_min() {
+      return __int_as_float(0x7f7f7f7f);
+    }
+
+    // v's smallest value over the block, in thread 0
+    __device__ __forceinline__ float block_min(float v) {
+      __shared__ float wmin[kPrepThreads / 32];
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        v = fminf(v, __shfl_xor_sync(0xffffffffu, v, o));
+      }
+      if ((threadIdx.x & 31) == 0) {
+        wmin[threadIdx.x >> 5] = v;
+      }
+      __syncthreads();
+      if (threadIdx.x == 0) {
+        for (int w = 1; w < kPrepThreads / 32; ++w) {
+          v = fminf(v, wmin[w]);
+        }
+      }
+      return v;
+    }
+
+    // v's sum over the block (in a fixed order), the same in every thread
+    __device__ __forceinline__ double block_sum(double v) {
+      __shared__ double wsum[kPrepThreads / 32];
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        v += __shfl_xor_sync(0xffffffffu, v, o);
+      }
+      __syncthreads(); // the last sum's values are read
+      if ((threadIdx.x & 31) == 0) {
+        wsum[threadIdx.x >> 5] = v;
+      }
+      __syncthreads();
+      v = 0.0;
+#pragma unroll
+      for (int w = 0; w < kPrepThreads / 32; ++w) {
+        v += wsum[w];
+      }
+      return v;
     }
 
     // Per photon (a thread each): its place in descending order of 1 / (4 e_s), and its terms of the
@@ -192,109 +240,128 @@ namespace rg {
         p.terms[4 * ns + at] = lni;
         p.terms[5 * ns + at] = ri;
       }
-      const int all = __syncthreads_and(ok);
+      const int all  = __syncthreads_and(ok);
+      float     imin = mine && i4 > 0.0f ? fminf(i4, no_min()) : no_min();
+      imin           = block_min(imin);
       if (threadIdx.x == 0) {
-        p.block_ok[blockIdx.x] = all;
+        p.blocks[blockIdx.x] = make_float2(imin, all ? 1.0f : 0.0f);
+        if (!all && p.ns > kRankMax) {
+          *p.regular = 0; // set before the launch: long tables skip their sums
+        }
       }
     }
 
-    // One block per sum (blockIdx.x = 0: W0, 1: V1, 2: V2, 3: V3): the photons are walked from the
-    // end in tiles of 1024, a thread summing four consecutive ones, in FP64 (the sums' range
-    // exceeds FP32's); four SMs share the FP64 additions.  Block 0 also decides which kernel runs.
+    // The sum of a term (0 .. 3) over a tile, for the tiles before it: block 4 tile + term.
+    __global__ void __launch_bounds__(kPrepThreads) ic_tiles_kernel(const __grid_constant__ IcParams p) {
+      const int     which = blockIdx.x & 3, tile = blockIdx.x >> 2;
+      const int64_t base = static_cast<int64_t>(tile) * kTile;
+      if (p.ns > kRankMax && !*p.regular) {
+        return;
+      }
+      double        v    = 0.0;
+#pragma unroll
+      for (int k = 0; k < kPrepItems; ++k) {
+        const int64_t s = base + k * kPrepThreads + threadIdx.x;
+        v += s < p.ns ? p.terms[which * static_cast<int64_t>(p.ns) + s] : 0.0;
+      }
+      v = block_sum(v);
+      if (threadIdx.x == 0) {
+        p.tiles[static_cast<int64_t>(which) * p.ntiles + tile] = v;
+      }
+    }
+
+    // One block per sum (0: W0, 1: V1, 2: V2, 3: V3) and tile of photons (block 4 tile + sum), a
+    // thread summing four consecutive ones from the tile's end, in FP64 (the sums' range exceeds
+    // FP32's), after the sums of the later tiles; several SMs share the FP64 additions.  Block 0
+    // also decides which kernel runs.  10 gamma bins x 10 IC bins: 16384 photons 62 us (one block walking
+    // all tiles, 7 us each: 160), 1e5 62 (720), 1e6 0.26 ms (7.1); evaluated directly 40, 59 and 0.27 ms.
     __global__ void __launch_bounds__(kPrepThreads) ic_sums_kernel(const __grid_constant__ IcParams p) {
       __shared__ double wtot[2][kPrepThreads / 32];
-      __shared__ float  wmin[kPrepThreads / 32];
-      const int     which = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-      const int     tile = kPrepThreads * kPrepItems;
-      const int64_t ns   = p.ns;
-      double        carry = 0.0, carry1 = 0.0; // sums over the tiles done (carry1: V3's sum of w i)
-      for (int64_t r0 = 0; r0 < ns; r0 += tile) {
-        double a[kPrepItems], a1[kPrepItems];
-        double t = 0.0, t1 = 0.0;
-#pragma unroll
-        for (int k = 0; k < kPrepItems; ++k) {
-          const int64_t s = ns - 1 - (r0 + tid * kPrepItems + k);
-          a[k]  = s >= 0 ? p.terms[which * ns + s] : 0.0;
-          a1[k] = (s >= 0 && which == 3) ? p.terms[ns + s] : 0.0;
-          t += a[k];
-          t1 += a1[k];
+      const int     which = blockIdx.x & 3, tile = blockIdx.x >> 2, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+      const int64_t ns   = p.ns, first = static_cast<int64_t>(tile) * kTile, end = min(ns, first + kTile);
+      double        carry = 0.0, carry1 = 0.0; // sums over the later tiles (carry1: V3's sum of w i)
+      if (p.ns > kRankMax && blockIdx.x != 0 && !*p.regular) {
+        return;
+      }
+      if (p.ntiles > 1) {
+        const double* later = p.tiles + static_cast<int64_t>(which) * p.ntiles;
+        const double* later1 = p.tiles + p.ntiles;
+        for (int k = tile + 1 + tid; k < p.ntiles; k += kPrepThreads) {
+          carry += later[k];
+          carry1 += which == 3 ? later1[k] : 0.0;
         }
-        // inclusive sums over the warp's threads
-        double x = t, x1 = t1;
+        carry  = block_sum(carry);
+        carry1 = which == 3 ? block_sum(carry1) : 0.0;
+      }
+      double a[kPrepItems], a1[kPrepItems];
+      double t = 0.0, t1 = 0.0;
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-          const double y  = __shfl_up_sync(0xffffffffu, x, o);
-          const double y1 = which == 3 ? __shfl_up_sync(0xffffffffu, x1, o) : 0.0;
-          if (lane >= o) {
-            x += y;
-            x1 += y1;
-          }
-        }
-        if (lane == 31) {
-          wtot[0][warp] = x;
-          wtot[1][warp] = x1;
-        }
-        __syncthreads();
-        double before = carry, before1 = carry1;
+      for (int k = 0; k < kPrepItems; ++k) {
+        const int64_t s = end - 1 - (tid * kPrepItems + k);
+        const bool    in = s >= first;
+        a[k]  = in ? p.terms[which * ns + s] : 0.0;
+        a1[k] = (in && which == 3) ? p.terms[ns + s] : 0.0;
+        t += a[k];
+        t1 += a1[k];
+      }
+      // inclusive sums over the warp's threads
+      double x = t, x1 = t1;
 #pragma unroll
-        for (int w = 0; w < kPrepThreads / 32; ++w) {
-          if (w == warp) {
-            before  = carry;
-            before1 = carry1;
-          }
-          carry += wtot[0][w];
-          carry1 += wtot[1][w];
+      for (int o = 1; o < 32; o <<= 1) {
+        const double y  = __shfl_up_sync(0xffffffffu, x, o);
+        const double y1 = which == 3 ? __shfl_up_sync(0xffffffffu, x1, o) : 0.0;
+        if (lane >= o) {
+          x += y;
+          x1 += y1;
         }
-        // the lane below holds this lane's exclusive sum within the warp
-        const double up = __shfl_up_sync(0xffffffffu, x, 1), up1 = __shfl_up_sync(0xffffffffu, x1, 1);
-        double       run = lane > 0 ? before + up : before, run1 = lane > 0 ? before1 + up1 : before1;
-        __syncthreads(); // wtot is reused by the next tile
+      }
+      if (lane == 31) {
+        wtot[0][warp] = x;
+        wtot[1][warp] = x1;
+      }
+      __syncthreads();
+      for (int w = 0; w < warp; ++w) {
+        carry += wtot[0][w];
+        carry1 += wtot[1][w];
+      }
+      // the lane below holds this lane's exclusive sum within the warp
+      const double up = __shfl_up_sync(0xffffffffu, x, 1), up1 = __shfl_up_sync(0xffffffffu, x1, 1);
+      double       run = lane > 0 ? carry + up : carry, run1 = lane > 0 ? carry1 + up1 : carry1;
 #pragma unroll
-        for (int k = 0; k < kPrepItems; ++k) {
-          const int64_t s = ns - 1 - (r0 + tid * kPrepItems + k);
-          run += a[k];
-          run1 += a1[k];
-          if (s >= 0) {
-            if (which == 0) {
-              p.sums.w0[s] = double_to_ff(run);
+      for (int k = 0; k < kPrepItems; ++k) {
+        const int64_t s = end - 1 - (tid * kPrepItems + k);
+        run += a[k];
+        run1 += a1[k];
+        if (s >= first) {
+          if (which == 0) {
+            p.sums.w0[s] = double_to_ff(run);
+          } else {
+            const double ri = p.terms[5 * ns + s];
+            if (which == 1) {
+              p.sums.v1[s] = double_to_ff(run * ri);
+            } else if (which == 2) {
+              p.sums.v2[s] = double_to_ff(run * ri * ri);
             } else {
-              const double ri = p.terms[5 * ns + s];
-              if (which == 1) {
-                p.sums.v1[s] = double_to_ff(run * ri);
-              } else if (which == 2) {
-                p.sums.v2[s] = double_to_ff(run * ri * ri);
-              } else {
-                p.sums.v3[s] = double_to_ff((run - p.terms[4 * ns + s] * run1) * ri);
-              }
+              p.sums.v3[s] = double_to_ff((run - p.terms[4 * ns + s] * run1) * ri);
             }
           }
         }
       }
-      if (which == 0) {
+      if (blockIdx.x == 0) {
         bool  ok   = true;
-        float imin = __int_as_float(0x7f7f7f7f); // above any 1 / (4 e_s) of a positive float
-        for (int64_t s = tid; s < ns; s += kPrepThreads) {
-          const float i4 = p.inv4es[s];
-          imin           = i4 > 0.0f ? fminf(imin, i4) : imin;
-        }
-        for (int k = tid; k < (p.ns + kPrepThreads - 1) / kPrepThreads; k += kPrepThreads) {
-          ok = ok && p.block_ok[k] != 0;
+        float imin = no_min();
+        for (int k = tid; k < p.nblocks; k += kPrepThreads) {
+          const float2 b = p.blocks[k];
+          imin           = fminf(imin, b.x);
+          ok             = ok && b.y != 0.0f;
         }
         const int all = __syncthreads_and(ok);
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-          imin = fminf(imin, __shfl_xor_sync(0xffffffffu, imin, o));
-        }
-        if (lane == 0) {
-          wmin[warp] = imin;
-        }
-        __syncthreads();
+        imin          = block_min(imin);
         if (tid == 0) {
-          for (int w = 1; w < kPrepThreads / 32; ++w) {
-            imin = fminf(imin, wmin[w]);
-          }
           *p.inv4es_min = imin;
-          *p.regular    = all;
+          if (ns <= kRankMax) { // otherwise ic_terms_kernel has said so, and other blocks read it
+            *p.regular = all;
+          }
         }
       }
     }
@@ -586,9 +653,11 @@ int rg_ic_spectrum(const float* gbins, const float* f, int32_t ng, int32_t log_s
   // one stream-ordered scratch allocation: photon arrays, sums, partial rows
   const auto     up       = [](size_t v) { return 256 * ((v + 255) / 256); };
   const size_t   n4 = up(sizeof(float) * ns), n8 = up(sizeof(float2) * ns), n48 = up(sizeof(double) * 6 * ns);
-  const int      term_blocks = (ns + rg::kPrepThreads - 1) / rg::kPrepThreads;
+  const int      term_blocks = (ns - 1) / rg::kPrepThreads + 1;
   const size_t   off_sums = 2 * n4, off_terms = off_sums + 5 * n8, off_min = off_terms + n48;
-  const size_t   off_ok = off_min + 256, off_pairs = off_ok + up(sizeof(int) * term_blocks);
+  const int      tiles  = (ns - 1) / rg::kTile + 1;
+  const size_t   off_blocks = off_min + 256, off_tiles = off_blocks + up(sizeof(float2) * term_blocks);
+  const size_t   off_pairs = off_tiles + up(sizeof(double) * 4 * tiles);
   const size_t   off_part = off_pairs + up(sizeof(double) * static_cast<size_t>(splits) * ne);
   const size_t   bytes    = off_part + sizeof(double) * static_cast<size_t>(grid) * nslices * slice_w;
   unsigned char* buf      = nullptr;
@@ -607,7 +676,10 @@ int rg_ic_spectrum(const float* gbins, const float* f, int32_t ng, int32_t log_s
     *sums[k] = reinterpret_cast<float2*>(buf + off_sums + k * n8);
   }
   p.terms      = reinterpret_cast<double*>(buf + off_terms);
-  p.block_ok   = reinterpret_cast<int*>(buf + off_ok);
+  p.blocks     = reinterpret_cast<float2*>(buf + off_blocks);
+  p.nblocks    = term_blocks;
+  p.tiles      = reinterpret_cast<double*>(buf + off_tiles);
+  p.ntiles     = tiles;
   p.inv4es_min = reinterpret_cast<float*>(buf + off_min);
   p.regular    = reinterpret_cast<int*>(buf + off_min + 128);
   p.ns         = ns;
@@ -617,10 +689,17 @@ int rg_ic_spectrum(const float* gbins, const float* f, int32_t ng, int32_t log_s
   p.slice_w    = slice_w;
   p.pairs      = reinterpret_cast<double*>(buf + off_pairs);
   p.partials   = reinterpret_cast<double*>(buf + off_part);
-  rg::ic_terms_kernel<<<term_blocks, rg::kPrepThreads, 0, s>>>(p);
-  cudaError_t e = cudaGetLastError();
+  cudaError_t e = ns > rg::kRankMax ? cudaMemsetAsync(p.regular, 1, sizeof(int), s) : cudaSuccess;
   if (e == cudaSuccess) {
-    rg::ic_sums_kernel<<<4, rg::kPrepThreads, 0, s>>>(p);
+    rg::ic_terms_kernel<<<term_blocks, rg::kPrepThreads, 0, s>>>(p);
+    e = cudaGetLastError();
+  }
+  if (e == cudaSuccess && tiles > 1) {
+    rg::ic_tiles_kernel<<<4 * tiles, rg::kPrepThreads, 0, s>>>(p);
+    e = cudaGetLastError();
+  }
+  if (e == cudaSuccess) {
+    rg::ic_sums_kernel<<<4 * tiles, rg::kPrepThreads, 0, s>>>(p);
     e = cudaGetLastError();
   }
   if (e == cudaSuccess) {

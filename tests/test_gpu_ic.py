@@ -181,3 +181,19 @@ def test_non_finite_photon_weights_spread_as_before(gpu, oracle_lib):
         fs[7] = bad
         got = gpu_ic(gb, fp, True, es, fs, eic, gpu)
         assert not np.any(np.isfinite(got))
+
+
+@pytest.mark.parametrize("ns", [255, 1023, 1024, 1025, 2049, 16384, 16385, 70001])
+def test_tables_of_several_tiles(gpu, oracle_lib, ns):
+    """Sums over more than one tile of 1024 photons, in order and (up to 16384, equal photons among
+    them) out of order, at the edges of tiles and of the blocks that rank the photons."""
+    rng = np.random.default_rng(ns)
+    gb = oracle_lib.logspace(10.0, 1e5, 19)
+    fp = (gb.astype(np.float64) ** -2.0).astype(np.float32)
+    es = np.repeat(oracle_lib.logspace(1e-8, 1e-3, (ns + 2) // 3), 3)[:ns]
+    fs = (rng.uniform(0.5, 1.5, ns) * es.astype(np.float64) ** -0.5).astype(np.float32)
+    eic = oracle_lib.logspace(1e-3, 1e5, 37)
+    want = oracle_lib.ic_spectrum_f64(gb, fp, True, es, fs, eic)
+    assert max_rel(gpu_ic(gb, fp, True, es, fs, eic, gpu), want) <= SPECTRUM_RTOL
+    order = rng.permutation(ns)
+    assert max_rel(gpu_ic(gb, fp, True, es[order], fs[order], eic, gpu), want) <= SPECTRUM_RTOL
