@@ -105,7 +105,8 @@ namespace rg {
     constexpr int kPrepItems   = 4; // photons per thread and tile
     constexpr int kTile        = kPrepThreads * kPrepItems;
     constexpr int kRankMax     = 16384; // photons that are ranked when they are out of order
-    constexpr int kRankTile    = 1024;
+    constexpr int kRankTile    = 1024; // a multiple of a block's photons
+    constexpr int kRankWays    = 4;     // threads that share a photon's comparisons
     // energies and |weights| of a regular table: far enough from the ends of the float range for
     // every double-float product of the pair kernel
     constexpr float kRegularLo = 1e-30f, kRegularHi = 1e30f;
@@ -176,42 +177,62 @@ namespace rg {
       return v;
     }
 
-    // Per photon (a thread each): its place in descending order of 1 / (4 e_s), and its terms of the
-    // four sums.  A table already in order keeps its places; one of up to kRankMax photons in any
-    // other order is ranked by comparing all pairs (ns^2 comparisons against ng x ne x ns evals of
-    // the direct kernel); a longer one is left to the direct kernel.  Quotients and logarithms are
-    // taken in double-floats, as FP64 issues at 1.6 operations per clock and SM.
+    // Per photon: its place in descending order of 1 / (4 e_s), and its terms of the four sums.  A table
+    // already in order keeps its places; one of up to kRankMax photons in any other order is ranked by
+    // comparing all pairs (ns^2 comparisons against ng x ne x ns evals of the direct kernel); a longer
+    // one is left to the direct kernel.  Where ranks may be needed, kRankWays threads share a
+    // photon's comparisons (and a block has fewer photons), so that they fill the chip: 16384 photons
+    // out of order take 56 us more than in order, with a thread per photon 215 us.  Quotients and
+    // logarithms are taken in double-floats, as FP64 issues at 1.6 operations per clock and SM.
     __global__ void __launch_bounds__(kPrepThreads) ic_terms_kernel(const __grid_constant__ IcParams p) {
-      __shared__ float keys[kRankTile];
-      const int  s    = blockIdx.x * kPrepThreads + threadIdx.x;
-      const bool mine = s < p.ns;
+      __shared__ float4 keys[kRankTile / 4];
       const bool rank = p.ns <= kRankMax;
+      const int  ways = rank ? kRankWays : 1, part = threadIdx.x & (ways - 1);
+      const int  s0   = blockIdx.x * (kPrepThreads / ways), s = s0 + static_cast<int>(threadIdx.x) / ways;
+      const bool mine = s < p.ns && part == 0;
       // in order over the whole table (each block decides for itself) or, above kRankMax, over
       // this block's photons
       bool out_of_order = false;
-      for (int k = rank ? static_cast<int>(threadIdx.x) : s; k < p.ns - 1; k += kPrepThreads) {
-        out_of_order = out_of_order || ic_inv4(p.es[k]) < ic_inv4(p.es[k + 1]);
-        if (!rank) {
-          break;
+      if (rank) {
+#pragma unroll 4
+        for (int k = threadIdx.x; k < p.ns - 1; k += kPrepThreads) {
+          out_of_order = out_of_order || ic_inv4(p.es[k]) < ic_inv4(p.es[k + 1]);
         }
+      } else {
+        out_of_order = s < p.ns - 1 && ic_inv4(p.es[s]) < ic_inv4(p.es[s + 1]);
       }
       const bool  unsorted = __syncthreads_or(out_of_order) != 0;
-      const float e = mine ? p.es[s] : 0.0f, f = mine ? p.fs[s] : 0.0f;
+      const float e = s < p.ns ? p.es[s] : 0.0f, f = s < p.ns ? p.fs[s] : 0.0f;
       const float i4  = ic_inv4(e);
       const bool  use = i4 <= 3.402823466e38f; // false for inf: a photon that contributes nothing
       int         at  = s;
       if (unsorted && rank) {
         at = 0;
         for (int t0 = 0; t0 < p.ns; t0 += kRankTile) {
-          const int m = min(kRankTile, p.ns - t0);
           __syncthreads();
-          for (int k = threadIdx.x; k < m; k += kPrepThreads) {
-            keys[k] = ic_inv4(p.es[t0 + k]);
+          for (int k = threadIdx.x; k < kRankTile; k += kPrepThreads) {
+            reinterpret_cast<float*>(keys)[k] = t0 + k < p.ns ? ic_inv4(p.es[t0 + k]) : -1.0f; // before no photon
           }
           __syncthreads();
-          for (int k = 0; k < m; ++k) {
-            at += (keys[k] > i4 || (keys[k] == i4 && t0 + k < s)) ? 1 : 0;
+          // equal keys keep their order: photons before this one count where they are equal too
+          const bool before = t0 + kRankTile <= s0, after = t0 > s0;
+#pragma unroll 4
+          for (int k = part; k < kRankTile / 4; k += kRankWays) {
+            const float4 v = keys[k];
+            if (before) {
+              at += (v.x >= i4) + (v.y >= i4) + (v.z >= i4) + (v.w >= i4);
+            } else if (after) {
+              at += (v.x > i4) + (v.y > i4) + (v.z > i4) + (v.w > i4);
+            } else {
+              const int t = t0 + 4 * k;
+              at += (v.x > i4 || (v.x == i4 && t < s)) + (v.y > i4 || (v.y == i4 && t + 1 < s)) +
+                    (v.z > i4 || (v.z == i4 && t + 2 < s)) + (v.w > i4 || (v.w == i4 && t + 3 < s));
+            }
           }
+        }
+#pragma unroll
+        for (int o = 1; o < kRankWays; o <<= 1) {
+          at += __shfl_xor_sync(0xffffffffu, at, o);
         }
       }
       bool ok = rank || !unsorted;
@@ -653,7 +674,8 @@ int rg_ic_spectrum(const float* gbins, const float* f, int32_t ng, int32_t log_s
   // one stream-ordered scratch allocation: photon arrays, sums, partial rows
   const auto     up       = [](size_t v) { return 256 * ((v + 255) / 256); };
   const size_t   n4 = up(sizeof(float) * ns), n8 = up(sizeof(float2) * ns), n48 = up(sizeof(double) * 6 * ns);
-  const int      term_blocks = (ns - 1) / rg::kPrepThreads + 1;
+  const int      per_block   = ns <= rg::kRankMax ? rg::kPrepThreads / rg::kRankWays : rg::kPrepThreads;
+  const int      term_blocks = (ns - 1) / per_block + 1;
   const size_t   off_sums = 2 * n4, off_terms = off_sums + 5 * n8, off_min = off_terms + n48;
   const int      tiles  = (ns - 1) / rg::kTile + 1;
   const size_t   off_blocks = off_min + 256, off_tiles = off_blocks + up(sizeof(float2) * term_blocks);
