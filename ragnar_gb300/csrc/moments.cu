@@ -272,10 +272,94 @@ namespace rg {
       *to = f;
     }
 
+    // The packed sums of a warp hold entries from 2^-kFinBelow to 2^kFinAbove times its scale with all their
+    // bits: split_double keeps 2^-44 down to 2^-74 and anything down to 2^-126, and the coefficients are
+    // not below 2^-34.  Rows that reach further start a new scale, and a row that spans more by itself
+    // (a particle that outweighs a neighbour by 1e18) is summed in FP64.
+    constexpr int kFinBelow = 60, kFinAbove = 40;
+
+    // The warp's bin sums into the slice's, in FP64, and back to zero.
+    __device__ __noinline__ void flush_sums(float2* acc, int nv, int scale, double* total) {
+      const double s = __hiloint2double((scale + 1023) << 20, 0);
+      for (int i = threadIdx.x & 31; i < nv; i += 32) {
+        const float2 a = acc[i];
+        if (a.x != 0.0f) {
+          atomicAdd(total + i, (static_cast<double>(a.x) + static_cast<double>(a.y)) * s);
+        }
+        acc[i] = make_float2(0.0f, 0.0f);
+      }
+    }
+
+    // A row of cell c in FP64, from its copy in shared memory: sums below in place, sums above beside
+    // it, then every bin's share into the slice's sums.
+    __device__ __noinline__ void wide_row(double2* row_sums, double2* above, const float4* coef, const FinBin* bins, int nv,
+                                          int c, int nseg_tab, double* total) {
+      const int lane = threadIdx.x & 31, row = nv + 1, per = (row + 31) / 32;
+      const int j0 = min(lane * per, row), j1 = min(j0 + per, row);
+      double    l0 = 0.0, l1 = 0.0;
+      for (int j = j0; j < j1; ++j) {
+        l0 += row_sums[j].x;
+        l1 += row_sums[j].y;
+      }
+      double u0 = l0, u1 = l1;
+      for (int o = 1; o < 32; o <<= 1) {
+        const double a0 = __shfl_up_sync(0xffffffffu, l0, o), a1 = __shfl_up_sync(0xffffffffu, l1, o);
+        const double b0 = __shfl_down_sync(0xffffffffu, u0, o), b1 = __shfl_down_sync(0xffffffffu, u1, o);
+        if (lane >= o) {
+          l0 += a0;
+          l1 += a1;
+        }
+        if (lane + o < 32) {
+          u0 += b0;
+          u1 += b1;
+        }
+      }
+      l0 = __shfl_up_sync(0xffffffffu, l0, 1);
+      l1 = __shfl_up_sync(0xffffffffu, l1, 1);
+      u0 = __shfl_down_sync(0xffffffffu, u0, 1);
+      u1 = __shfl_down_sync(0xffffffffu, u1, 1);
+      if (lane == 0) {
+        l0 = l1 = 0.0;
+      }
+      if (lane == 31) {
+        u0 = u1 = 0.0;
+      }
+      for (int j = j1 - 1; j >= j0; --j) {
+        above[j] = make_double2(u0, u1);
+        u0 += row_sums[j].x;
+        u1 += row_sums[j].y;
+      }
+      for (int j = j0; j < j1; ++j) {
+        l0 += row_sums[j].x;
+        l1 += row_sums[j].y;
+        row_sums[j] = make_double2(l0, l1);
+      }
+      __syncwarp();
+      const double unit = 1.0 / (1u << kMomFrac);
+      for (int i = lane; i < nv; i += 32) {
+        const FinBin b = bins[i];
+        const int    s = c - b.Dc;
+        if (s >= 0 && s <= nseg_tab) {
+          const float4  ku = coef[s + 1], kl = coef[s];
+          const double2 U = above[b.pos], L = row_sums[b.pos];
+          const double  nD = static_cast<double>(b.nDh) + static_cast<double>(b.nDl);
+          const double  mD = static_cast<double>(b.mDh) + static_cast<double>(b.mDl);
+          const double  y  = (static_cast<double>(ku.x) + static_cast<double>(ku.y)) * U.x +
+                           (static_cast<double>(ku.z) + static_cast<double>(ku.w)) * (U.y * unit + nD * U.x) +
+                           (static_cast<double>(kl.x) + static_cast<double>(kl.y)) * L.x +
+                           (static_cast<double>(kl.z) + static_cast<double>(kl.w)) * (L.y * unit + mD * L.x);
+          if (y != 0.0) {
+            atomicAdd(total + i, y);
+          }
+        }
+      }
+      __syncwarp(); // the row's buffer takes the next row
+    }
+
     // One warp per cell row, kFinWarps rows in flight per block, blockIdx.y = (segment, slice).
-    // The row is copied to shared memory (coalesced) and set back to zero; a lane takes C consecutive entries (M0, and M1 in segment units, as packed
-    // double-floats scaled by a power of two), and the warp leaves the row's sums below (L) and
-    // above (U) every threshold in shared memory.  U is summed from the row's end, not as
+    // The row is copied to shared memory (coalesced) and set back to zero; a lane takes C consecutive
+    // entries (M0, and M1 in segment units, as packed double-floats scaled by a power of two), and the
+    // warp leaves the row's sums below (L) and above (U) every threshold in shared memory.  U is summed from the row's end, not as
     // total - L, so that a bin with no particle above its threshold gets an exact zero.  Then
     // lanes own bins in the order of their cells, so that whole groups of 32 skip the cells their
     // table segments do not reach.  Double-floats (2^-44) because the FP64 pipe issues 1.6
@@ -285,7 +369,7 @@ namespace rg {
     // with it two blocks fit an SM (146 us) instead of three.  Blocks add their bins' sums in FP64; the last block of a (segment, slice) writes the
     // spectrum.
     template <int C>
-    __global__ void __launch_bounds__(kFinThreads) moments_finish_kernel(const __grid_constant__ MomentFinishParams r) {
+    __global__ void __launch_bounds__(kFinThreads, C <= 4 ? 4 : C <= 8 ? 3 : C <= 12 ? 2 : 1) moments_finish_kernel(const __grid_constant__ MomentFinishParams r) {
       extern __shared__ __align__(16) unsigned char smem[];
       __shared__ int   wscale[kFinWarps];
       __shared__ bool  last;
@@ -300,6 +384,7 @@ namespace rg {
       float4*    buf   = reinterpret_cast<float4*>(sums + kFinWarps * groups) + 2 * warp * row;
       float4*    Us    = buf + row;
       double2*   hist  = r.hist + seg * r.per_seg + ms.z;
+      double*    total = r.acc + static_cast<int64_t>(blockIdx.y) * kSliceBins;
       const int  c0 = blockIdx.x * kFinWarps + warp, cstep = gridDim.x * kFinWarps;
       auto fetch = [&](int c) {
         if (c < ms.y) {
@@ -337,14 +422,17 @@ namespace rg {
         __syncwarp(); // every lane's copies of this row have landed
         double2* h = hist + static_cast<int64_t>(c) * row;
         double2  d[C];
-        int      top = 0; // largest exponent of the row
+        int      top = 0, low = 0x7ff; // largest and smallest exponent of the row
 #pragma unroll
         for (int k = 0; k < C; ++k) {
           const int j = lane * C + k;
           d[k]        = j < row ? *reinterpret_cast<const double2*>(buf + j) : make_double2(0.0, 0.0);
-          top = max(top, max((__double2hiint(d[k].x) >> 20) & 0x7ff, ((__double2hiint(d[k].y) >> 20) & 0x7ff) - kMomFrac));
+          const int e0 = (__double2hiint(d[k].x) >> 20) & 0x7ff, e1 = ((__double2hiint(d[k].y) >> 20) & 0x7ff) - kMomFrac;
+          top = max(top, max(e0, e1));
+          low = min(low, e0 > 0 ? e0 : e1 > 0 ? e1 : 0x7ff); // of M0; M1 matters beside it only as much as it is large
         }
         top = __reduce_max_sync(0xffffffffu, top);
+        low = __reduce_min_sync(0xffffffffu, low);
         if (top == 0) { // an empty row
           continue;
         }
@@ -354,11 +442,14 @@ namespace rg {
         if (failed) {
           continue;
         }
-        if (top - 1023 > scale + 40) { // room for sums 2^40 above the first row's largest entry
-          const int   down = top - 1023 - scale;
-          const float f    = down > 126 ? 0.0f : __uint_as_float(static_cast<uint32_t>(127 - down) << 23);
-          for (int i = lane; i < groups; i += 32) {
-            acc[i] = make_float2(acc[i].x * f, acc[i].y * f);
+        if (top - low > kFinBelow) {
+          __syncwarp(); // every lane has read the row
+          wide_row(reinterpret_cast<double2*>(buf), reinterpret_cast<double2*>(Us), coef, bins, nv, c, r.nseg_tab, total);
+          continue;
+        }
+        if (top - 1023 > scale + kFinAbove || low - 1023 < scale - kFinBelow) {
+          if (scale > -2000) {
+            flush_sums(acc, nv, scale, total);
           }
           scale = top - 1023;
         }
@@ -440,20 +531,24 @@ namespace rg {
       for (int w = 1; w < kFinWarps; ++w) {
         top = max(top, wscale[w]);
       }
-      double* total = r.acc + static_cast<int64_t>(blockIdx.y) * kSliceBins;
       if (top > -2000) {
         const double s2 = __hiloint2double((top + 1023) << 20, 0);
         for (int i = threadIdx.x; i < nv; i += kFinThreads) {
-          ff t { 0.0f, 0.0f };
+          ff     t { 0.0f, 0.0f };
+          double far = 0.0; // of warps whose scale is too far below for the packed sum
 #pragma unroll
           for (int w = 0; w < kFinWarps; ++w) {
             const int    down = top - wscale[w];
-            const float  f    = down > 126 ? 0.0f : __uint_as_float(static_cast<uint32_t>(127 - down) << 23);
             const float2 a    = sums[w * groups + i];
-            t                 = ff_add(t, ff { a.x * f, a.y * f });
+            if (down <= kFinAbove) {
+              const float f = __uint_as_float(static_cast<uint32_t>(127 - down) << 23);
+              t             = ff_add(t, ff { a.x * f, a.y * f });
+            } else if (a.x != 0.0f) {
+              far += (static_cast<double>(a.x) + static_cast<double>(a.y)) * __hiloint2double((wscale[w] + 1023) << 20, 0);
+            }
           }
-          if (t.hi != 0.0f) {
-            atomicAdd(total + i, (static_cast<double>(t.hi) + static_cast<double>(t.lo)) * s2);
+          if (t.hi != 0.0f || far != 0.0) {
+            atomicAdd(total + i, (static_cast<double>(t.hi) + static_cast<double>(t.lo)) * s2 + far);
           }
         }
       }

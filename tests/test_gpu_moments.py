@@ -215,3 +215,42 @@ def test_moments_nearly_cancelling_force(gpu, oracle_lib, table, mode, efield, t
         xmin, xmax = float(np.exp(lnx)), float(np.exp(lnx + coef.shape[0] * dln))
         truth = oracle_lib.sync_smooth_f64(P, bins, 1.0, 1.0, 1.0, coef, xmin, xmax)
     assert max_rel(out.cpu().numpy(), truth) <= SPECTRUM_RTOL
+
+
+@pytest.mark.parametrize("mode", ["reference"])
+@pytest.mark.parametrize("nseg,spread", [(1, "near"), (1, "far"), (300, "near"), (300, "far")])
+def test_moments_of_very_unequal_weights(gpu, oracle_lib, table, mode, nseg, spread):
+    """One particle outweighs the others by 1e39, in their own cell and the next ones or over decades of
+    energies; bins below the heavy one's table range see only the light ones, whose sums the FP64
+    moments hold exactly whatever else their cell or its neighbours hold."""
+    heavy = 1e4
+    k  = np.arange(1, 61)
+    ep = heavy / np.concatenate([[1.0], 1.0 + 4e-3 * k if spread == "near" else 1.2**k])
+    a  = np.sqrt((np.sqrt(1.0 + 4.0 * ep * ep) - 1.0) / 2.0)  # e_peak = u sqrt(1 + u^2) for u across a unit B
+    z  = np.zeros(len(a), np.float32)
+    P  = {"ux": a.astype(np.float32), "uy": z, "uz": z, "bx": z, "by": z, "bz": z + np.float32(1.0),
+          "w": np.concatenate([[1e30], np.resize([1e-9, 3e-9, 2e-9], 60)]).astype(np.float32)}
+    bins = oracle_lib.logspace(1e-6 * ep.min() * 1.001, 1e-6 * heavy * 1.01, 24 if spread == "near" else 200)
+    plan = capi.SpectrumPlan(bins, 1.0, 1.0, 1.0,
+                             capi.RG_TABLE_SMOOTH if mode == "smooth" else capi.RG_TABLE_REFERENCE)
+    assert plan.algorithm(nseg) == capi.RG_ALGO_MOMENTS
+    xmin = 1e-6
+    if mode == "reference":
+        truth = oracle_lib.sync_spectrum_f64(P, bins, 1.0, 1.0, 1.0, table)
+    else:
+        coef, lnx, dln = plan.smooth_table()
+        xmin, xmax = float(np.exp(lnx)), float(np.exp(lnx + coef.shape[0] * dln))
+        truth = oracle_lib.sync_smooth_f64(P, bins, 1.0, 1.0, 1.0, coef, xmin, xmax)
+    # bins next to the low end of a particle's table range count it or not by rounding
+    keep = np.all(np.abs(bins[:, None].astype(np.float64) / (xmin * ep[None, :]) - 1.0) > 1e-4, axis=1)
+    assert keep.sum() >= 20 and np.all(truth[keep] > 0.0) and truth[keep].max() > 1e36 * truth[keep].min()
+    T, prt = _device({k: np.tile(v, nseg) for k, v in P.items()}, gpu)
+    out = torch.full((nseg, len(bins)), -1.0, device=gpu)
+    if nseg == 1:
+        plan.run(prt, out)
+    else:
+        offs = torch.arange(nseg + 1, device=gpu, dtype=torch.int64) * len(a)
+        plan.run_batched(prt, offs, nseg, out)
+    plan.check()
+    got = out.cpu().numpy().astype(np.float64)[:, keep]
+    assert np.max(np.abs(got - truth[keep]) / truth[keep]) <= SPECTRUM_RTOL
