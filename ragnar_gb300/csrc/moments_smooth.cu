@@ -192,6 +192,11 @@ namespace rg {
     };
 
     constexpr int kFinCells = 16; // cells per block: two per warp
+    // Cells up to 2^-kFinBelow of the block's largest keep all their bits in its packed sums, whose products
+    // with coefficients down to the smallest float (the table's far end) are kept exact by the
+    // moments' unit 2^-kFinUnit; blocks whose cells span more (a particle that outweighs others by
+    // 1e18) sum in FP64.
+    constexpr int kFinBelow = 60, kFinUnit = 60;
 
     // Block: kFinCells cells of one segment (blockIdx.y).  Its warps sum the cells' slots in FP64 and
     // clear them, and leave the cells that hold anything in shared memory as double-floats scaled
@@ -207,7 +212,7 @@ namespace rg {
       __shared__ double sums[kFinCells][4];
       __shared__ float4 Mh[kFinCells + 1], Ml[kFinCells + 1]; // moments of the block's live cells, hi and lo
       __shared__ int    live[kFinCells + 1], nlive, scale;
-      __shared__ bool   last;
+      __shared__ bool   wide, last;
       const int  seg = blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
       const int  c0 = blockIdx.x * kFinCells, ncell = min(kFinCells, r.nc - c0);
       const bool failed = *r.status != kDevOk;
@@ -261,13 +266,15 @@ namespace rg {
       }
       __syncthreads();
       if (warp == 0) { // the live cells in order, and the scale: the largest exponent
-        int top = 0;
+        int top = 0, low = 0x7ff; // the cell's largest exponent; that of its sum of amplitudes
         if (lane < ncell) {
 #pragma unroll
           for (int j = 0; j < 4; ++j) {
             top = max(top, (__double2hiint(sums[lane][j]) >> 20) & 0x7ff);
           }
+          low = top > 0 ? (__double2hiint(sums[lane][0]) >> 20) & 0x7ff : 0x7ff;
         }
+        low = __reduce_min_sync(0xffffffffu, low);
         const unsigned on  = __ballot_sync(0xffffffffu, top > 0);
         const int      all = __reduce_max_sync(0xffffffffu, top) - 1023;
         if (top > 0) {
@@ -275,7 +282,7 @@ namespace rg {
           float2    f[4];
 #pragma unroll
           for (int j = 0; j < 4; ++j) {
-            f[j] = split_double(sums[lane][j], all);
+            f[j] = split_double(sums[lane][j], all - kFinUnit);
           }
           live[at] = c0 + lane;
           Mh[at]   = make_float4(f[0].x, f[1].x, f[2].x, f[3].x);
@@ -286,13 +293,32 @@ namespace rg {
           live[n]     = -1; // the second cell of an odd last pair: in no bin's table
           Mh[n] = Ml[n] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
           nlive = n;
-          scale = all;
+          scale = all - kFinUnit;
+          wide  = all + 1023 - low > kFinBelow;
         }
       }
       __syncthreads();
       const int n     = nlive;
       double*   total = r.acc + static_cast<int64_t>(seg) * r.acc_stride;
-      if (n > 0 && !failed) {
+      if (n > 0 && !failed && wide) {
+        for (int b = threadIdx.x; b < r.nbins; b += kPairThreads) {
+          const int4 bi = r.binfo[b];
+          double     A = 0.0, B = 0.0;
+          for (int k = 0; k < n && bi.w; ++k) {
+            const int s = live[k] - bi.x;
+            if (s >= 0 && s < r.nseg_tab) {
+              const double* M = sums[live[k] - c0];
+              const float4  c = coef[s];
+              A += c.x * M[0] + c.y * M[1] + c.z * M[2] + c.w * M[3];
+              B += c.y * M[0] + 2.0 * c.z * M[1] + 3.0 * c.w * M[2];
+            }
+          }
+          const double t = A + static_cast<double>(__int_as_float(bi.y)) * B;
+          if (t != 0.0) {
+            atomicAdd(total + b, t);
+          }
+        }
+      } else if (n > 0 && !failed) {
         const double s2 = __hiloint2double((scale + 1023) << 20, 0);
         for (int b = threadIdx.x; b < r.nbins; b += kPairThreads) {
           const int4 bi = r.binfo[b];

@@ -217,7 +217,7 @@ def test_moments_nearly_cancelling_force(gpu, oracle_lib, table, mode, efield, t
     assert max_rel(out.cpu().numpy(), truth) <= SPECTRUM_RTOL
 
 
-@pytest.mark.parametrize("mode", ["reference"])
+@pytest.mark.parametrize("mode", ["reference", "smooth"])
 @pytest.mark.parametrize("nseg,spread", [(1, "near"), (1, "far"), (300, "near"), (300, "far")])
 def test_moments_of_very_unequal_weights(gpu, oracle_lib, table, mode, nseg, spread):
     """One particle outweighs the others by 1e39, in their own cell and the next ones or over decades of
