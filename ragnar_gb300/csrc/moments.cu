@@ -68,6 +68,7 @@ namespace rg {
       const uint32_t* bucket;  // per slice: kMomBuckets entries (bucket_entry)
       double*         hist;    // nseg x per_seg interval moments (M0, M1)
       int64_t         per_seg;
+      RunSums         run;
     };
 
     // A bucket's entry: with `first` thresholds below the bucket and at most one inside it, at
@@ -133,6 +134,7 @@ namespace rg {
       __shared__ __align__(16) uint32_t bucket[kMomBuckets]; // staged 16 bytes at a time
       __shared__ int64_t                logt[kLogEntries];
       __shared__ uint32_t               soff[kSeg ? kMomSharedSeg + 1 : 1];
+      clear_run_sums(m.run);
       const int  slice = blockIdx.y;
       const int4 ms    = m.mslice[slice];
       stage_log_table(m.log, kMomExtra, m.range[2 * slice + 1], logt, kPairThreads);
@@ -234,8 +236,8 @@ namespace rg {
       int             nbins;
       const float*    ebins;
       const unsigned* status;
-      double*         acc;      // [nseg][nslices][kSliceBins], zero between runs
-      unsigned*       done;     // [nseg][nslices] blocks finished, zero between runs
+      double*         acc;      // [nseg][nslices][kSliceBins], cleared by the deposit
+      unsigned*       done;     // [nseg][nslices] blocks finished, cleared by the deposit
       float*          out;      // nseg x nbins
     };
 
@@ -574,13 +576,9 @@ namespace rg {
       for (int i = threadIdx.x; i < nv; i += kFinThreads) {
         const double t = __ldcg(total + i);
         const int    j = r.bins[slice * kSliceBins + i].w;
-        total[i]       = 0.0;
         if (!failed) {
           out[j] = __double2float_rn(t * static_cast<double>(r.ebins[n0 + j]));
         }
-      }
-      if (threadIdx.x == 0) {
-        r.done[blockIdx.y] = 0;
       }
     }
 
@@ -746,9 +744,11 @@ namespace rg {
     return static_cast<size_t>(nseg) * static_cast<size_t>(pl->hist_per_seg) * sizeof(double2) <= kMomMaxBytes;
   }
 
-  // Moment tables for nseg segments.  They are zero between runs: zeroed here when they are
-  // allocated, and by each run's finish kernel, which reads every entry anyway (a memset per
-  // run costs a launch for one spectrum, and a pass over 350 MB for 256).
+  // Moment tables and sums for nseg segments.  The tables are zero between runs: zeroed here when they
+  // are allocated, and by each run's finish kernel, which reads every entry anyway (a memset per run
+  // costs a launch for one spectrum, and a pass over 350 MB for 256).  Runs that overlapped (which a
+  // plan does not allow) leave them zero too: the finish that starts last comes after all deposits and
+  // clears what it finds.
   int moments_reserve(rg_spectrum_plan* pl, int nseg, cudaStream_t s) {
     const size_t need = static_cast<size_t>(nseg) * static_cast<size_t>(pl->hist_per_seg);
     if (need > pl->hist_cap) {
@@ -765,8 +765,7 @@ namespace rg {
       pl->d_msum   = nullptr;
       pl->msum_cap = 0;
       const size_t bytes = sums * (sizeof(double) * kSliceBins + sizeof(unsigned));
-      RG_CUDA_TRY(cudaMalloc(&pl->d_msum, bytes));
-      RG_CUDA_TRY(cudaMemsetAsync(pl->d_msum, 0, bytes, s));
+      RG_CUDA_TRY(cudaMalloc(&pl->d_msum, bytes)); // cleared by each run
       pl->msum_cap = sums;
     }
     return RG_OK;
@@ -778,7 +777,6 @@ namespace rg {
     RG_TRY(moments_reserve(pl, nseg, s));
     if (pl->hist_dirty) {
       RG_CUDA_TRY(cudaMemsetAsync(pl->d_hist, 0, sizeof(double2) * pl->hist_cap, s));
-      RG_CUDA_TRY(cudaMemsetAsync(pl->d_msum, 0, pl->msum_cap * (sizeof(double) * kSliceBins + sizeof(unsigned)), s));
     }
     pl->hist_dirty = true;
     return RG_OK;
@@ -786,6 +784,14 @@ namespace rg {
 
   // Adds the particles [0, n) (one segment, d_off null) or the nseg segments of d_off to
   // the interval moments.
+  // A run without particles has no deposit.
+  int moments_clear_sums(rg_spectrum_plan* pl, cudaStream_t s) {
+    const RunSums r = run_sums(pl, 1);
+    RG_CUDA_TRY(cudaMemsetAsync(r.sums, 0, sizeof(double) * r.nsums, s));
+    RG_CUDA_TRY(cudaMemsetAsync(r.done, 0, sizeof(unsigned) * r.ndone, s));
+    return RG_OK;
+  }
+
   int moments_deposit(rg_spectrum_plan* pl, const float* const comp[kComps], const int64_t* d_off, int64_t n,
                       int nseg, cudaStream_t s) {
     if (pl->aligned) {
@@ -800,11 +806,12 @@ namespace rg {
     m.bucket  = pl->d_bucket;
     m.hist    = reinterpret_cast<double*>(pl->d_hist);
     m.per_seg = pl->hist_per_seg;
+    m.run     = run_sums(pl, d_off ? nseg : 1);
     fill_log_params(pl, m.log);
     DeviceContext* ctx = nullptr;
     RG_TRY(context(&ctx));
     if (n == 0 && !d_off) {
-      return RG_OK;
+      return moments_clear_sums(pl, s);
     }
     std::pair<cudaEvent_t, cudaEvent_t> ev { nullptr, nullptr };
     if (pl->timing) {

@@ -60,6 +60,7 @@ namespace rg {
       float          tau_scale; // 2^-F
       int            nc;        // cells
       double*        hist;      // [nseg][nc][kSub][4]
+      RunSums        run;       // the deposit's
       uint2*         place;     // single-segment runs: per particle (cell, fraction bits) or
                                 // (kNoCell, 0) for a particle that adds nothing; null: not kept
     };
@@ -113,6 +114,7 @@ namespace rg {
       smooth_deposit_kernel(const __grid_constant__ SmoothMomParams m) {
       __shared__ int64_t  logt[kLogEntries];
       __shared__ uint32_t soff[kSeg ? kPairSharedSeg + 1 : 1];
+      clear_run_sums(m.run);
       stage_log_table(m.log, m.log.fx, m.Pmax, logt, kPairThreads);
       if (!stage_segments<kSeg>(m.in, m.fp.status, soff)) {
         return;
@@ -185,8 +187,8 @@ namespace rg {
       int             nbins;
       const float*    ebins;
       const unsigned* status;
-      double*         acc;   // [nseg][acc_stride], zero between runs
-      unsigned*       done;  // [nseg] blocks finished, zero between runs
+      double*         acc;   // [nseg][acc_stride], cleared by the deposit
+      unsigned*       done;  // [nseg] blocks finished, cleared by the deposit
       int             acc_stride;
       float*          out;   // nseg x nbins
     };
@@ -372,12 +374,8 @@ namespace rg {
       __threadfence();
       for (int b = threadIdx.x; b < r.nbins; b += kPairThreads) {
         const double t = __ldcg(total + b);
-        total[b]       = 0.0;
         r.out[static_cast<int64_t>(seg) * r.nbins + b] =
           failed ? __int_as_float(0x7fffffff) : __double2float_rn(t * static_cast<double>(r.ebins[b]));
-      }
-      if (threadIdx.x == 0) {
-        r.done[seg] = 0;
       }
     }
 
@@ -769,10 +767,11 @@ namespace rg {
   int smooth_moments_deposit(rg_spectrum_plan* pl, const float* const comp[kComps], const int64_t* d_off, int64_t n,
                              int nseg, cudaStream_t s, uint2* place) {
     if (n == 0 && !d_off) {
-      return RG_OK;
+      return moments_clear_sums(pl, s);
     }
     SmoothMomParams m;
     fill_smooth_params(pl, comp, d_off, n, nseg, m);
+    m.run = run_sums(pl, d_off ? nseg : 1);
     DeviceContext* ctx = nullptr;
     RG_TRY(context(&ctx));
     std::pair<cudaEvent_t, cudaEvent_t> ev { nullptr, nullptr };

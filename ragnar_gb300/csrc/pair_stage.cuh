@@ -388,6 +388,31 @@ namespace rg {
     return static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(steps, static_cast<int64_t>(sms) * per_sm)));
   }
 
+  // The finish kernel's bin sums and block counts, cleared by the deposit that comes before it on the
+  // stream, whatever an earlier run left in them.
+  struct RunSums {
+    double*   sums;
+    int64_t   nsums;
+    unsigned* done;
+    int64_t   ndone;
+  };
+
+  inline RunSums run_sums(const rg_spectrum_plan* pl, int nseg) {
+    const int64_t rows = static_cast<int64_t>(nseg) * pl->nslices;
+    return { pl->d_msum, rows * kSliceBins, reinterpret_cast<unsigned*>(pl->d_msum + pl->msum_cap * kSliceBins), rows };
+  }
+
+  __device__ __forceinline__ void clear_run_sums(const RunSums& r) {
+    const int64_t step = static_cast<int64_t>(gridDim.x) * gridDim.y * kPairThreads;
+    const int64_t i0   = (static_cast<int64_t>(blockIdx.y) * gridDim.x + blockIdx.x) * kPairThreads + threadIdx.x;
+    for (int64_t i = i0; i < r.nsums; i += step) {
+      r.sums[i] = 0.0;
+    }
+    for (int64_t i = i0; i < r.ndone; i += step) {
+      r.done[i] = 0u;
+    }
+  }
+
   // Stages the segments' offsets, clamped to the window and relative to its start; false for the
   // whole block if they decrease or leave [0, n], or if the status word is set.
   template <bool kSeg>

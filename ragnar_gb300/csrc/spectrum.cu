@@ -1302,6 +1302,9 @@ int rg_spectrum_run_host(rg_spectrum_plan* pl, const rg_particles* p, float* out
     }
     RG_CUDA_TRY(cudaEventRecord(st->consumed[b], s));
   }
+  if (moments && n == 0) {
+    RG_TRY(rg::moments_clear_sums(pl, s));
+  }
   if (moments) {
     return rg::moments_finish(pl, 1, out, s);
   }

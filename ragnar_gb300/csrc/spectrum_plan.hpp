@@ -54,7 +54,7 @@ struct rg_spectrum_plan {
   int64_t               hist_per_seg = 0;      // double2 entries of one segment's histograms
   double2*              d_hist      = nullptr; // zero between runs (the finish kernels clear what they read)
   size_t                hist_cap    = 0;       // double2 entries
-  double*               d_msum      = nullptr; // per (segment, slice): bin sums, then block counts; zero between runs
+  double*               d_msum      = nullptr; // per (segment, slice): bin sums, then block counts; cleared by each run
   size_t                msum_cap    = 0;       // (segment, slice) pairs
   bool                  hist_dirty  = false;   // a run has deposited and not finished
   // fixed-point logarithm of the pair stage (pair_stage.cuh)
@@ -96,6 +96,7 @@ namespace rg {
   int  moments_reserve(rg_spectrum_plan* pl, int nseg, cudaStream_t s);
   int  fixed_log_prepare(rg_spectrum_plan* pl, int F, double dln);
   int  moments_begin(rg_spectrum_plan* pl, int nseg, cudaStream_t s);
+  int  moments_clear_sums(rg_spectrum_plan* pl, cudaStream_t s);
   int  moments_deposit(rg_spectrum_plan* pl, const float* const comp[10], const int64_t* d_off, int64_t n,
                        int nseg, cudaStream_t s);
   int  moments_finish(rg_spectrum_plan* pl, int nseg, float* out, cudaStream_t s);
