@@ -744,20 +744,20 @@ namespace rg {
     return static_cast<size_t>(nseg) * static_cast<size_t>(pl->hist_per_seg) * sizeof(double2) <= kMomMaxBytes;
   }
 
-  // Moment tables and sums for nseg segments.  The tables are zero between runs: zeroed here when they
-  // are allocated, and by each run's finish kernel, which reads every entry anyway (a memset per run
-  // costs a launch for one spectrum, and a pass over 350 MB for 256).  Runs that overlapped (which a
+  // Moment tables and sums for nseg segments.  The tables are zero between runs: zeroed after they are
+  // allocated (moments_clear), and by each run's finish kernel, which reads every entry anyway (a memset
+  // per run costs a launch for one spectrum, and a pass over 350 MB for 256).  Runs that overlapped (which a
   // plan does not allow) leave them zero too: the finish that starts last comes after all deposits and
   // clears what it finds.
-  int moments_reserve(rg_spectrum_plan* pl, int nseg, cudaStream_t s) {
+  int moments_reserve(rg_spectrum_plan* pl, int nseg) {
     const size_t need = static_cast<size_t>(nseg) * static_cast<size_t>(pl->hist_per_seg);
     if (need > pl->hist_cap) {
       cudaFree(pl->d_hist);
       pl->d_hist   = nullptr;
       pl->hist_cap = 0;
       RG_CUDA_TRY(cudaMalloc(&pl->d_hist, sizeof(double2) * need));
-      RG_CUDA_TRY(cudaMemsetAsync(pl->d_hist, 0, sizeof(double2) * need, s));
-      pl->hist_cap = need;
+      pl->hist_cap   = need;
+      pl->hist_dirty = true; // not zero yet
     }
     const size_t sums = static_cast<size_t>(nseg) * pl->nslices;
     if (sums > pl->msum_cap) {
@@ -771,19 +771,32 @@ namespace rg {
     return RG_OK;
   }
 
-  // Before a run's deposits: the tables of nseg segments, zero (also after a run that failed
-  // between its deposit and its finish).
-  int moments_begin(rg_spectrum_plan* pl, int nseg, cudaStream_t s) {
-    RG_TRY(moments_reserve(pl, nseg, s));
+  // The tables zero, as of the work queued on s before this call.
+  int moments_clear(rg_spectrum_plan* pl, cudaStream_t s) {
     if (pl->hist_dirty) {
       RG_CUDA_TRY(cudaMemsetAsync(pl->d_hist, 0, sizeof(double2) * pl->hist_cap, s));
+      pl->hist_dirty = false;
     }
-    pl->hist_dirty = true;
     return RG_OK;
   }
 
-  // Adds the particles [0, n) (one segment, d_off null) or the nseg segments of d_off to
-  // the interval moments.
+  // Before a run's deposits: the tables of nseg segments, zero (also new ones, and after a run that
+  // failed between its deposit and its finish).  A captured run only records its memset and its
+  // finish: tables that were not zero before it are still not zero for the next run that executes.
+  int moments_begin(rg_spectrum_plan* pl, int nseg, cudaStream_t s) {
+    RG_TRY(moments_reserve(pl, nseg));
+    bool recorded = false;
+    if (pl->hist_dirty) {
+      cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+      RG_CUDA_TRY(cudaStreamIsCapturing(s, &capture));
+      recorded = capture != cudaStreamCaptureStatusNone;
+    }
+    RG_TRY(moments_clear(pl, s));
+    pl->hist_dirty       = true;
+    pl->hist_stays_dirty = recorded;
+    return RG_OK;
+  }
+
   // A run without particles has no deposit.
   int moments_clear_sums(rg_spectrum_plan* pl, cudaStream_t s) {
     const RunSums r = run_sums(pl, 1);
@@ -921,7 +934,7 @@ namespace rg {
         return set_error(RG_ERR_UNSUPPORTED, "more than 512 bins in a slice");
     }
     RG_TRY(st);
-    pl->hist_dirty = false;
+    pl->hist_dirty = pl->hist_stays_dirty;
     return RG_OK;
   }
 

@@ -828,7 +828,7 @@ namespace rg {
     smooth_finish_kernel<<<dim3((pl->sm_cells + kFinCells - 1) / kFinCells, nseg), kPairThreads,
                            sizeof(float4) * pl->smooth->nseg, s>>>(r);
     RG_CUDA_TRY(cudaGetLastError());
-    pl->hist_dirty = false;
+    pl->hist_dirty = pl->hist_stays_dirty;
     return RG_OK;
   }
 

@@ -762,9 +762,9 @@ namespace rg {
     // the interval moments of max_seg segments, so that runs allocate nothing (and can be
     // captured in a CUDA graph)
     if (moments_selected(pl, max_seg)) {
-      const size_t cap = pl->hist_cap, sums = pl->msum_cap;
-      RG_TRY(moments_reserve(pl, max_seg, nullptr));
-      if (pl->hist_cap != cap || pl->msum_cap != sums) {
+      RG_TRY(moments_reserve(pl, max_seg));
+      if (pl->hist_dirty) {
+        RG_TRY(moments_clear(pl, nullptr));
         RG_CUDA_TRY(cudaStreamSynchronize(nullptr)); // zeroed before any stream's run
       }
       // the smooth moment path's per-cell scratch (the adjoint's cubics)

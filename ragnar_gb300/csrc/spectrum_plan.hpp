@@ -56,7 +56,8 @@ struct rg_spectrum_plan {
   size_t                hist_cap    = 0;       // double2 entries
   double*               d_msum      = nullptr; // per (segment, slice): bin sums, then block counts; cleared by each run
   size_t                msum_cap    = 0;       // (segment, slice) pairs
-  bool                  hist_dirty  = false;   // a run has deposited and not finished
+  bool                  hist_dirty  = false;   // d_hist may not be zero: new, or a run has deposited and not finished
+  bool                  hist_stays_dirty = false; // ... and the run in progress only records that it clears it
   // fixed-point logarithm of the pair stage (pair_stage.cuh)
   int64_t*              d_logt      = nullptr;
   int                   log_fx      = 0;
@@ -93,7 +94,8 @@ namespace rg {
   int  moments_prepare(rg_spectrum_plan* pl, const std::vector<uint8_t>& valid, double ln_xmin, double dln,
                        double ln_k0);
   bool moments_selected(const rg_spectrum_plan* pl, int nseg);
-  int  moments_reserve(rg_spectrum_plan* pl, int nseg, cudaStream_t s);
+  int  moments_reserve(rg_spectrum_plan* pl, int nseg);
+  int  moments_clear(rg_spectrum_plan* pl, cudaStream_t s);
   int  fixed_log_prepare(rg_spectrum_plan* pl, int F, double dln);
   int  moments_begin(rg_spectrum_plan* pl, int nseg, cudaStream_t s);
   int  moments_clear_sums(rg_spectrum_plan* pl, cudaStream_t s);

@@ -15,6 +15,8 @@ rounding for interval moments, whose FP64 atomic sums do not fix the order).
 
 from __future__ import annotations
 
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -488,3 +490,55 @@ def test_fused_item_sizes(gpu, oracle_lib, n, source):
             plan.check()
             want = oracle_lib.sync_from_dist_f64(g, f, True, bins, 1.0, 1.0, table)[0]
         assert max_rel(out.cpu().numpy(), want) <= SPECTRUM_RTOL
+
+
+def test_first_run_recorded_into_a_graph(gpu, oracle_lib):
+    """A plan whose larger tables are first allocated while a graph records: the graph's memset has not run
+    when the next run executes, so that run clears them itself."""
+    P    = particles(20000, seed=41, bfield="iso", weights=True)
+    bins = oracle_lib.logspace(1e-2, 1e7, 20)
+    T, prt = to_device(P, gpu)
+    offs = torch.tensor([0, 3000, 9000, 20000], device=gpu, dtype=torch.int64)
+    want, out = torch.empty((3, 20), device=gpu), torch.empty((3, 20), device=gpu)
+    make_plan(bins).run_batched(prt, offs, 3, want)
+    # memory that holds something: the tables of a plan whose run failed after its deposit
+    other = make_plan(bins)
+    other.reserve(3)
+    assert capi.lib().rg_malloc(ctypes.byref(ctypes.c_void_p()), 1 << 60) == capi.RG_ERR_CUDA  # left pending
+    with pytest.raises(capi.RgError):
+        other.run_batched(prt, offs, 3, out)
+    plan = make_plan(bins)
+    torch.cuda.synchronize()
+    other.close()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, capture_error_mode="relaxed"):
+        plan.run_batched(prt, offs, 3, out, torch.cuda.current_stream(gpu).cuda_stream)
+    out.fill_(-1.0)
+    plan.run_batched(prt, offs, 3, out)
+    plan.check()
+    assert torch.allclose(out, want, rtol=1e-6, atol=0.0)
+    for _ in range(2):
+        out.fill_(-1.0)
+        graph.replay()
+        plan.check()
+        assert torch.allclose(out, want, rtol=1e-6, atol=0.0)
+
+
+def test_run_after_one_that_failed_halfway(gpu, oracle_lib, algo):
+    """A run whose launch reports an error after its deposit (here an earlier call's error that is still
+    pending): the next run starts from clear tables."""
+    P    = particles(20000, seed=42, bfield="iso", weights=True)
+    bins = oracle_lib.logspace(1e-2, 1e7, 200)
+    T, prt = to_device(P, gpu)
+    plan = make_plan(bins, algo=algo)
+    want, out = torch.empty(200, device=gpu), torch.empty(200, device=gpu)
+    plan.run(prt, want)
+    plan.check()
+    none = ctypes.c_void_p()
+    assert capi.lib().rg_malloc(ctypes.byref(none), 1 << 60) == capi.RG_ERR_CUDA  # out of memory, and left pending
+    with pytest.raises(capi.RgError):
+        plan.run(prt, out)
+    for _ in range(2):
+        plan.run(prt, out)
+        plan.check()
+        same(out, want, algo)
