@@ -967,22 +967,59 @@ namespace rg {
     constexpr std::size_t kParticlePlans = 32, kDistPlans = 8;
     using PlanKey = std::tuple<int, std::vector<float>, float, float, float>;
 
+    // A kept particle plan.  Its callers share its tables, so its runs are ordered on the GPU: a run on
+    // another stream waits for the last one.
+    struct ParticlePlan {
+      rg_spectrum_plan* plan = nullptr;
+      cudaEvent_t       done = nullptr; // after the last run, where that was not on the null stream
+      cudaStream_t      last = nullptr;
+      bool              used = false;
+
+      ~ParticlePlan() {
+        rg_spectrum_plan_destroy(plan);
+        if (done) {
+          cudaEventDestroy(done);
+        }
+      }
+    };
+
+    // Runs a kept plan on s after its last run.  The event after a run on the null stream is recorded
+    // when another stream asks for it (that stream is never destroyed), so that the calls of a
+    // program that only uses the null stream carry no events.  A run that is captured is ordered by its
+    // graph's launches alone.
+    int run_ordered(ParticlePlan& e, const rg_particles* p, float* out, cudaStream_t s) {
+      const bool              null    = s == nullptr || s == cudaStreamLegacy;
+      cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+      if (!null) {
+        RG_CUDA_TRY(cudaStreamIsCapturing(s, &capture));
+      }
+      if (capture != cudaStreamCaptureStatusNone) {
+        return rg_spectrum_run(e.plan, p, out, s);
+      }
+      if (e.used && !(null && !e.last)) {
+        if (!e.last) {
+          RG_CUDA_TRY(cudaEventRecord(e.done, nullptr));
+        }
+        RG_CUDA_TRY(cudaStreamWaitEvent(s, e.done, 0));
+      }
+      const int st = rg_spectrum_run(e.plan, p, out, s);
+      e.used       = true;
+      e.last       = null ? nullptr : s;
+      if (!null) {
+        RG_CUDA_TRY(cudaEventRecord(e.done, s));
+      }
+      return st;
+    }
+
     struct PlanCaches {
       std::mutex                                            mu;
-      std::map<PlanKey, rg_spectrum_plan*>                  particles;
+      std::map<PlanKey, std::unique_ptr<ParticlePlan>>      particles;
       std::vector<std::pair<PlanKey, rg_spectrum_plan*>>    dist; // idle, most recent last
     };
 
     PlanCaches& plan_caches() { // never destroyed: its plans are device memory (rg_finalize frees them)
       static auto* c = new PlanCaches();
       return *c;
-    }
-
-    void free_particle_plans(PlanCaches& c) {
-      for (auto& kv : c.particles) {
-        rg_spectrum_plan_destroy(kv.second);
-      }
-      c.particles.clear();
     }
 
   } // namespace
@@ -993,7 +1030,7 @@ namespace rg {
     if (!c.particles.empty()) {
       cudaDeviceSynchronize();
     }
-    free_particle_plans(c);
+    c.particles.clear();
     for (auto& kv : c.dist) {
       rg_spectrum_plan_destroy(kv.second);
     }
@@ -1376,21 +1413,20 @@ int rg_synchrotron_spectrum(const rg_particles* p, const float* bins, int32_t nb
   int dev = 0;
   RG_CUDA_TRY(cudaGetDevice(&dev));
   rg::PlanKey                 key { dev, std::vector<float>(bins, bins + nbins), B0, g_syn, e_syn_at_g_syn };
-  rg::PlanCaches&             c  = rg::plan_caches();
-  rg_spectrum_plan*           pl = nullptr;
+  rg::PlanCaches&             c = rg::plan_caches();
   std::lock_guard<std::mutex> lock(c.mu); // also while the run's launches are queued: they share the plan's tables
   auto                        it = c.particles.find(key);
   if (it == c.particles.end()) {
-    RG_TRY(rg_spectrum_plan_create(bins, nbins, B0, g_syn, e_syn_at_g_syn, RG_TABLE_REFERENCE, &pl));
+    auto e = std::make_unique<rg::ParticlePlan>();
+    RG_TRY(rg_spectrum_plan_create(bins, nbins, B0, g_syn, e_syn_at_g_syn, RG_TABLE_REFERENCE, &e->plan));
+    RG_CUDA_TRY(cudaEventCreateWithFlags(&e->done, cudaEventDisableTiming));
     if (c.particles.size() >= rg::kParticlePlans) {
       RG_CUDA_TRY(cudaDeviceSynchronize());
-      rg::free_particle_plans(c);
+      c.particles.clear();
     }
-    c.particles.emplace(std::move(key), pl);
-  } else {
-    pl = it->second;
+    it = c.particles.emplace(std::move(key), std::move(e)).first;
   }
-  return rg_spectrum_run(pl, p, out, stream);
+  return rg::run_ordered(*it->second, p, out, static_cast<cudaStream_t>(stream));
 }
 
 int rg_dist_run(const rg_spectrum_plan* plan, const float* gbeta, const float* f, int32_t ng, float* out,

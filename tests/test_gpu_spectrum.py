@@ -542,3 +542,24 @@ def test_run_after_one_that_failed_halfway(gpu, oracle_lib, algo):
         plan.run(prt, out)
         plan.check()
         same(out, want, algo)
+
+
+def test_one_shot_spectra_on_two_streams(gpu, oracle_lib, table):
+    """rg_synchrotron_spectrum takes no plan, so calls with the same bins and scalars share a kept one: their
+    runs are ordered over streams (null, and ones that do not wait for it), and a call after them is right."""
+    bins = oracle_lib.logspace(1e-2, 1e7, 300)
+    L    = capi.lib()
+    sets = [particles(n, seed=n, bfield="iso", weights=True) for n in (300001, 20011, 100003)]
+    want = [oracle_lib.sync_spectrum_f64(P, bins, 1.0, 1.0, 1.0, table) for P in sets]
+    dev  = [to_device(P, gpu) for P in sets]
+    streams = [torch.cuda.Stream(gpu).cuda_stream, torch.cuda.Stream(gpu).cuda_stream, 0]
+    outs = torch.full((60, 300), -1.0, device=gpu)
+    torch.cuda.synchronize()
+    for i in range(60):
+        prt = dev[i % 3][1]
+        capi.check(L.rg_synchrotron_spectrum(ctypes.byref(prt), bins.ctypes.data, 300, 1.0, 1.0, 1.0,
+                                             outs[i].data_ptr(), streams[(i * 7 // 3) % 3]))
+    torch.cuda.synchronize()
+    got = outs.cpu().numpy()
+    for i in range(60):
+        assert max_rel(got[i], want[i % 3]) <= SPECTRUM_RTOL, i
