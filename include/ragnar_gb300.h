@@ -58,7 +58,9 @@ enum {
  * device array and kernels resident.  Idempotent. */
 int rg_init(int device);
 
-/* rg.Finalize (pyinterface.cpp:40-49): release cached plans and tables. */
+/* rg.Finalize (pyinterface.cpp:40-49): release cached plans and tables.  Waits for calls of
+ * rg_synchrotron_spectrum and rg_synchrotron_spectrum_from_dist on other threads; plans that the
+ * caller made must not be used afterwards. */
 int rg_finalize(void);
 
 /* Message of the last failed call on this thread ("" if none). */

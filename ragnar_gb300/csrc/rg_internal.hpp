@@ -10,6 +10,7 @@
 #include <cstdint>
 #include <memory>
 #include <mutex>
+#include <shared_mutex>
 #include <string>
 #include <vector>
 
@@ -173,6 +174,9 @@ namespace rg {
   void free_threshold_cache();
   // Plans kept for the calls that take none (spectrum.cu).
   void free_plan_caches();
+  // Shared by the calls that keep a plan, which points to the library's tables, for the next one;
+  // rg_finalize takes it alone, so that no call puts a plan back whose tables are gone.
+  std::shared_mutex& library_mutex();
 
   // Host grids with the reference's float/double arithmetic.
   float logspace_point(float start, float stop, std::size_t num, std::size_t i);

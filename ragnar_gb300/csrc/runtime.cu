@@ -24,6 +24,11 @@ namespace rg {
     }
   } // namespace
 
+  std::shared_mutex& library_mutex() {
+    static std::shared_mutex m;
+    return m;
+  }
+
   int set_error(int status, const std::string& msg) {
     g_last_error = msg;
     return status;
@@ -239,6 +244,7 @@ int rg_init(int device) {
 }
 
 int rg_finalize(void) {
+  std::unique_lock<std::shared_mutex> alone(rg::library_mutex());
   rg::free_threshold_cache();
   rg::free_plan_caches();
   rg::free_idle_blocks();

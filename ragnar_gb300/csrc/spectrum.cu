@@ -1414,6 +1414,7 @@ int rg_synchrotron_spectrum(const rg_particles* p, const float* bins, int32_t nb
   RG_CUDA_TRY(cudaGetDevice(&dev));
   rg::PlanKey                 key { dev, std::vector<float>(bins, bins + nbins), B0, g_syn, e_syn_at_g_syn };
   rg::PlanCaches&             c = rg::plan_caches();
+  std::shared_lock<std::shared_mutex> life(rg::library_mutex());
   std::lock_guard<std::mutex> lock(c.mu); // also while the run's launches are queued: they share the plan's tables
   auto                        it = c.particles.find(key);
   if (it == c.particles.end()) {
@@ -1457,6 +1458,7 @@ int rg_synchrotron_spectrum_from_dist(const float* gbeta, const float* f, int32_
   }
   int dev = 0;
   RG_CUDA_TRY(cudaGetDevice(&dev));
+  std::shared_lock<std::shared_mutex> life(rg::library_mutex()); // until the plan is put back
   rg::PlanKey       key { dev, std::vector<float>(bins, bins + nbins), log_spaced ? 1.0f : 0.0f, g_syn, e_syn_at_g_syn };
   rg::PlanCaches&   c = rg::plan_caches();
   rg_spectrum_plan* pl = nullptr;

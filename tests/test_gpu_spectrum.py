@@ -16,6 +16,9 @@ rounding for interval moments, whose FP64 atomic sums do not fix the order).
 from __future__ import annotations
 
 import ctypes
+import os
+import subprocess
+import sys
 
 import numpy as np
 import pytest
@@ -563,3 +566,55 @@ def test_one_shot_spectra_on_two_streams(gpu, oracle_lib, table):
     got = outs.cpu().numpy()
     for i in range(60):
         assert max_rel(got[i], want[i % 3]) <= SPECTRUM_RTOL, i
+
+
+def test_calls_while_another_thread_finalizes(gpu):
+    """rg_finalize waits for one-shot calls of other threads, and no plan is kept whose tables it has
+    freed.  In a process of its own: plans of other tests end with rg_finalize."""
+    code = """
+import ctypes, threading
+import numpy as np, torch
+from ragnar_gb300 import capi
+L = capi.lib()
+capi.check(L.rg_init(0))
+dev = torch.device("cuda:0")
+bins = np.logspace(-2, 7, 100).astype(np.float32)
+g = torch.logspace(0.1, 4, 500, device=dev)
+f, one = g ** -2.5, torch.ones_like(g)
+zero = torch.zeros_like(g)
+prt = capi.particles([g, zero, zero], b=[zero, zero, one], w=f)
+torch.cuda.synchronize()
+def spectra():
+    out = torch.empty((2, 100), device=dev)
+    s = torch.cuda.Stream(dev)
+    s.wait_stream(torch.cuda.current_stream(dev))
+    capi.check(L.rg_synchrotron_spectrum_from_dist(g.data_ptr(), f.data_ptr(), 500, 1, bins.ctypes.data, 100, 1.0, 1.0,
+                                                   out[0].data_ptr(), s.cuda_stream))
+    capi.check(L.rg_synchrotron_spectrum(ctypes.byref(prt), bins.ctypes.data, 100, 1.0, 1.0, 1.0, out[1].data_ptr(),
+                                         s.cuda_stream))
+    s.synchronize()
+    return out.cpu().numpy()
+want = spectra()
+bad, stop = [], threading.Event()
+def work():
+    try:
+        torch.cuda.set_device(0)
+        while not stop.is_set():
+            if not np.allclose(spectra(), want, rtol=1e-6, atol=0.0):
+                bad.append("differs")
+    except Exception as e:
+        bad.append(repr(e))
+threads = [threading.Thread(target=work) for _ in range(2)]
+for t in threads: t.start()
+for _ in range(30):
+    spectra()
+    capi.check(L.rg_finalize())
+stop.set()
+for t in threads: t.join()
+assert not bad, bad[:3]
+assert np.allclose(spectra(), want, rtol=1e-6, atol=0.0)
+print("done")
+"""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", code], cwd=root, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and r.stdout.strip().endswith("done"), r.stdout + r.stderr
