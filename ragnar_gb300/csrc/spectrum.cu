@@ -963,8 +963,9 @@ namespace rg {
     // scalars).  Particle plans stay in the map (at most kParticlePlans).  A plan of
     // rg_synchrotron_spectrum_from_dist, which returns when its result is there, is taken out of the
     // list while a call uses it, so that calls of several threads or streams never share one (at
-    // most kDistPlans idle ones): making it anew costs eight allocations and five copies.
-    constexpr std::size_t kParticlePlans = 32, kDistPlans = 8;
+    // most kDistPlans idle ones of kDistBytes together): making it anew costs eight allocations and
+    // five copies.  A plan's partial rows take 1.3 MB per 512 bins.
+    constexpr std::size_t kParticlePlans = 32, kDistPlans = 8, kDistBytes = std::size_t(64) << 20;
     using PlanKey = std::tuple<int, std::vector<float>, float, float, float>;
 
     // A kept particle plan.  Its callers share its tables, so its runs are ordered on the GPU: a run on
@@ -1016,6 +1017,11 @@ namespace rg {
       std::map<PlanKey, std::unique_ptr<ParticlePlan>>      particles;
       std::vector<std::pair<PlanKey, rg_spectrum_plan*>>    dist; // idle, most recent last
     };
+
+    // Device memory of a distribution plan (its partial rows, nearly).
+    std::size_t dist_bytes(const rg_spectrum_plan* pl) {
+      return sizeof(double) * pl->partial_cap + 16 * sizeof(float) * static_cast<std::size_t>(pl->nslices) * kSliceBins;
+    }
 
     PlanCaches& plan_caches() { // never destroyed: its plans are device memory (rg_finalize frees them)
       static auto* c = new PlanCaches();
@@ -1504,16 +1510,25 @@ int rg_synchrotron_spectrum_from_dist(const float* gbeta, const float* f, int32_
     rg_spectrum_plan_destroy(pl);
     return st;
   }
-  rg_spectrum_plan* old = nullptr;
-  {
+  std::vector<rg_spectrum_plan*> old; // destroyed outside the lock
+  if (rg::dist_bytes(pl) > rg::kDistBytes) {
+    old.push_back(pl);
+  } else {
     std::lock_guard<std::mutex> lock(c.mu);
-    if (c.dist.size() >= rg::kDistPlans) {
-      old = c.dist.front().second;
+    c.dist.emplace_back(std::move(key), pl);
+    std::size_t bytes = 0;
+    for (const auto& kv : c.dist) {
+      bytes += rg::dist_bytes(kv.second);
+    }
+    while (c.dist.size() > rg::kDistPlans || bytes > rg::kDistBytes) {
+      old.push_back(c.dist.front().second);
+      bytes -= rg::dist_bytes(c.dist.front().second);
       c.dist.erase(c.dist.begin());
     }
-    c.dist.emplace_back(std::move(key), pl);
   }
-  rg_spectrum_plan_destroy(old);
+  for (rg_spectrum_plan* q : old) {
+    rg_spectrum_plan_destroy(q);
+  }
   return RG_OK;
 }
 

@@ -618,3 +618,26 @@ print("done")
     root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
     r = subprocess.run([sys.executable, "-c", code], cwd=root, capture_output=True, text=True, timeout=300)
     assert r.returncode == 0 and r.stdout.strip().endswith("done"), r.stdout + r.stderr
+
+
+def test_kept_distribution_plans_are_small(gpu):
+    """The plan of a call over very many bins is given back, not kept for the next call with its bins."""
+    g = torch.logspace(0.1, 4, 500, device=gpu)
+    f = g**-2.5
+
+    def call(nbins):
+        bins = np.logspace(-2, 7, nbins).astype(np.float32)
+        out = torch.empty(nbins, device=gpu)
+        capi.check(capi.lib().rg_synchrotron_spectrum_from_dist(g.data_ptr(), f.data_ptr(), 500, 1, bins.ctypes.data, nbins,
+                                                                1.0, 1.0, out.data_ptr(), 0))
+        return out
+
+    call(200000)
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info(gpu)[0]
+    a = call(300000)  # 590 slices: 0.7 GB of partial rows
+    for n in range(1000, 25000, 1000):
+        call(n)
+    torch.cuda.synchronize()
+    assert free - torch.cuda.mem_get_info(gpu)[0] <= 128 << 20
+    assert torch.equal(a, call(300000)) and bool(torch.isfinite(a).all())
