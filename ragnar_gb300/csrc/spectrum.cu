@@ -968,16 +968,25 @@ namespace rg {
     constexpr std::size_t kParticlePlans = 32, kDistPlans = 8, kDistBytes = std::size_t(64) << 20;
     using PlanKey = std::tuple<int, std::vector<float>, float, float, float>;
 
-    // A kept particle plan.  Its callers share its tables, so its runs are ordered on the GPU: a run on
-    // another stream waits for the last one.
+    // A kept particle plan.  Its callers share its tables, so one of them queues its run at a time (others
+    // go on with their own plans), and its runs are ordered on the GPU: a run on another stream waits
+    // for the last one.
     struct ParticlePlan {
-      rg_spectrum_plan* plan = nullptr;
+      std::mutex        mu;             // held while the plan is made and while a run is queued
+      rg_spectrum_plan* plan = nullptr; // made by the first call
       cudaEvent_t       done = nullptr; // after the last run, where that was not on the null stream
       cudaStream_t      last = nullptr;
       bool              used = false;
 
-      ~ParticlePlan() {
-        rg_spectrum_plan_destroy(plan);
+      ~ParticlePlan() { // by the last of its callers if it was dropped from the map meanwhile
+        if (plan) {
+          int cur = 0;
+          cudaGetDevice(&cur);
+          cudaSetDevice(plan->device);
+          cudaDeviceSynchronize();
+          rg_spectrum_plan_destroy(plan);
+          cudaSetDevice(cur);
+        }
         if (done) {
           cudaEventDestroy(done);
         }
@@ -1014,7 +1023,7 @@ namespace rg {
 
     struct PlanCaches {
       std::mutex                                            mu;
-      std::map<PlanKey, std::unique_ptr<ParticlePlan>>      particles;
+      std::map<PlanKey, std::shared_ptr<ParticlePlan>>      particles;
       std::vector<std::pair<PlanKey, rg_spectrum_plan*>>    dist; // idle, most recent last
     };
 
@@ -1033,9 +1042,6 @@ namespace rg {
   void free_plan_caches() {
     PlanCaches&                 c = plan_caches();
     std::lock_guard<std::mutex> lock(c.mu);
-    if (!c.particles.empty()) {
-      cudaDeviceSynchronize();
-    }
     c.particles.clear();
     for (auto& kv : c.dist) {
       rg_spectrum_plan_destroy(kv.second);
@@ -1421,19 +1427,41 @@ int rg_synchrotron_spectrum(const rg_particles* p, const float* bins, int32_t nb
   rg::PlanKey                 key { dev, std::vector<float>(bins, bins + nbins), B0, g_syn, e_syn_at_g_syn };
   rg::PlanCaches&             c = rg::plan_caches();
   std::shared_lock<std::shared_mutex> life(rg::library_mutex());
-  std::lock_guard<std::mutex> lock(c.mu); // also while the run's launches are queued: they share the plan's tables
-  auto                        it = c.particles.find(key);
-  if (it == c.particles.end()) {
-    auto e = std::make_unique<rg::ParticlePlan>();
-    RG_TRY(rg_spectrum_plan_create(bins, nbins, B0, g_syn, e_syn_at_g_syn, RG_TABLE_REFERENCE, &e->plan));
-    RG_CUDA_TRY(cudaEventCreateWithFlags(&e->done, cudaEventDisableTiming));
-    if (c.particles.size() >= rg::kParticlePlans) {
-      RG_CUDA_TRY(cudaDeviceSynchronize());
-      c.particles.clear();
+  std::shared_ptr<rg::ParticlePlan> e;
+  {
+    std::lock_guard<std::mutex> lock(c.mu);
+    auto&                       slot = c.particles[key];
+    if (!slot) {
+      slot = std::make_shared<rg::ParticlePlan>();
     }
-    it = c.particles.emplace(std::move(key), std::move(e)).first;
+    e = slot;
   }
-  return rg::run_ordered(*it->second, p, out, static_cast<cudaStream_t>(stream));
+  std::lock_guard<std::mutex> lock(e->mu);
+  if (!e->plan) {
+    int st = RG_OK;
+    if (!e->done) {
+      const cudaError_t err = cudaEventCreateWithFlags(&e->done, cudaEventDisableTiming);
+      st = err == cudaSuccess ? RG_OK : rg::cuda_error(err, "rg_synchrotron_spectrum");
+    }
+    if (st == RG_OK) {
+      st = rg_spectrum_plan_create(bins, nbins, B0, g_syn, e_syn_at_g_syn, RG_TABLE_REFERENCE, &e->plan);
+    }
+    std::map<rg::PlanKey, std::shared_ptr<rg::ParticlePlan>> dropped; // destroyed outside the caches' lock
+    std::lock_guard<std::mutex>                              caches(c.mu);
+    const auto                                               it = c.particles.find(key);
+    const bool own = it != c.particles.end() && it->second == e;
+    if (st != RG_OK) {
+      if (own) {
+        c.particles.erase(it);
+      }
+      return st;
+    }
+    if (own && c.particles.size() > rg::kParticlePlans) {
+      dropped.swap(c.particles);
+      c.particles.emplace(key, e);
+    }
+  }
+  return rg::run_ordered(*e, p, out, static_cast<cudaStream_t>(stream));
 }
 
 int rg_dist_run(const rg_spectrum_plan* plan, const float* gbeta, const float* f, int32_t ng, float* out,

@@ -19,6 +19,7 @@ import ctypes
 import os
 import subprocess
 import sys
+import threading
 
 import numpy as np
 import pytest
@@ -641,3 +642,35 @@ def test_kept_distribution_plans_are_small(gpu):
     torch.cuda.synchronize()
     assert free - torch.cuda.mem_get_info(gpu)[0] <= 128 << 20
     assert torch.equal(a, call(300000)) and bool(torch.isfinite(a).all())
+
+
+def test_one_shot_spectra_from_threads(gpu, oracle_lib, table):
+    """Threads with streams of their own and more sets of bins between them than plans are kept: a plan
+    that is dropped while another thread uses it lives until that call is done."""
+    P    = particles(3001, seed=3, bfield="iso", weights=True)
+    sets = [oracle_lib.logspace(1e-2 * (1.0 + 0.01 * i), 1e6, 40 + i) for i in range(40)]
+    want = [oracle_lib.sync_spectrum_f64(P, b, 1.0, 1.0, 1.0, table) for b in sets]
+    T, prt = to_device(P, gpu)
+    torch.cuda.synchronize()
+    errors = []
+
+    def work(k):
+        try:
+            torch.cuda.set_device(0)
+            s = torch.cuda.Stream(gpu)
+            for i in np.random.default_rng(k).integers(0, 40, 120):
+                with torch.cuda.stream(s):
+                    out = torch.full((len(sets[i]),), -1.0, device=gpu)
+                capi.check(capi.lib().rg_synchrotron_spectrum(ctypes.byref(prt), sets[i].ctypes.data, len(sets[i]), 1.0,
+                                                              1.0, 1.0, out.data_ptr(), s.cuda_stream))
+                s.synchronize()
+                assert max_rel(out.cpu().numpy(), want[i]) <= SPECTRUM_RTOL, i
+        except Exception as e:  # noqa: BLE001
+            errors.append(repr(e))
+
+    threads = [threading.Thread(target=work, args=(k,)) for k in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors, errors[:2]
