@@ -750,11 +750,12 @@ namespace rg {
     int             nan_index = 0, cell_shift = 0, cell_base = 0, ncells = 0;
   };
 
-  // Thresholds and cell table of a bin set on the current device.
+  // Thresholds and cell table of a bin set on the current device.  The caller holds thr_mutex until the
+  // kernel that reads them is queued: another thread's bin set may evict this one, which waits for the
+  // device and frees it.
   int device_thresholds(const float* bins, int n, bool fourvel, DeviceBins& out) {
     int device = 0;
     RG_CUDA_TRY(cudaGetDevice(&device));
-    std::lock_guard<std::mutex> lock(thr_mutex());
     auto&                       cache = thr_cache();
     auto                        it    = cache.begin();
     for (; it != cache.end(); ++it) {
@@ -857,7 +858,8 @@ int rg_energy_distribution(const float* ux, const float* uy, const float* uz, in
     return rg::set_error(RG_ERR_UNSUPPORTED, "energyDistribution supports at most 4096 bins");
   }
   auto           s = static_cast<cudaStream_t>(stream);
-  rg::DeviceBins db;
+  std::lock_guard<std::mutex> lock(rg::thr_mutex()); // see device_thresholds
+  rg::DeviceBins              db;
   RG_TRY(rg::device_thresholds(bins, nbins, fourvel != 0, db));
 
   rg::DeviceContext* ctx = nullptr;

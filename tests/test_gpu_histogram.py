@@ -8,6 +8,7 @@ above the top bin, NaN and infinity), unaligned and ragged sizes.
 from __future__ import annotations
 
 import ctypes
+import threading
 
 import numpy as np
 import pytest
@@ -230,3 +231,37 @@ def test_without_counts(gpu, oracle_lib, many, n, offset, nb, log_spaced, fourve
     fin = np.isfinite(h64)
     assert np.array_equal(np.isnan(h), np.isnan(h64)) and np.array_equal(np.isinf(h), np.isinf(h64))
     assert np.all(np.abs(h[fin] - h64[fin]) <= 1e-6 * h64[fin])
+
+
+def test_many_bin_sets_from_threads(gpu, oracle_lib):
+    """Threads whose bin sets evict each other's thresholds."""
+    P = particles(40001, seed=21, umax=3e3)
+    u = [P[k] for k in ("ux", "uy", "uz")]
+    sets = [oracle_lib.logspace(1e-2, 1e3 + i, n) for i, n in enumerate([400, 1000, 200, 100, 300] * 6)]
+    want = [oracle_lib.energy_distribution(*u, b, True, True)[2] for b in sets]
+    T = [torch.from_numpy(c).to(gpu) for c in u]
+    torch.cuda.synchronize()
+    errors = []
+
+    def work(k):
+        try:
+            torch.cuda.set_device(0)
+            s = torch.cuda.Stream(gpu)
+            for i in np.random.default_rng(k).integers(0, len(sets), 60):
+                n = len(sets[i])
+                with torch.cuda.stream(s):
+                    hist, cnt = torch.full((n,), -1.0, device=gpu), torch.full((n,), -1, device=gpu, dtype=torch.int64)
+                capi.check(capi.lib().rg_energy_distribution(T[0].data_ptr(), T[1].data_ptr(), T[2].data_ptr(), 40001,
+                                                             sets[i].ctypes.data, n, 1, 1, hist.data_ptr(), cnt.data_ptr(),
+                                                             s.cuda_stream))
+                s.synchronize()
+                np.testing.assert_array_equal(cnt.cpu().numpy().astype(np.uint64), want[i].astype(np.uint64))
+        except BaseException as e:  # noqa: BLE001
+            errors.append(repr(e)[:500])
+
+    threads = [threading.Thread(target=work, args=(k,)) for k in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors, errors[:2]
