@@ -309,6 +309,11 @@ namespace rg {
              sizeof(float) * kLaneCopies * static_cast<size_t>(nb) * warps + 16;
     }
 
+    // Shared memory of the atomics kernel.
+    size_t atomics_smem(int nb, int ncells) {
+      return (((2 + kSumCopies) * sizeof(float) * nb + 15) & ~size_t(15)) + sizeof(float2) * nb + sizeof(uint16_t) * (ncells + 1);
+    }
+
     // Warps of the lane kernel, or 0 where the atomics are faster: with fewer than ten warps on an SM
     // latencies are not hidden, and clearing and summing the copies takes as long as a million
     // particles.  Per call, sums of |u|^-1 over log bins, lanes against atomics: 3.3e7 particles x 25
@@ -878,11 +883,12 @@ int rg_energy_distribution(const float* ux, const float* uy, const float* uz, in
     smem = rg::lane_smem(nbins, db.lncells, warps);
     G    = ctx->sms * std::max(1, std::min(static_cast<int>(rg::kLaneSmem / smem), 2048 / (32 * rg::kLaneMaxWarps)));
   } else {
-    smem = (((2 + rg::kSumCopies) * sizeof(float) * nbins + 15) & ~size_t(15)) + sizeof(float2) * nbins +
-           sizeof(uint16_t) * (db.ncells + 1);
-    if (smem > 48 * 1024) {
-      RG_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
-    }
+    smem = rg::atomics_smem(nbins, db.ncells);
+    // the limit once for all sizes: set to a call's own size it may be lowered by another thread's call
+    // before the launch
+    static std::atomic<uint64_t> configured[3];
+    RG_CUDA_TRY(rg::ensure_max_dynamic_smem(kernel, static_cast<int>(rg::atomics_smem(rg::kHistMaxBins, rg::kMaxCells)),
+                                            configured[!need_sum ? 0 : need_count ? 1 : 2]));
     int per_sm = 0;
     RG_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, rg::kHistThreads, smem));
     per_sm = std::max(1, std::min(per_sm, 8));

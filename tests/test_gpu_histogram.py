@@ -234,10 +234,10 @@ def test_without_counts(gpu, oracle_lib, many, n, offset, nb, log_spaced, fourve
 
 
 def test_many_bin_sets_from_threads(gpu, oracle_lib):
-    """Threads whose bin sets evict each other's thresholds."""
+    """Threads whose bin sets evict each other's thresholds, of sizes whose shared memory differs."""
     P = particles(40001, seed=21, umax=3e3)
     u = [P[k] for k in ("ux", "uy", "uz")]
-    sets = [oracle_lib.logspace(1e-2, 1e3 + i, n) for i, n in enumerate([400, 1000, 200, 100, 300] * 6)]
+    sets = [oracle_lib.logspace(1e-2, 1e3 + i, n) for i, n in enumerate([1400, 4000, 2000, 100, 300] * 6)]
     want = [oracle_lib.energy_distribution(*u, b, True, True)[2] for b in sets]
     T = [torch.from_numpy(c).to(gpu) for c in u]
     torch.cuda.synchronize()
