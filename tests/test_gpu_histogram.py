@@ -265,3 +265,31 @@ def test_many_bin_sets_from_threads(gpu, oracle_lib):
     for t in threads:
         t.join()
     assert not errors, errors[:2]
+
+
+@pytest.mark.parametrize("nb", [200, 300])
+def test_sums_carried_over_flushes(gpu, oracle_lib, nb):
+    """Enough particles that the per-lane copies of the bins are flushed inside the loop (512 particles a
+    lane: 4e7 at 200 bins, 2.5e7 at 300), twice and not at its end: against the sums in FP64."""
+    n = 90_000_003
+    g = torch.Generator(device=gpu).manual_seed(nb)
+    mag = 10.0 ** (4.0 * torch.rand(n, device=gpu, generator=g) - 1.5)
+    u = [mag * 0.6, mag * 0.48, mag * 0.64]
+    bins = oracle_lib.logspace(1e-2, 1e3, nb)
+    L = capi.lib()
+    hist, ref, cnt = torch.empty(nb, device=gpu), torch.empty(nb, device=gpu), torch.empty(nb, device=gpu, dtype=torch.int64)
+    capi.check(L.rg_energy_distribution(u[0].data_ptr(), u[1].data_ptr(), u[2].data_ptr(), n, bins.ctypes.data, nb, 1, 1,
+                                        hist.data_ptr(), None, 0))
+    torch.cuda.synchronize()
+    # the same bins by counts (the other kernel), in runs that it sums in one flush of a block
+    want = torch.zeros(nb, device=gpu, dtype=torch.float64)
+    total = torch.zeros(nb, device=gpu, dtype=torch.int64)
+    for a in range(0, n, 1 << 20):
+        m = min(1 << 20, n - a)
+        capi.check(L.rg_energy_distribution(u[0][a:].data_ptr(), u[1][a:].data_ptr(), u[2][a:].data_ptr(), m,
+                                            bins.ctypes.data, nb, 1, 1, ref.data_ptr(), cnt.data_ptr(), 0))
+        torch.cuda.synchronize()
+        want += ref.double()
+        total += cnt
+    assert int(total.sum()) == n
+    assert torch.all((hist.double() - want).abs() <= 1e-6 * want)
