@@ -239,6 +239,7 @@ namespace rg {
       double*         acc;      // [nseg][nslices][kSliceBins], cleared by the deposit
       unsigned*       done;     // [nseg][nslices] blocks finished, cleared by the deposit
       float*          out;      // nseg x nbins
+      f2              nz;       // of product2
     };
 
     constexpr int kFinWarps = 8;
@@ -509,9 +510,9 @@ namespace rg {
             const float4 U = Us[b.pos], Lo = buf[b.pos];
             // pairs (U, L): x = M1 - (Dl, Dl - 1) M0, then c0 M0 + c1 x
             const ff2 M0 { pack2(U.x, Lo.x), pack2(U.z, Lo.z) }, M1 { pack2(U.y, Lo.y), pack2(U.w, Lo.w) };
-            const ff2 x = ff_add2(M1, ff_mul2(ff2 { pack2(b.nDh, b.mDh), pack2(b.nDl, b.mDl) }, M0));
+            const ff2 x = ff_add2(M1, ff_mul2(ff2 { pack2(b.nDh, b.mDh), pack2(b.nDl, b.mDl) }, M0, r.nz));
             const ff2 k0 { pack2(ku.x, kl.x), pack2(ku.y, kl.y) }, k1 { pack2(ku.z, kl.z), pack2(ku.w, kl.w) };
-            const ff2 y = ff_add2(ff_mul2(k0, M0), ff_mul2(k1, x));
+            const ff2 y = ff_add2(ff_mul2(k0, M0, r.nz), ff_mul2(k1, x, r.nz));
             float     h0, h1, l0, l1;
             unpack2(y.hi, h0, h1);
             unpack2(y.lo, l0, l1);
@@ -915,6 +916,7 @@ namespace rg {
     r.acc      = pl->d_msum;
     r.done     = reinterpret_cast<unsigned*>(pl->d_msum + pl->msum_cap * kSliceBins);
     r.out      = out;
+    r.nz       = negative_zeros();
     const int    rows   = nseg * pl->nslices;
     const int    nv     = max_valid(pl);
     const size_t smem   = finish_smem(nv, r.nseg_tab);

@@ -191,6 +191,7 @@ namespace rg {
       unsigned*       done;  // [nseg] blocks finished, cleared by the deposit
       int             acc_stride;
       float*          out;   // nseg x nbins
+      f2              nz;    // of product2
     };
 
     constexpr int kFinCells = 16; // cells per block: two per warp
@@ -342,7 +343,7 @@ namespace rg {
             f2 p[4], e[4];
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
-              p[j] = mul2(c[j], h[j]);
+              p[j] = product2(c[j], h[j], r.nz);
               e[j] = sub2(mul2(c[j], l[j]), fma2(neg2(c[j]), h[j], p[j]));
             }
             const ff2 s01 = two_sum2(p[0], p[1]), s23 = two_sum2(p[2], p[3]);
@@ -474,13 +475,13 @@ namespace rg {
     // dL/dw and dL/du of two particles without an E field, as particle_gradient (same formulas,
     // the cross product in double-floats); bit j of the result: particle j is done, otherwise it
     // takes the scalar form (ranges in which the reciprocals below would leave FP32's normal numbers).
-    __device__ __forceinline__ unsigned gradient2(const f2 (&v)[kComps], float amp, f2 R1, f2 R2, f2& gw, f2 (&gu)[3]) {
+    __device__ __forceinline__ unsigned gradient2(const f2 (&v)[kComps], float amp, f2 R1, f2 R2, f2& gw, f2 (&gu)[3], f2 nz) {
       const f2  u[3] = { v[0], v[1], v[2] }, B[3] = { v[6], v[7], v[8] };
       const f2  n[3] = { neg2(u[0]), neg2(u[1]), neg2(u[2]) };
       const f2  G    = fma2(u[0], u[0], fma2(u[1], u[1], fma2(u[2], u[2], set2(1.0f))));
-      const f2  c[3] = { diff_of_products2(u[1], n[1], B[2], u[2], n[2], B[1]).hi,
-                         diff_of_products2(u[2], n[2], B[0], u[0], n[0], B[2]).hi,
-                         diff_of_products2(u[0], n[0], B[1], u[1], n[1], B[0]).hi };
+      const f2  c[3] = { diff_of_products2(u[1], n[1], B[2], u[2], n[2], B[1], nz).hi,
+                         diff_of_products2(u[2], n[2], B[0], u[0], n[0], B[2], nz).hi,
+                         diff_of_products2(u[0], n[0], B[1], u[1], n[1], B[0], nz).hi };
       const f2  W    = fma2(c[2], c[2], fma2(c[1], c[1], mul2(c[0], c[0])));
       const f2  nc[3] = { neg2(c[0]), neg2(c[1]), neg2(c[2]) };
       // d W / du / 2 = B x c
@@ -604,7 +605,7 @@ namespace rg {
         unsigned done = 0;
         if (!kE) {
           f2 gw2, gu2[3];
-          done = gradient2(v, m.fp.amp, pack2(R1[0], R1[1]), pack2(R2[0], R2[1]), gw2, gu2);
+          done = gradient2(v, m.fp.amp, pack2(R1[0], R1[1]), pack2(R2[0], R2[1]), gw2, gu2, m.log.nz);
           unpack2(gw2, gw[0], gw[1]);
 #pragma unroll
           for (int d = 0; d < 3; ++d) {
@@ -823,6 +824,7 @@ namespace rg {
     r.acc_stride = pl->nslices * kSliceBins;
     r.done       = reinterpret_cast<unsigned*>(pl->d_msum + pl->msum_cap * kSliceBins);
     r.out        = out;
+    r.nz         = negative_zeros();
     static std::atomic<uint64_t> configured { 0 };
     RG_CUDA_TRY(ensure_max_dynamic_smem(smooth_finish_kernel, static_cast<int>(sizeof(float4) * kSmoothMaxSegments), configured));
     smooth_finish_kernel<<<dim3((pl->sm_cells + kFinCells - 1) / kFinCells, nseg), kPairThreads,

@@ -64,9 +64,9 @@ namespace rg {
     return r;
   }
 
-  // The compiler contracts a packed product that only one packed sum reads into an fma, .rn or not
-  // (measured: 489284 of 1048576 sums of three squares differ from the separately rounded ones).  A
-  // product whose rounding matters below is read again for its remainder, which keeps it a product.
+  // The compiler may contract a packed product and a packed sum into an fma, .rn or not (measured:
+  // 489284 of 1048576 sums of three squares differ from the separately rounded ones).  A product whose
+  // own rounding a sum takes for granted is a product2.
   __device__ __forceinline__ f2 mul2(f2 a, f2 b) {
     f2 r;
     asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
@@ -77,6 +77,16 @@ namespace rg {
     f2 r;
     asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
     return r;
+  }
+
+  // a b, rounded: nz is a pair of -0 that the kernel gets as a parameter, so that the compiler sees an
+  // fma with an unknown addend and has nothing to contract.
+  __device__ __forceinline__ f2 product2(f2 a, f2 b, f2 nz) {
+    return fma2(a, b, nz);
+  }
+
+  inline f2 negative_zeros() {
+    return { 0x8000000080000000ull };
   }
 
   // a - b: one rounding, as a subtraction
@@ -117,27 +127,27 @@ namespace rg {
 
   // a b - c d with na = -a and nc = -c, as a normalised pair: when the products nearly cancel,
   // their remainders carry the whole value.
-  __device__ __forceinline__ ff2 diff_of_products2(f2 a, f2 na, f2 b, f2 c, f2 nc, f2 d) {
-    const f2  p = mul2(a, b), q = mul2(nc, d);
+  __device__ __forceinline__ ff2 diff_of_products2(f2 a, f2 na, f2 b, f2 c, f2 nc, f2 d, f2 nz) {
+    const f2  p = product2(a, b, nz), q = product2(nc, d, nz);
     const f2  e = add2(fma2(na, b, p), fma2(c, d, q)); // -(remainder of p + remainder of q)
     const ff2 r = two_sum2(p, q);
     return fast_two_sum2(r.hi, sub2(r.lo, e));
   }
 
   // a^2 of a pair: hi = a.hi^2 and the negative of everything below it
-  __device__ __forceinline__ void square2(ff2 a, f2& hi, f2& nlo) {
-    hi  = mul2(a.hi, a.hi);
+  __device__ __forceinline__ void square2(ff2 a, f2& hi, f2& nlo, f2 nz) {
+    hi  = product2(a.hi, a.hi, nz);
     nlo = fma2(mul2(a.hi, set2(-2.0f)), a.lo, fma2(neg2(a.hi), a.hi, hi));
   }
 
   template <bool kE>
-  __device__ __forceinline__ Kin2 kinematics2(const f2 (&v)[kComps]) {
+  __device__ __forceinline__ Kin2 kinematics2(const f2 (&v)[kComps], f2 nz) {
     const f2 ux = v[0], uy = v[1], uz = v[2];
-    const f2 nx = neg2(ux), ny = neg2(uy), nz = neg2(uz);
+    const f2 nx = neg2(ux), ny = neg2(uy), mz = neg2(uz);
     Kin2     k;
     {
-      const f2  x2 = mul2(ux, ux), y2 = mul2(uy, uy), z2 = mul2(uz, uz);
-      const f2  e  = add2(add2(fma2(nx, ux, x2), fma2(ny, uy, y2)), fma2(nz, uz, z2));
+      const f2  x2 = product2(ux, ux, nz), y2 = product2(uy, uy, nz), z2 = product2(uz, uz, nz);
+      const f2  e  = add2(add2(fma2(nx, ux, x2), fma2(ny, uy, y2)), fma2(mz, uz, z2));
       const ff2 s  = two_sum2(x2, y2);
       const ff2 t  = two_sum2(s.hi, z2);
       const ff2 g  = two_sum2(set2(1.0f), t.hi);
@@ -145,14 +155,14 @@ namespace rg {
       k.nGl        = sub2(e, add2(add2(s.lo, t.lo), g.lo));
     }
     const f2 bx = v[6], by = v[7], bz = v[8];
-    ff2      cx = diff_of_products2(uy, ny, bz, uz, nz, by);
-    ff2      cy = diff_of_products2(uz, nz, bx, ux, nx, bz);
-    ff2      cz = diff_of_products2(ux, nx, by, uy, ny, bx);
+    ff2      cx = diff_of_products2(uy, ny, bz, uz, mz, by, nz);
+    ff2      cy = diff_of_products2(uz, mz, bx, ux, nx, bz, nz);
+    ff2      cz = diff_of_products2(ux, nx, by, uy, ny, bx, nz);
     if (!kE) {
       f2 hx, hy, hz, lx, ly, lz;
-      square2(cx, hx, lx);
-      square2(cy, hy, ly);
-      square2(cz, hz, lz);
+      square2(cx, hx, lx, nz);
+      square2(cy, hy, ly, nz);
+      square2(cz, hz, lz, nz);
       const ff2 s = two_sum2(hx, hy);
       const ff2 t = two_sum2(s.hi, hz);
       k.Wh        = t.hi;
@@ -168,23 +178,23 @@ namespace rg {
     const f2 gl = mul2(sub2(fma2(neg2(gh), gh, k.Gh), k.nGl), mul2(y, set2(0.5f)));
     const f2 ng = neg2(gh);
     auto     term = [&](f2 e, ff2 c) { // gamma e + c
-      const f2 p = mul2(gh, e);
+      const f2 p = product2(gh, e, nz);
       return ff_add2(ff2 { p, sub2(mul2(gl, e), fma2(ng, e, p)) }, c);
     };
     cx = term(ex, cx);
     cy = term(ey, cy);
     cz = term(ez, cz);
     // u.E
-    const f2  px = mul2(ux, ex), py = mul2(uy, ey), pz = mul2(uz, ez);
-    const f2  e  = add2(add2(fma2(nx, ex, px), fma2(ny, ey, py)), fma2(nz, ez, pz));
+    const f2  px = product2(ux, ex, nz), py = product2(uy, ey, nz), pz = product2(uz, ez, nz);
+    const f2  e  = add2(add2(fma2(nx, ex, px), fma2(ny, ey, py)), fma2(mz, ez, pz));
     const ff2 s  = two_sum2(px, py);
     const ff2 t  = two_sum2(s.hi, pz);
     const ff2 d  = fast_two_sum2(t.hi, sub2(add2(s.lo, t.lo), e));
     f2        hx, hy, hz, hd, lx, ly, lz, ld;
-    square2(cx, hx, lx);
-    square2(cy, hy, ly);
-    square2(cz, hz, lz);
-    square2(d, hd, ld);
+    square2(cx, hx, lx, nz);
+    square2(cy, hy, ly, nz);
+    square2(cz, hz, lz, nz);
+    square2(d, hd, ld, nz);
     const ff2 a = two_sum2(hx, hy);
     const ff2 b = two_sum2(a.hi, hz);
     const ff2 w = two_sum2(b.hi, neg2(hd));
@@ -210,6 +220,7 @@ namespace rg {
     int64_t        Cfx;    // round(S ln 2)
     int            fx;
     const int64_t* table;  // round(S ln c), kLogEntries; then the constants of stand_in
+    f2             nz;     // of product2
   };
 
   inline void fill_log_params(const rg_spectrum_plan* pl, LogParams& g) {
@@ -218,6 +229,7 @@ namespace rg {
     g.Cfx   = pl->log_Cfx;
     g.fx    = pl->log_fx;
     g.table = pl->d_logt;
+    g.nz    = negative_zeros();
   }
 
   // What a deposit reads, with a stride of 0, for a particle stream that is not given: zero field,
@@ -265,7 +277,7 @@ namespace rg {
   template <bool kE>
   __device__ __forceinline__ Place2 place2(const f2 (&v)[kComps], const FusedParams& p, const LogParams& g,
                                            const int64_t* logt, int64_t Pmin, int64_t Pmax, int64_t L) {
-    const Kin2 k = kinematics2<kE>(v);
+    const Kin2 k = kinematics2<kE>(v, g.nz);
     // X = G W = xh - nxl
     const f2 nG  = neg2(k.Gh);
     const f2 xh  = mul2(k.Gh, k.Wh);
@@ -309,7 +321,7 @@ namespace rg {
     const f2 q   = mul2(xh, yy);
     const f2 mt  = fma2(nxl, yy, fma2(xh, nyy, q)); // -(low part of X y + remainder of q)
     const f2 e   = fma2(mt, yy, fma2(q, nyy, set2(1.0f)));
-    const f2 s0  = mul2(k.Wh, yy);
+    const f2 s0  = product2(k.Wh, yy, g.nz);
     const f2 u   = fma2(mul2(s0, set2(0.5f)), e, mul2(k.Wl, yy));
     const f2 chi = add2(s0, sub2(u, fma2(k.Wh, nyy, s0)));
     const f2 A   = mul2(mul2(chi, set2(p.amp)), v[9]);
@@ -492,8 +504,8 @@ namespace rg {
     return e >= 1 ? r : make_float2(0.0f, 0.0f);
   }
 
-  __device__ __forceinline__ ff2 ff_mul2(ff2 a, ff2 b) {
-    const f2 p = mul2(a.hi, b.hi);
+  __device__ __forceinline__ ff2 ff_mul2(ff2 a, ff2 b, f2 nz) {
+    const f2 p = product2(a.hi, b.hi, nz);
     const f2 e = sub2(fma2(a.hi, b.lo, mul2(a.lo, b.hi)), fma2(neg2(a.hi), b.hi, p));
     return fast_two_sum2(p, e);
   }
