@@ -97,6 +97,14 @@ namespace rg {
               sum            = ff_add(sum, ff { v.x, v.y });
             }
             t = static_cast<double>(sum.hi) + static_cast<double>(sum.lo);
+            if (!isfinite(sum.hi)) { // above the float range together, or infinite or NaN: as below
+              t = 0.0;
+#pragma unroll 1
+              for (int w = 0; w < kWarps; ++w) {
+                const float2 v = pairs[(r * kWarps + w) * 32 + lane];
+                t += static_cast<double>(v.x) + static_cast<double>(v.y);
+              }
+            }
           } else {
 #pragma unroll
             for (int w = 0; w < kWarps; ++w) {

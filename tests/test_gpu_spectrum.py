@@ -674,3 +674,18 @@ def test_one_shot_spectra_from_threads(gpu, oracle_lib, table):
     for t in threads:
         t.join()
     assert not errors, errors[:2]
+
+
+def test_short_run_above_the_float_range(gpu, oracle_lib):
+    """Sums that are floats warp by warp but not together, times a photon energy that brings the spectrum
+    back into range."""
+    gb, f = np.ones(32, np.float32), np.full(32, 3e37, np.float32)
+    bins = oracle_lib.logspace(1e-4, 1e-3, 20)
+    table = oracle_lib.tabulate_ffunc()
+    want = oracle_lib.sync_from_dist_f64(gb, f, False, bins, 1.0, 1e-3, table)[0]
+    assert np.max(want / bins) > 3.5e38 and np.max(want) < 1e36
+    g, F = torch.from_numpy(gb).to(gpu), torch.from_numpy(f).to(gpu)
+    out = torch.full((20,), -1.0, device=gpu)
+    capi.check(capi.lib().rg_synchrotron_spectrum_from_dist(g.data_ptr(), F.data_ptr(), 32, 0, bins.ctypes.data, 20, 1.0,
+                                                            1e-3, out.data_ptr(), 0))
+    assert max_rel(out.cpu().numpy(), want) <= SPECTRUM_RTOL
