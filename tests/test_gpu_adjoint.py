@@ -349,3 +349,33 @@ def test_moment_pair_edges(gpu, oracle_lib, n, nbins, efield):
         assert max_rel(S.cpu().numpy(), S64) <= SPECTRUM_RTOL
         got = np.stack([t.cpu().numpy() for t in g]).astype(np.float64)
         assert np.max(np.abs(got - g64) / scale) < 1e-4
+
+
+def test_gradient_of_nearly_parallel_fields(gpu, oracle_lib):
+    """B within 2^-14 of the direction of u: the force is the small difference of products, and its
+    gradient too.  Some twenty FP32 roundings (1.2e-6) and up to ten times that where the two terms of the
+    chain rule nearly cancel: 2e-5 of the largest value, a sixth of what a cross product in FP32 leaves
+    (2^-24 / 2^-14 in each of its components, twice)."""
+    n = 3001
+    rng = np.random.default_rng(17)
+    P = particles(n, seed=17, bfield="iso", weights=True, umax=1e3)
+    u = np.stack([P[k] for k in ("ux", "uy", "uz")]).astype(np.float64)
+    b = u / np.sqrt(np.sum(u * u, axis=0)) * (1.0 + 2.0**-14 * rng.uniform(-1.0, 1.0, (3, n)))
+    P.update({k: b[d].astype(np.float32) for d, k in enumerate(("bx", "by", "bz"))})
+    bins = oracle_lib.logspace(1e-6, 1e4, 200)
+    plan = rt.spectrum_plan(bins)
+    coef, xmin, xmax = plan_table(plan)
+    S64 = oracle_lib.sync_smooth_f64(P, bins, 1.0, 1.0, 1.0, coef, xmin, xmax)
+    gS = 1.0 / np.maximum(S64, 1e-6 * S64.max())
+    gw64, gu64 = oracle_lib.sync_smooth_grad_f64(P, bins, 1.0, 1.0, 1.0, coef, gS, xmin, xmax)
+    T = _device(P, gpu)
+    prt = capi.particles([T["ux"], T["uy"], T["uz"]], b=[T["bx"], T["by"], T["bz"]], w=T["w"], n=n)
+    S, gout = torch.empty(200, device=gpu), torch.from_numpy(gS.astype(np.float32)).to(gpu)
+    g = [torch.full((n,), float("nan"), device=gpu) for _ in range(4)]
+    plan.run(prt, S)
+    plan.adjoint(prt, gout, g[0], g[1:])
+    plan.check()
+    got = np.stack([t.cpu().numpy() for t in g]).astype(np.float64)
+    want = np.vstack([gw64[None], gu64])
+    assert max_rel(S.cpu().numpy(), S64) <= SPECTRUM_RTOL
+    assert np.all(np.max(np.abs(got - want), axis=1) <= 2e-5 * np.max(np.abs(want), axis=1))
