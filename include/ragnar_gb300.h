@@ -237,7 +237,9 @@ int rg_spectrum_run_plain(const rg_spectrum_plan* plan, const rg_particles* p, f
                           void* stream);
 
 /* One-shot drop-in for SynchrotronSpectrum<D> (synchrotron.cpp:107-145): plan
- * (cached by arguments) + run, reference table mode. */
+ * (cached by arguments) + run, reference table mode.  Calls with the same arguments share the
+ * plan, from any thread: their runs are ordered on the GPU, also between streams (a call that a
+ * graph records is ordered by the graph's launches, which must not overlap other calls). */
 int rg_synchrotron_spectrum(const rg_particles* p, const float* bins, int32_t nbins, float B0,
                             float g_syn, float e_syn_at_g_syn, float* out, void* stream);
 

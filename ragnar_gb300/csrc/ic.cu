@@ -44,11 +44,12 @@
 // (deterministic).  Non-positive or non-finite IC bins give 0 (the reference produces NaN
 // there).
 //
-// Measured at 1024 gamma x 1024 soft-photon x 1024 IC bins, back to back on one stream: 54 us a
-// call (67 us with the photons shuffled) against 356 us with every triple evaluated, the largest
+// Measured at 1024 gamma x 1024 soft-photon x 1024 IC bins, back to back on one stream: 47.5 us a
+// call (52 us with the photons shuffled) against 369 us with every triple evaluated, the largest
 // error against FP64 1e-7 against 2.2e-5 (a line of photons at the Klein-Nishina edge).  The
-// kernels: terms 9 us, sums 10 us (latency of one tile), pairs 21 us (issue: ~250 instructions
-// a pair, 40 of them the search), the direct kernel's early return 2.5 us, reduction 4.5 us.
+// kernels: terms 8 us, sums 9.5 us (FP64 pipe of four SMs), pairs 23 us (issue and latency: ~340
+// instructions a pair), the direct kernel's early return 4 us, reduction 5 us (under a profiler,
+// serialised).
 #include "moments_common.cuh"
 
 #include <algorithm>
@@ -107,8 +108,10 @@ namespace rg {
     constexpr int kRankMax     = 16384; // photons that are ranked when they are out of order
     constexpr int kRankTile    = 1024; // a multiple of a block's photons
     constexpr int kRankWays    = 4;     // threads that share a photon's comparisons
-    // energies and |weights| of a regular table: far enough from the ends of the float range for
-    // every double-float product of the pair kernel
+    // energies and largest |weight| of a regular table: far enough from the ends of the float range for
+    // every double-float product of the pair kernel.  Small weights need no bound: their products lose
+    // low parts below 2^-126, but no more than the direct kernel's FP32 loses there (weights of 1e-38:
+    // 1.1e-7 against 3.2e-7).
     constexpr float kRegularLo = 1e-30f, kRegularHi = 1e30f;
 
     __device__ __forceinline__ ff ff_div(ff a, ff b) {

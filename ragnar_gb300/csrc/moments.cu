@@ -122,8 +122,8 @@ namespace rg {
     // and need no copies between registers.  28 B per particle (u, B, w).  The grid is what fits
     // at once.  Indices are 32-bit within the launch's window of at most 2^31 particles; streams
     // that are not given read a constant with a stride of 0, so the loads carry no tests.
-    // Measured on 9.9e7 dump particles x 512 bins: 0.88 ms in two launches (1.13e11 particles/s,
-    // 3.2 TB/s) against 1.45 ms for one particle per thread with scalar double-floats, 444
+    // Measured on 9.9e7 dump particles x 512 bins: 0.89 ms in two launches (1.11e11 particles/s,
+    // 3.1 TB/s) against 1.45 ms for one particle per thread with scalar double-floats, 444
     // instructions a particle and two reduction requests; now 171 and one.  Without the
     // reductions it would take 0.65 ms, the reductions alone 0.69 ms: the L2's reduction requests
     // and the loads behind them set its pace.  Also measured: three blocks per SM 0.95 ms, loads
@@ -369,8 +369,8 @@ namespace rg {
     // operations per clock and SM: the FP64 scan and reduce kernels this replaces took 503 and
     // 449 us for 256 spectra of 200 bins (this kernel 124 us, and no memset of 350 MB before the
     // run).  What bounds it is the latency of its chains: rows fetched one ahead take a third buffer, and
-    // with it two blocks fit an SM (146 us) instead of three.  Blocks add their bins' sums in FP64; the last block of a (segment, slice) writes the
-    // spectrum.
+    // with it two blocks fit an SM (146 us) instead of three; the launch bounds keep the registers to
+    // that.  Blocks add their bins' sums in FP64; the last block of a (segment, slice) writes the spectrum.
     template <int C>
     __global__ void __launch_bounds__(kFinThreads, C <= 4 ? 4 : C <= 8 ? 3 : C <= 12 ? 2 : 1) moments_finish_kernel(const __grid_constant__ MomentFinishParams r) {
       extern __shared__ __align__(16) unsigned char smem[];
@@ -864,8 +864,9 @@ namespace rg {
   namespace {
 
     // Blocks per (segment, slice): those with which the waves of `resident` blocks take the fewest rows
-    // of a warp, a block's setup and epilogue counted as kFinSetup rows (256 spectra: 5 blocks each,
-    // 124 us; counted as 6, 3 blocks: 138 us).
+    // of a warp, a block's setup and epilogue counted as kFinSetup rows.  Runs of few particles (counted as
+    // 0 / 1 / 3 rows): 256 spectra x 200 bins 193 / 122 / 128 us, 256 x 512 641 / 368 / 354, 1024 x 100 485 /
+    // 258 / 257, 16 x 512 66 / 44 / 44; from one to four spectra, and 64 x 200, the same with all three.
     constexpr size_t kFinSmSmem = 227 * 1024;
     constexpr int    kFinSetup  = 1;
     int finish_blocks(int rows, int cells, int resident) {

@@ -154,7 +154,7 @@ namespace rg {
   // Stream-ordered scratch of one call, given back by cudaFreeAsync on the same stream.  It comes
   // from a pool of the library's own that keeps up to kScratchKept idle bytes: the device's default
   // pool returns its memory to the driver at every synchronisation, so that a call after one maps
-  // it anew (with the drop-in's arrays from blocks, a 3.3e7-particle histogram 312 -> 138 us).
+  // it anew (with the drop-in's arrays, most of the 200 us that its calls spent on the host).
   constexpr uint64_t kScratchKept = uint64_t(64) << 20;
   int scratch_alloc(void** p, size_t bytes, cudaStream_t s);
   int reference_table(const RefTable** t);

@@ -28,8 +28,8 @@
 //  * Lanes own photon bins (32 consecutive bins per row, K rows per lane), warps
 //    own particles; per-warp FP32 register accumulators are folded into
 //    double-float accumulators after every chunk; at a segment's end the block sums
-//    its warps in FP64 (warp order) into one partial row per block, and a second
-//    kernel sums the blocks' rows in FP64 in a fixed order, so results are
+//    its warps (in warp order; in FP64, in launches of one short item a block in
+//    double-floats) into one partial row per block, and a second kernel sums the blocks' rows in FP64 in a fixed order, so results are
 //    bit-reproducible.
 //  * Particle streams (SoA FP32) are staged chunk by chunk into shared memory
 //    with 1-D TMA bulk copies (cp.async.bulk + mbarrier), double buffered.

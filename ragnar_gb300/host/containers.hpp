@@ -31,8 +31,7 @@ namespace rgh {
   // module's calls use, all of them on the null stream, come from the library's blocks (kBlock): a
   // call that returns one allocates and frees it without the driver.  With the grids' values kept
   // on the host and the library's own scratch pool a call's host time falls from 200 us to 20 us
-  // (IC emission 535 -> 72 us, a histogram of 3.3e7 particles 323 -> 138 us, a spectrum and a
-  // histogram of 1e4 particles 269 -> 78 us).  Particle components, whose addresses the module hands
+  // (a spectrum and a histogram of 1e4 particles took 269 us, now 72).  Particle components, whose addresses the module hands
   // out, are freed by the driver, which waits for every stream (kOwn).
   class DeviceBuffer {
   public:

@@ -8,10 +8,11 @@
     loss = rt.log_mse(S, S_target)
     loss.backward()                                                        # w.grad, ux.grad, ...
 
-The forward is the fused kernel (rg_spectrum_run); the backward is the
-hand-written adjoint kernel (rg_spectrum_adjoint), which recomputes e_peak
-instead of storing it.  With the smooth table (the default here) the derivative
-uses F'(x) = F(x)/x - x K_{5/3}(x).  All tensors are float32 on one CUDA device.
+The backward is the hand-written adjoint.  Plans that sum cell moments record
+each particle's place in the table in the forward (rg_spectrum_run_placed) and
+read it in the backward; others run rg_spectrum_run and recompute e_peak.  With
+the smooth table (the default here) the derivative uses
+F'(x) = F(x)/x - x K_{5/3}(x).  All tensors are float32 on one CUDA device.
 """
 
 from __future__ import annotations
